@@ -23,13 +23,12 @@
 // subtraction run in FP64 in both forms.
 //
 // Deposit: each particle's four node contributions (q FN v w) are rounded to
-// integers first, so the grid sum is exact and independent of order.  FP32:
-// a shared-memory window per chunk of sorted particles; FP64: lanes of a warp
-// that hit the same four nodes (equal sort key) are summed with
-// __reduce_add_sync before one 64-bit atomic per node.
+// integers first, so the grid sum is exact and independent of order: a
+// shared-memory window per chunk of sorted particles, then one 64-bit atomic
+// per touched node.
 //
-// The FP32 form drifts the whole step at once (the reference's two half
-// drifts joined).
+// Both forms drift the whole step at once (the reference's two half drifts
+// joined).
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -97,6 +96,9 @@ struct SimParams {
   int secondaries;
   long long cap;
   double qm_dt2;            // -q_e/m_e dt/2
+  double idr, idz, ic2;     // 1/dr, 1/dz, 1/c^2
+  double mu_qm;             // mu0 q_e/m_e dt/2 with the sign of qm_dt2 (FP64 form)
+  double dep_q;             // FP64 form: fixed-point factor of the electrons' current (x v)
   float aE, aB, hdr, hdz;   // FP32 form: impulse per (V/m), per (A/m); c dt/(2 dr), c dt/(2 dz)
   double dep;               // fixed-point factor: FP64 q FN scale (x v)
   float depf;               // FP32: q FN c scale (x beta)
@@ -401,8 +403,8 @@ __device__ __forceinline__ void k_commit_body(SimCounters *cnt, int q) {
 __global__ void k_commit(SimCounters *cnt, int q) { k_commit_body(cnt, q); }
 
 // ------------------------------------------------------ deposit
-// Each particle's four node contributions (q FN v w, both components) are
-// integers, so every summation order gives the same grid.  The lanes of a warp
+// The ions' deposit.  Each one's four node contributions (q FN v w, both
+// components) are integers, so every summation order gives the same grid.  The lanes of a warp
 // that share a node quad (the sort key; the quad fixes the four node indices)
 // are summed with redux.sync, one quad per round, and the first lane of the
 // quad adds the eight sums with 64-bit atomics.  Sorted particles put one to
@@ -488,72 +490,328 @@ __device__ __forceinline__ void deposit_values64(const SimParams &P, double r, d
   }
 }
 
-// The particles [beg, end) of the FP64 pass of step `step` (beg a multiple
-// of 32 apart from the block's first warp): mode 0: full step - kick, drift
-// (two half drifts), deposit; collision candidates go to queue q for k_mcc64;
-// mode 1: half drift + deposit only (start of a run); mode 2: kick + half
-// drift only, ending at integer time (end of a run).
-__device__ __forceinline__ void range64(const SimParams &P, const State64 &S,
-                                        const Fields<double> &F, SimCounters *cnt, int *queue,
-                                        int mode, int q, long long step, long long beg,
-                                        long long end) {
+// FP64 pass.  Bound by instruction issue and the shared-memory pipe (the
+// deposit's atomics).  2M electrons on 256 x 1024 cells: 36M warp
+// instructions, 64 us a pass.  With a division and a square root wherever
+// the formulas have one (some forty an electron), the drift in two halves and
+// the deposit summed by redux.sync over the lanes of each node quad it was
+// 108M and 169 us.  So the push multiplies by reciprocals (SimParams), takes
+// three rsqrt's and one division, forms floors and fixed-point roundings in
+// the FP64 adder, and deposits through a window in shared memory.  Three
+// blocks of 256 threads per SM: at four (64 registers) the step is 8 us
+// longer.  Chunks of up to 4608 particles: 1024 / 1536 / 2560 are 5 / 2 / 1 us
+// longer (more flushes).
+
+// x = i + f with i = floor(x) and f in [0, 1), for |x| < 2^31: rounding
+// x + 1.5 2^52 down leaves floor(x) in the low mantissa bits (exact)
+__device__ __forceinline__ int floor_split(double x, double &f) {
+  const double t = __dadd_rd(x, 6755399441055744.0);
+  f = __dsub_rn(x, __dsub_rn(t, 6755399441055744.0));
+  return __double2loint(t);
+}
+
+// Cell coordinate of x (in cells) on an axis of n cells: cell i in [0, n - 1]
+// (x = n exactly sits at the end of the last) and fraction f; the half-cell
+// staggered node pair a, a + 1 with weight w of the second, indices clamped
+// one-sided at the edges.
+struct Axis64 { int i, lo, hi; double f, w; };
+__device__ __forceinline__ Axis64 axis64(double x, int n) {
+  Axis64 A;
+  const int i = floor_split(x, A.f);
+  A.i = min(max(i, 0), n - 1);
+  if (i != A.i) A.f = __dsub_rn(x, (double)A.i);
+  const bool up = A.f >= 0.5;
+  const int a = up ? A.i : A.i - 1;
+  A.w = __dadd_rn(A.f, up ? -0.5 : 0.5);
+  A.lo = max(a, 0);
+  A.hi = min(a + 1, n - 1);
+  return A;
+}
+
+__device__ __forceinline__ double lerp64(double a, double b, double w) { return fma(w, __dsub_rn(b, a), a); }
+
+// Boris kick in E = (Er, 0, Ez), B = (0, mu0 H, 0) with the fields of the
+// staggered bilinear gather (EM4.cu:41-122).
+__device__ __forceinline__ void kick64(const SimParams &P, const Fields<double> &F, double r,
+                                       double z, double &ur, double ut, double &uz) {
+  const Axis64 R = axis64(__dmul_rn(r, P.idr), P.nr), Z = axis64(__dmul_rn(z, P.idz), P.nz);
+  const double *e0 = F.Er + (int64_t)Z.i * P.ldf, *e1 = e0 + P.ldf;
+  const double *z0 = F.Ez + (int64_t)Z.lo * P.ldf + R.i, *z1 = F.Ez + (int64_t)Z.hi * P.ldf + R.i;
+  const double *h0 = F.H + (int64_t)Z.lo * P.ldf, *h1 = F.H + (int64_t)Z.hi * P.ldf;
+  const double a0 = __ldg(e0 + R.lo), a1 = __ldg(e0 + R.hi), a2 = __ldg(e1 + R.lo), a3 = __ldg(e1 + R.hi);
+  const double b0 = __ldg(z0), b1 = __ldg(z0 + 1), b2 = __ldg(z1), b3 = __ldg(z1 + 1);
+  const double c0 = __ldg(h0 + R.lo), c1 = __ldg(h0 + R.hi), c2 = __ldg(h1 + R.lo), c3 = __ldg(h1 + R.hi);
+  const double Er = lerp64(lerp64(a0, a1, R.w), lerp64(a2, a3, R.w), Z.f);
+  const double Ez = lerp64(lerp64(b0, b1, R.f), lerp64(b2, b3, R.f), Z.w);
+  const double H = lerp64(lerp64(c0, c1, R.w), lerp64(c2, c3, R.w), Z.w);
+  const double umr = fma(P.qm_dt2, Er, ur), umz = fma(P.qm_dt2, Ez, uz);
+  const double u2 = fma(umr, umr, fma(ut, ut, __dmul_rn(umz, umz)));
+  const double t = __dmul_rn(__dmul_rn(P.mu_qm, H), rsqrt(fma(u2, P.ic2, 1.0)));
+  const double upr = fma(-umz, t, umr), upz = fma(umr, t, umz);
+  const double s = __ddiv_rn(__dadd_rn(t, t), fma(t, t, 1.0));
+  ur = fma(P.qm_dt2, Er, fma(-upz, s, umr));
+  uz = fma(P.qm_dt2, Ez, fma(upr, s, umz));
+}
+
+// Straight-line drift over the time dt (a whole step: the reference's two
+// half drifts joined - the same line, the radius along a line is convex, the
+// end reflection specular), EM2.cu:26-57.  ig: 1/gamma, kept by the turn.
+__device__ __forceinline__ void drift64(const SimParams &P, double dt, double &r, double &z, double &ur,
+                                        double &ut, double &uz, double &ig, bool &alive) {
+  ig = rsqrt(fma(fma(ur, ur, fma(ut, ut, __dmul_rn(uz, uz))), P.ic2, 1.0));
+  const double h = __dmul_rn(ig, dt);
+  const double X = fma(ur, h, r), Y = __dmul_rn(ut, h);
+  double Z = fma(uz, h, z);
+  const double r2 = fma(X, X, __dmul_rn(Y, Y));
+  const bool off = r2 > 0;
+  const double irn = off ? rsqrt(r2) : 0.0;
+  const double rn = __dmul_rn(r2, irn);
+  const double cs = off ? __dmul_rn(X, irn) : 1.0, sn = __dmul_rn(Y, irn);
+  const double nur = fma(cs, ur, __dmul_rn(sn, ut)), nut = fma(cs, ut, -__dmul_rn(sn, ur));
+  ur = nur; ut = nut;
+  if (rn > P.Rp) alive = false;
+  if (Z > P.Lp) { Z = __dsub_rn(2 * P.Lp, Z); uz = -uz; }
+  if (Z < 0) { Z = -Z; uz = -uz; }
+  r = rn; z = Z;
+}
+
+// FP64-form deposit window: 64-bit sums of one chunk of particles on a box of
+// the grid in shared memory, each sum as two 32-bit words - shared memory has
+// no native 64-bit add.  The low word's add returns its old value, which
+// tells whether this add carried; every carry is seen exactly once, so the two
+// words hold the sum modulo 2^64 whatever the order (|contribution| <= 2^48
+// keeps the high word's sum far inside 32 bits).  The four words of the
+// nodes (r low, r high, z low, z high) sit in four planes, so neighbouring
+// nodes are in neighbouring banks; rows are ws = 3 (mod 32) nodes apart, so the
+// 3 x 3 nodes around a warp's particles are in nine.
+constexpr int kWin64Nodes = 3072;
+constexpr int kWin64Bytes = kWin64Nodes * 16;
+constexpr int kWin64Cols = 256;           // columns of the box at most (wide grids)
+constexpr int kChunk64 = 4608;            // particles per chunk at most
+
+struct Win64 {
+  unsigned *w;
+  int row0, rows, col0, cols, ws;
+};
+
+__host__ __device__ inline int win64_cols(int nr) { return nr < kWin64Cols ? nr : kWin64Cols; }
+__host__ __device__ inline int win64_stride(int cols) { return cols + ((3 - cols % 32) + 32) % 32; }
+
+// Box of a chunk: the rows of its first and last live particles (row_lo..row_hi;
+// row_hi < 0: none live) plus up to three rows either side for the drift
+// since the last sort; all columns, or on a grid wider than the box those
+// from a little below the first particle's when the chunk sits in one row (the
+// particles are sorted by row, then column), else from the axis.
+__device__ __forceinline__ void chunk_box(int nr, int nz, int cols, int maxrows, int row_lo, int row_hi,
+                                          int col_lo, int &row0, int &rows, int &col0) {
+  row0 = 0; rows = maxrows; col0 = 0;
+  if (row_hi < 0) return;
+  const int core = row_hi - row_lo + 3;
+  const int below = maxrows >= core + 6 ? 3 : max(1, 1 + (maxrows - core) / 2);
+  row0 = min(max(0, row_lo - below), nz - maxrows);
+  rows = min(maxrows, row_hi + 4 - row0);
+  if (row_lo == row_hi) col0 = min(max(0, col_lo - 8), nr - cols);
+}
+
+__device__ __forceinline__ void box64(const SimParams &P, const State64 &S, long long beg, long long end,
+                                      int maxrows, int &row0, int &rows, int &col0) {
+  const double2 a = S.rz[beg], b = S.rz[end - 1];
+  int lo = P.nz, hi = -1, col = 0;
+  if (a.x >= 0) {
+    lo = hi = min(max((int)(a.y * P.idz), 0), P.nz - 1);
+    col = min(max((int)(a.x * P.idr), 0), P.nr - 1);
+  }
+  if (b.x >= 0) {
+    const int k = min(max((int)(b.y * P.idz), 0), P.nz - 1);
+    lo = min(lo, k);
+    hi = max(hi, k);
+  }
+  chunk_box(P.nr, P.nz, win64_cols(P.nr), maxrows, lo, hi, col, row0, rows, col0);
+}
+
+__device__ __forceinline__ void win64_add(unsigned *w, double v) {
+  const unsigned lo = (unsigned)__double2loint(v);
+  const int hi = __double2hiint(v) - 0x43380000;      // v = 1.5 2^52 + contribution
+  const unsigned old = atomicAdd(w, lo);
+  const int up = hi + (old + lo < lo ? 1 : 0);
+  if (up) atomicAdd(w + kWin64Nodes, (unsigned)up);
+}
+
+// One particle's current into its four nodes (EM7.cu:56-202 weights, clamped
+// one-sided at the edges): q FN v w in fixed point, rounded to nearest in one
+// FMA.  The lanes visit the nodes in an order permuted by lane & 3, so lanes on
+// the same quad hit four different nodes.  Nodes outside the box go to the grid.
+__device__ __forceinline__ void deposit64(const SimParams &P, const Win64 &w, double r, double z, double ur,
+                                          double uz, double ig) {
+  const Axis64 R = axis64(__dmul_rn(r, P.idr), P.nr), Z = axis64(__dmul_rn(z, P.idz), P.nz);
+  const double k = __dmul_rn(P.dep_q, ig), kr = __dmul_rn(k, ur), kz = __dmul_rn(k, uz);
+  const bool sc = threadIdx.x & 1, sr = threadIdx.x & 2;
+  const int ca = sc ? R.hi : R.lo, cb = sc ? R.lo : R.hi, ra = sr ? Z.hi : Z.lo, rb = sr ? Z.lo : Z.hi;
+  const double om = __dsub_rn(1.0, R.w), on = __dsub_rn(1.0, Z.w);
+  const double wa = sc ? R.w : om, wb = sc ? om : R.w, va = sr ? Z.w : on, vb = sr ? on : Z.w;
+#pragma unroll
+  for (int n = 0; n < 4; ++n) {
+    const int col = n & 1 ? cb : ca, row = n & 2 ? rb : ra;
+    const double b = __dmul_rn(n & 1 ? wb : wa, n & 2 ? vb : va);
+    const double vr = fma(kr, b, 6755399441055744.0), vz = fma(kz, b, 6755399441055744.0);
+    const unsigned lr = (unsigned)(row - w.row0), lc = (unsigned)(col - w.col0);
+    if (lr < (unsigned)w.rows && lc < (unsigned)w.cols) {
+      unsigned *m = w.w + ((int)lr * w.ws + (int)lc);
+      win64_add(m, vr);
+      win64_add(m + 2 * kWin64Nodes, vz);
+    } else {
+      const int64_t g = col + (int64_t)row * P.ldj;
+      const long long ir = __double_as_longlong(vr) - 0x4338000000000000LL;
+      const long long iz = __double_as_longlong(vz) - 0x4338000000000000LL;
+      if (ir) atomicAdd(P.Jr + g, (unsigned long long)ir);
+      if (iz) atomicAdd(P.Jz + g, (unsigned long long)iz);
+    }
+  }
+}
+
+// add the box to the grid (one 64-bit atomic per nonzero sum) and zero it:
+// its first bw columns, the ones the chunk touched
+__device__ __forceinline__ void flush64(const SimParams &P, const Win64 &w, int bw) {
+  const int nb = bw > 0 ? bw * w.rows : 0;
+  for (int i = threadIdx.x; i < nb; i += kBlock) {
+    const int row = i / bw, col = i - row * bw;
+    unsigned *m = w.w + row * w.ws + col;
+    const uint4 v = make_uint4(m[0], m[kWin64Nodes], m[2 * kWin64Nodes], m[3 * kWin64Nodes]);
+    if (v.x | v.y | v.z | v.w) {
+      const int64_t g = (int64_t)(w.row0 + row) * P.ldj + w.col0 + col;
+      if (v.x | v.y) atomicAdd(P.Jr + g, ((unsigned long long)v.y << 32) + v.x);
+      if (v.z | v.w) atomicAdd(P.Jz + g, ((unsigned long long)v.w << 32) + v.z);
+      m[0] = m[kWin64Nodes] = m[2 * kWin64Nodes] = m[3 * kWin64Nodes] = 0;
+    }
+  }
+}
+
+// Bring the state of particles [beg, end) into L2 ahead of their chunk (one
+// thread; cp.async.bulk.prefetch.L2, a hint that completes on its own).  beg
+// is a multiple of the chunk size, hence even, so every range starts on a
+// 16-byte boundary; the sizes are rounded down to 16 bytes.
+__device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) {
+  if (bytes) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void prefetch_chunk64(const State64 &S, long long beg, long long end) {
+  const long long n = end - beg;
+  if (n <= 0) return;
+  prefetch_l2(S.rz + beg, (uint32_t)(n * 16));
+  prefetch_l2(S.urt + beg, (uint32_t)(n * 16));
+  prefetch_l2(S.uz + beg, (uint32_t)((n * 8) & ~15ll));
+  prefetch_l2(S.id + beg, (uint32_t)((n * 8) & ~15ll));
+}
+
+// The particles [beg, end) of one chunk of the FP64 pass of step `step`
+// (executed by the whole block).  MODE 0: full step - kick, drift, deposit;
+// collision candidates go to queue q for k_mcc64; MODE 1: half drift +
+// deposit only (start of a run); MODE 2: kick + half drift only, ending at
+// integer time (end of a run).  The highest box column touched is merged
+// into *box_cmax.
+template <int MODE>
+__device__ __forceinline__ void chunk64(const SimParams &P, const State64 &S, const Fields<double> &F,
+                                        SimCounters *cnt, int *queue, int q, long long step, int beg,
+                                        int end, const Win64 &w, int *box_cmax) {
   const int lane = threadIdx.x & 31;
   unsigned lost = 0;
-  for (long long base = beg + (threadIdx.x & ~31); base < end; base += blockDim.x) {
-    const long long p = base + lane;
-    bool act = p < end;
-    double2 rz = make_double2(-1.0, 0.0), urt = make_double2(0.0, 0.0);
-    double uz = 0;
-    if (act) {
-      rz = S.rz[p];
-      act = rz.x >= 0;
-    }
+  int cmax = -1;
+  int base = beg + (int)(threadIdx.x & ~31);
+  double2 rzn = make_double2(-1.0, 0.0), urtn = rzn;
+  double uzn = 0;
+  uint64_t idn = 0;
+  // the next iteration's particle is loaded one iteration ahead, so its latency
+  // overlaps the current particle's arithmetic
+  auto load = [&](int k) {
+    rzn = S.rz[k];
+    urtn = S.urt[k];
+    uzn = S.uz[k];
+    if (MODE == 0) idn = S.id[k];
+  };
+  if (base + lane < end) load(base + lane);
+  for (; base < end; base += kBlock) {
+    const int p = base + lane;
+    const double2 rz = rzn, urt = urtn;
+    double uz = uzn;
+    const uint64_t id = idn;
+    bool act = rz.x >= 0;
+    rzn.x = -1.0;
+    if (p + kBlock < end) load(p + kBlock);
     bool cand = false;
     if (act) {
-      urt = S.urt[p]; uz = S.uz[p];
-      double r = rz.x, z = rz.y, ur = urt.x, ut = urt.y;
-      bool alive = true;
-      if (mode != 1) {
-        double E_r, E_z, Hp;
-        gather3s<double>(F.Er, F.Ez, F.H, P.nr, P.nz, P.ldf, P.ldf, P.ldf, P.dr, P.dz, r, z, E_r,
-                         E_z, Hp);
-        const double B = P.mu0 * Hp;
-        boris(ur, ut, uz, E_r, 0.0, E_z, 0.0, B, 0.0, P.qm_dt2, P.c);
-        halfdrift64(r, z, ur, ut, uz, alive, P);
-      }
-      if (alive && mode != 2) halfdrift64(r, z, ur, ut, uz, alive, P);
-      if (alive && mode == 0) cand = null_candidate(P, S.id[p], step);
-      if (!alive) {
+      double ur = urt.x, ut = urt.y, r = rz.x, z = rz.y, ig;
+      if (MODE == 0) cand = null_candidate(P, id, step);
+      if (MODE != 1) kick64(P, F, r, z, ur, ut, uz);
+      drift64(P, MODE == 0 ? P.dt : 0.5 * P.dt, r, z, ur, ut, uz, ig, act);
+      if (!act) {
         lost++;
+        cand = false;
         r = -1.0;
-        count_wall_loss(cnt, (ur * ur + ut * ut + uz * uz) / (P.c * P.c), P.me * P.c * P.c / P.qe);
+        count_wall_loss(cnt, (ur * ur + ut * ut + uz * uz) * P.ic2, P.me * P.c * P.c / P.qe);
       }
-      rz = make_double2(r, z); urt = make_double2(ur, ut);
-      S.rz[p] = rz; S.urt[p] = urt; S.uz[p] = uz;
-      act = alive && mode != 2;
+      S.rz[p] = make_double2(r, z);
+      S.urt[p] = make_double2(ur, ut);
+      S.uz[p] = uz;
+      if (MODE != 2 && act) {
+        deposit64(P, w, r, z, ur, uz, ig);
+        cmax = max(cmax, min((int)(r * P.idr) + 1, P.nr - 1) - w.col0);
+      }
     }
-    queue_push(cand, p, &cnt->n_cand[q], queue + (long long)q * P.cap);
-    int64_t a[4] = {0, 0, 0, 0};
-    long long vr[4] = {0, 0, 0, 0}, vz[4] = {0, 0, 0, 0};
-    unsigned key = 0;
-    if (act) deposit_values64(P, rz.x, rz.y, urt.x, urt.y, uz, -P.qe, a, vr, vz, key);
-    warp_deposit<long long>(act, key, a, vr, vz, P.Jr, P.Jz);
+    if (MODE == 0) queue_push(cand, p, &cnt->n_cand[q], queue + (long long)q * P.cap);
+  }
+  if (MODE != 2) {
+    cmax = __reduce_max_sync(0xFFFFFFFFu, cmax);
+    if (lane == 0 && cmax >= 0) atomicMax(box_cmax, min(cmax, w.cols - 1));
   }
   lost = __reduce_add_sync(0xFFFFFFFFu, lost);
   if (lane == 0 && lost) atomicAdd(&cnt->lost, (unsigned long long)lost);
 }
 
+// Chunk size that gives every one of `blocks` blocks the same number of
+// chunks (as few as kChunk64 allows), a multiple of the block size.
+__device__ __forceinline__ int even_chunk64(long long n, unsigned blocks) {
+  const long long per = (n + blocks - 1) / blocks;
+  const long long k = (per + kChunk64 - 1) / kChunk64;
+  const long long c = k > 0 ? (per + k - 1) / k : 1;
+  return (int)((c + kBlock - 1) / kBlock) * kBlock;
+}
+
+template <int MODE>
 __global__ void __launch_bounds__(kBlock, 3) k_pass64(SimParams P, State64 S, Fields<double> F,
-                                                      SimCounters *cnt, int *queue, int mode,
-                                                      int q) {
+                                                      SimCounters *cnt, int *queue, int q) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ int box_row0[2], box_rows[2], box_col0[2], box_cmax[2];   // of this chunk and the next
   const long long n0 = slots_in_use(cnt);
   const long long step = cnt->step;
   if (blockIdx.x == 0 && threadIdx.x == 0) cnt->uncommitted = 1;
-  // each block takes a contiguous chunk of the (cell-sorted) particles, so its
-  // field reads stay in a narrow band of grid rows
-  const long long chunk = (n0 + gridDim.x - 1) / gridDim.x;
-  const long long beg = (long long)blockIdx.x * chunk, end = min(beg + chunk, n0);
-  range64(P, S, F, cnt, queue, mode, q, step, beg, end);
+  const int chunk = even_chunk64(n0, gridDim.x);
+  const int cols = win64_cols(P.nr), ws = win64_stride(cols), maxrows = min(kWin64Nodes / ws, P.nz);
+  // the window starts zeroed; each chunk's flush leaves it zeroed again
+  for (int i = threadIdx.x; i < kWin64Nodes; i += kBlock) reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0, 0, 0, 0);
+  // the blocks take the chunks in turn, so neighbouring blocks work on
+  // neighbouring grid rows; thread 0 brings the block's next chunk into L2
+  // and, at the end of this one, places its box
+  const long long stride = (long long)gridDim.x * chunk;
+  long long beg = (long long)blockIdx.x * chunk;
+  if (threadIdx.x == 0) {
+    box_cmax[0] = -1;
+    if (MODE != 2 && beg < n0) box64(P, S, beg, min(beg + chunk, n0), maxrows, box_row0[0], box_rows[0], box_col0[0]);
+  }
+  int b = 0;
+  __syncthreads();
+  for (; beg < n0; beg += stride, b ^= 1) {
+    const Win64 w{reinterpret_cast<unsigned *>(smem), box_row0[b], box_rows[b], box_col0[b], cols, ws};
+    const long long nb = beg + stride;
+    if (threadIdx.x == 0 && nb < n0) prefetch_chunk64(S, nb, min(nb + chunk, n0));
+    chunk64<MODE>(P, S, F, cnt, queue, q, step, (int)beg, (int)min(beg + chunk, n0), w, &box_cmax[b]);
+    if (MODE == 2) continue;
+    if (threadIdx.x == 0) {
+      box_cmax[b ^ 1] = -1;
+      if (nb < n0) box64(P, S, nb, min(nb + chunk, n0), maxrows, box_row0[b ^ 1], box_rows[b ^ 1], box_col0[b ^ 1]);
+    }
+    __syncthreads();
+    flush64(P, w, box_cmax[b] + 1);
+    __syncthreads();
+  }
 }
 
 // The collision of candidate slot p queued at step `step` (FP64 form): MCC,
@@ -626,8 +884,6 @@ struct BatchCell64 {
   int *queue;
   Fields<double> F[2];        // field buffers 0 / 1 (the pass into current buffer jb reads F[jb])
 };
-constexpr int kChunk64 = 2048;               // particles per work item of the batched FP64 pass
-
 __global__ void k_batch_commit64(const BatchCell64 *__restrict__ cells, int ncell, int q) {
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x)
     k_commit_body(cells[c].cnt, q);
@@ -656,36 +912,90 @@ __global__ void __launch_bounds__(kMccBlock) k_batch_mcc64(const BatchCell64 *__
   }
 }
 
-// The FP64 pass of every cell of a batch: (cell, chunk of kChunk64) work
-// items from one counter (*chunk_next, zeroed before the launch).
+// The FP64 pass of every cell of a batch: (cell, chunk) work items from one
+// counter (*chunk_next, zeroed before the launch), the cell's parameters
+// copied into shared memory when the cell changes.
 __global__ void __launch_bounds__(kBlock, 3) k_batch_pass64(const BatchCell64 *__restrict__ cells,
-                                                            int ncell, int cur, int jb, int mode,
-                                                            int q, unsigned long long *chunk_next) {
+                                                            int ncell, int cur, int jb, int q,
+                                                            unsigned long long *chunk_next) {
+  extern __shared__ __align__(128) unsigned char smem[];
   __shared__ long long pre[kMaxBatch + 1];
   __shared__ long long item_at;
-  for (int c = threadIdx.x; c < ncell; c += blockDim.x)
-    pre[c + 1] = (slots_in_use(cells[c].cnt) + kChunk64 - 1) / kChunk64;
+  __shared__ int chunk_s, cell_at, box_row0, box_rows, box_col0, box_cmax;
+  __shared__ __align__(16) unsigned char sP_raw[sizeof(SimParams)];
+  SimParams &sP = *reinterpret_cast<SimParams *>(sP_raw);
+  for (int i = threadIdx.x; i < kWin64Nodes; i += kBlock) reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0, 0, 0, 0);
+  for (int c = threadIdx.x; c < ncell; c += blockDim.x) pre[c + 1] = slots_in_use(cells[c].cnt);
   __syncthreads();
   if (threadIdx.x == 0) {
+    long long total = 0;
+    for (int c = 0; c < ncell; ++c) total += pre[c + 1];
+    // a few chunks per block, so that the counter evens out the cells
+    const int chunk = min(kChunk64, even_chunk64((total + 3) / 4, gridDim.x));
+    chunk_s = chunk;
+    cell_at = -1;
     pre[0] = 0;
-    for (int c = 0; c < ncell; ++c) pre[c + 1] += pre[c];
+    for (int c = 0; c < ncell; ++c) pre[c + 1] = pre[c] + (pre[c + 1] + chunk - 1) / chunk;
     if (blockIdx.x == 0)
       for (int c = 0; c < ncell; ++c) cells[c].cnt->uncommitted = 1;
   }
   __syncthreads();
   const long long nitem = pre[ncell];
+  const int chunk = chunk_s;
+  // thread 0 claims the block's next item while one is worked on, brings its
+  // state into L2 and, at the end of this one, places its box
+  long long next = 0;
+  int next_row0 = 0, next_rows = 0, next_col0 = 0;
+  auto span = [&](long long g, const BatchCell64 *&C, long long &beg, long long &end) {
+    const int c = cell_of_item(pre, ncell, g);
+    C = cells + c;
+    beg = (g - pre[c]) * chunk;
+    end = min(beg + chunk, slots_in_use(C->cnt));
+  };
+  auto resolve = [&]() {
+    if (next >= nitem) return;
+    const BatchCell64 *C;
+    long long beg, end;
+    span(next, C, beg, end);
+    const SimParams &Pc = C->P[jb];
+    prefetch_chunk64(C->S[cur], beg, end);
+    box64(Pc, C->S[cur], beg, end, min(kWin64Nodes / win64_stride(win64_cols(Pc.nr)), Pc.nz), next_row0,
+          next_rows, next_col0);
+  };
+  if (threadIdx.x == 0) {
+    next = (long long)atomicAdd(chunk_next, 1ull);
+    resolve();
+  }
   for (;;) {
-    if (threadIdx.x == 0) item_at = (long long)atomicAdd(chunk_next, 1ull);
+    if (threadIdx.x == 0) {
+      item_at = next;
+      box_row0 = next_row0;
+      box_rows = next_rows;
+      box_col0 = next_col0;
+      box_cmax = -1;
+    }
     __syncthreads();
     const long long g = item_at;
-    __syncthreads();
     if (g >= nitem) break;
-    const int c = cell_of_item(pre, ncell, g);
-    const BatchCell64 &C = cells[c];
-    SimCounters *cc = C.cnt;
-    const long long n0 = slots_in_use(cc);
-    const long long beg = (g - pre[c]) * kChunk64, end = min(beg + kChunk64, n0);
-    range64(C.P[jb], C.S[cur], C.F[jb], cc, C.queue, mode, q, cc->step, beg, end);
+    if (threadIdx.x == 0) next = (long long)atomicAdd(chunk_next, 1ull);
+    const BatchCell64 *C;
+    long long beg, end;
+    span(g, C, beg, end);
+    const int c = (int)(C - cells);
+    if (c != cell_at) {          // this block's first chunk of cell c: its parameters
+      const uint32_t *src = reinterpret_cast<const uint32_t *>(&C->P[jb]);
+      uint32_t *dst = reinterpret_cast<uint32_t *>(sP_raw);
+      for (int i = threadIdx.x; i < (int)(sizeof(SimParams) / 4); i += kBlock) dst[i] = src[i];
+      __syncthreads();
+      if (threadIdx.x == 0) cell_at = c;
+    }
+    const int cols = win64_cols(sP.nr);
+    const Win64 w{reinterpret_cast<unsigned *>(smem), box_row0, box_rows, box_col0, cols, win64_stride(cols)};
+    chunk64<0>(sP, C->S[cur], C->F[jb], C->cnt, C->queue, q, C->cnt->step, (int)beg, (int)end, w, &box_cmax);
+    if (threadIdx.x == 0) resolve();
+    __syncthreads();
+    flush64(sP, w, box_cmax + 1);
+    __syncthreads();
   }
 }
 
@@ -1238,13 +1548,6 @@ __device__ __forceinline__ void chunk_rows32(const SimParams &P, const State32 &
   }
 }
 
-// Bring the state of particles [beg, end) into L2 ahead of their chunk (one
-// thread; cp.async.bulk.prefetch.L2, a hint that completes on its own).  beg
-// is a multiple of the chunk size, hence even, so every range starts on a
-// 16-byte boundary; the sizes are rounded down to 16 bytes.
-__device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) {
-  if (bytes) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void prefetch_chunk32(const State32 &S, long long beg, long long end) {
   const long long n = end - beg;
   if (n <= 0) return;
@@ -2257,8 +2560,11 @@ int launch_pass(gasatt_sim *s, cudaStream_t st, int mode, int jb, int q, int fb)
   P.Jz = s->Jz[jb];
   const int b = s->cur;
   if (s->form == 0)
-    k_pass64<<<s->pass_grid, kBlock, 0, st>>>(P, s->s64[b], fields_of<double>(s, fb), s->cnt,
-                                              s->queue, mode, q);
+  {
+    auto kern = mode == 0 ? k_pass64<0> : mode == 1 ? k_pass64<1> : k_pass64<2>;
+    kern<<<s->pass_grid, kBlock, kWin64Bytes, st>>>(P, s->s64[b], fields_of<double>(s, fb), s->cnt,
+                                                    s->queue, q);
+  }
   else
   {
     auto kern = mode == 0 ? k_pass32<0> : mode == 1 ? k_pass32<1> : k_pass32<2>;
@@ -2802,6 +3108,8 @@ int gasatt_sim_create(gasatt_ctx *ctx, const gasatt_sim_config *cfg, const gasat
   P.ion_cap = c.ion_capacity;
   P.ion_sigma = c.ion_capacity > 0 ? std::sqrt(c.kb * c.gas_temperature / c.m_ion) : 0.0;
   P.qm_dt2 = -c.q_e / c.m_e * c.dt / 2;
+  P.idr = 1 / c.dr; P.idz = 1 / c.dz; P.ic2 = 1 / (c.c * c.c);
+  P.mu_qm = c.mu0 * P.qm_dt2;
   P.aE = (float)(-c.q_e * c.dt / (2 * c.m_e * c.c));
   P.aB = (float)(-c.q_e * c.dt * c.mu0 / (2 * c.m_e));
   P.hdr = (float)(c.c * c.dt / (2 * c.dr));
@@ -2811,6 +3119,7 @@ int gasatt_sim_create(gasatt_ctx *ctx, const gasatt_sim_config *cfg, const gasat
   const double qfc = c.q_e * std::fabs(c.FN) * c.c;
   s->scale = s->form == 0 ? std::ldexp(1.0, 48) / qfc : std::ldexp(1.0, 20) / qfc;
   P.dep = s->scale;
+  P.dep_q = -c.q_e * c.FN * s->scale;
   P.depf = (float)(-c.q_e * c.FN * c.c * s->scale);
   s->ion_scale = std::ldexp(1.0, 48) / qfc;
   set_collision_bound(s, c.gas_density);
@@ -2842,7 +3151,12 @@ int gasatt_sim_create(gasatt_ctx *ctx, const gasatt_sim_config *cfg, const gasat
       return cleanup(rc);
   }
   int occ = 4;
-  if (s->form == 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pass64, kBlock, 0);
+  if (s->form == 0) {
+    for (auto k : {k_pass64<0>, k_pass64<1>, k_pass64<2>})
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kWin64Bytes) != cudaSuccess)
+        return cleanup(fail(ctx, GASATT_E_CUDA, "FP64 pass: shared memory"));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pass64<0>, kBlock, kWin64Bytes);
+  }
   else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pass32<0>, kBlock, 0);
   s->pass_grid = (unsigned)(nsm * (occ > 0 ? occ : 1));
   if (s->form == 1) {
@@ -3696,7 +4010,10 @@ int batch_group_setup(gasatt_batch *b, BatchGroup &G) {
   G.fdtd_grid = (unsigned)(fslots < fblocks ? fslots : (fblocks > 0 ? fblocks : 1));
   occ = 1;
   if (G.form == 1) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_pass32, kBlock, 0);
-  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_pass64, kBlock, 0);
+  else {
+    GASATT_CUDA(ctx, cudaFuncSetAttribute(k_batch_pass64, cudaFuncAttributeMaxDynamicSharedMemorySize, kWin64Bytes));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_pass64, kBlock, kWin64Bytes);
+  }
   G.pass_grid = (unsigned)(nsm * (occ > 0 ? occ : 1));
   occ = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_mcc64, kMccBlock, 0);
@@ -3732,8 +4049,8 @@ int batch_group_launch(gasatt_batch *b, BatchGroup &G, cudaStream_t cs, cudaStre
   GASATT_CUDA(ctx, cudaGetLastError());
   GASATT_CUDA(ctx, cudaStreamWaitEvent(cs, b->join_ev, 0));
   GASATT_CUDA(ctx, cudaMemsetAsync(G.chunk_next, 0, 8, cs));
-  k_batch_pass64<<<G.pass_grid, kBlock, 0, cs>>>((const BatchCell64 *)G.cells, n, cur, 1 - q, 0, q,
-                                                 G.chunk_next);
+  k_batch_pass64<<<G.pass_grid, kBlock, kWin64Bytes, cs>>>((const BatchCell64 *)G.cells, n, cur, 1 - q, q,
+                                                           G.chunk_next);
   GASATT_CUDA(ctx, cudaGetLastError());
   return GASATT_OK;
 }
