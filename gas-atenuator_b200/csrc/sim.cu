@@ -1903,11 +1903,14 @@ __global__ void __launch_bounds__(kMccBlock) k_batch_collide32(const BatchCell32
   }
 }
 
-// every cell's collision queue of parity q emptied, after its collisions ran
+// every cell's collision queue of parity q (q < 0: both) emptied, after its
+// collisions ran
 template <typename Cell>
 __global__ void k_batch_clear_cand(const Cell *__restrict__ cells, int ncell, int q) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x)
-    cells[c].cnt->n_cand[q] = 0;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x) {
+    if (q != 1) cells[c].cnt->n_cand[0] = 0;
+    if (q != 0) cells[c].cnt->n_cand[1] = 0;
+  }
 }
 
 // ------------------------------------------------------------- FDTD
@@ -2610,7 +2613,14 @@ int flush_collisions(gasatt_sim *s) {
   cudaStream_t st = s->ctx->stream;
   if (s->form == 0) SIM_TRY(launch_commit(s, st, q));
   SIM_TRY(launch_mcc(s, st, q));
-  GASATT_CUDA(s->ctx, cudaMemsetAsync(&s->cnt->n_cand[q], 0, sizeof(unsigned long long), st));
+  // The FP32 kernels pick their queue by the parity of the device's step
+  // counter, which gasatt_sim_run_host moves against host_step's, so both
+  // queues are emptied (the other one was consumed by the last pass); the
+  // FP64 kernels are told the parity q.
+  if (s->form == 1)
+    GASATT_CUDA(s->ctx, cudaMemsetAsync(s->cnt->n_cand, 0, sizeof(s->cnt->n_cand), st));
+  else
+    GASATT_CUDA(s->ctx, cudaMemsetAsync(&s->cnt->n_cand[q], 0, sizeof(unsigned long long), st));
   s->mcc_pending = false;
   return GASATT_OK;
 }
@@ -4139,7 +4149,7 @@ int batch_flush_collisions(gasatt_batch *b) {
     const int n = (int)G.sims.size(), cur = s0->cur, q = (int)((s0->host_step - 1) & 1);
     if (G.form == 1) {
       k_batch_collide32<<<G.pass_grid, kMccBlock, 0, st>>>((const BatchCell32 *)G.cells, n, cur);
-      k_batch_clear_cand<<<1, 256, 0, st>>>((const BatchCell32 *)G.cells, n, q);
+      k_batch_clear_cand<<<1, 256, 0, st>>>((const BatchCell32 *)G.cells, n, -1);   // see flush_collisions
       ctx->launches += 2;
     } else {
       k_batch_commit64<<<1, 256, 0, st>>>((const BatchCell64 *)G.cells, n, q);
