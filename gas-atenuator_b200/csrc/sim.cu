@@ -55,8 +55,9 @@ struct SimCounters {
   unsigned long long sorted_total;
   long long cand_step[2];        // FP64: the pass that queued each queue
   int uncommitted;               // FP64: a pass ran since the last commit (k_commit)
-  int pad0_;
-  unsigned long long pad1_[9];
+  int chunk;                     // FP32: particles per chunk of the next pass
+  int chunk_fixed, pass_blocks;  // FP32: the configured chunk (0: by population), blocks of a pass
+  unsigned long long pad1_[8];
   unsigned long long n_births;   // slots claimed by births since the last commit
   unsigned long long pad2_[15];
   unsigned long long n_cand[2];  // collision candidates queued, per queue parity
@@ -82,6 +83,18 @@ __device__ __forceinline__ long long slots_in_use(const SimCounters *cnt) {
   return (long long)(nt < cnt->cap ? nt : cnt->cap);
 }
 
+// Chunk size that gives every one of `blocks` blocks the same number of
+// chunks, as few as `most` particles a chunk allow: a multiple of the block
+// size.  A small population is spread over all blocks: with chunks of 1792 the
+// FP32 pass ran 4,000 electrons on 3 blocks (step 33 us, now 21) and 300,000 on
+// 168 of the 592 that fit (41 us, now 32); 2M electrons fill the blocks either way.
+__host__ __device__ inline int even_chunk(unsigned n, unsigned blocks, int most) {
+  const unsigned per = n / blocks + 1;
+  const unsigned k = (per + most - 1) / most;
+  return (int)(((per + k - 1) / k + kBlock - 1) / kBlock) * kBlock;
+}
+constexpr int kChunkMax = 7 * kBlock;     // FP32 pass: 1792 particles a chunk at most
+
 // N2+ ions (FP64 in both forms): (r, z), (u_r, u_theta), u_z, id, charge number
 struct IonState { double2 *rz; double2 *urt; double *uz; uint64_t *id; int8_t *q; };
 
@@ -103,7 +116,7 @@ struct SimParams {
   double dep;               // fixed-point factor: FP64 q FN scale (x v)
   float depf;               // FP32: q FN c scale (x beta)
   uint64_t cand_below;      // null-collision candidate iff the 52-bit draw is below this
-  int chunk;                // FP32 pass: particles per chunk (a multiple of the block, <= kChunkMax)
+  int chunk;                // FP32 pass: particles per chunk (a multiple of the block, <= kChunkMax; 0: chosen by population)
   // tables
   const double *sig;        // 3 x G (el, ion, exc)
   const double *cdf;        // G x 181
@@ -766,15 +779,6 @@ __device__ __forceinline__ void chunk64(const SimParams &P, const State64 &S, co
   if (lane == 0 && lost) atomicAdd(&cnt->lost, (unsigned long long)lost);
 }
 
-// Chunk size that gives every one of `blocks` blocks the same number of
-// chunks (as few as kChunk64 allows), a multiple of the block size.
-__device__ __forceinline__ int even_chunk64(long long n, unsigned blocks) {
-  const long long per = (n + blocks - 1) / blocks;
-  const long long k = (per + kChunk64 - 1) / kChunk64;
-  const long long c = k > 0 ? (per + k - 1) / k : 1;
-  return (int)((c + kBlock - 1) / kBlock) * kBlock;
-}
-
 template <int MODE>
 __global__ void __launch_bounds__(kBlock, 3) k_pass64(SimParams P, State64 S, Fields<double> F,
                                                       SimCounters *cnt, int *queue, int q) {
@@ -783,7 +787,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_pass64(SimParams P, State64 S, Fi
   const long long n0 = slots_in_use(cnt);
   const long long step = cnt->step;
   if (blockIdx.x == 0 && threadIdx.x == 0) cnt->uncommitted = 1;
-  const int chunk = even_chunk64(n0, gridDim.x);
+  const int chunk = even_chunk((unsigned)n0, gridDim.x, kChunk64);
   const int cols = win64_cols(P.nr), ws = win64_stride(cols), maxrows = min(kWin64Nodes / ws, P.nz);
   // the window starts zeroed; each chunk's flush leaves it zeroed again
   for (int i = threadIdx.x; i < kWin64Nodes; i += kBlock) reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0, 0, 0, 0);
@@ -931,7 +935,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_batch_pass64(const BatchCell64 *_
     long long total = 0;
     for (int c = 0; c < ncell; ++c) total += pre[c + 1];
     // a few chunks per block, so that the counter evens out the cells
-    const int chunk = min(kChunk64, even_chunk64((total + 3) / 4, gridDim.x));
+    const int chunk = even_chunk((unsigned)min((total + 3) / 4, 0x7FFFFFFFll), gridDim.x, kChunk64);
     chunk_s = chunk;
     cell_at = -1;
     pre[0] = 0;
@@ -1330,7 +1334,6 @@ __device__ __forceinline__ void deposit_nodes32(const SimParams &P, int ir, int 
 // outside the window go straight to the grid with 64-bit atomics; the window
 // is added to the grid with one 64-bit atomic per touched node.
 constexpr int kWinNodes = 4096;           // nodes (two int32 sums each)
-constexpr int kChunkMax = 7 * kBlock;     // 1792 particles (the default chunk)
 
 struct Win32 {
   int *rz;                  // node k: r at rz[2k], z at rz[2k + 1]
@@ -1685,29 +1688,36 @@ __global__ void __launch_bounds__(kBlock, 4) k_pass32(SimParams P, State32 S, Fi
   for (int i = threadIdx.x; i < kWinNodes; i += kBlock) reinterpret_cast<int2 *>(win_rz)[i] = make_int2(0, 0);
   const int ws = win_stride(P.nr);
   const int maxrows = min(kWinNodes / ws, P.nz);
-  const int chunk = P.chunk;
-  const long long nchunk = (n0 + chunk - 1) / chunk;
+  const int chunk = max(cnt->chunk, kBlock);      // chosen with the commit (no division here)
+  if (mode != 1) {
+    // The candidates go to the last blocks, kCandLanes per warp, one per lane;
+    // where there are fewer chunks than blocks, to the warps of all blocks that
+    // would otherwise be idle, fewer per warp.  A block takes its chunks after
+    // its candidates.
+    const long long nq = (long long)cnt->n_cand[par ^ 1];
+    const int *qin = queue + (long long)(par ^ 1) * P.cap;
+    int lanes = kCandLanes;
+    if (n0 <= (long long)chunk * (gridDim.x - 1)) {
+      const unsigned idle = (gridDim.x - ((unsigned)n0 + chunk - 1) / chunk) * (kBlock / 32);
+      lanes = (int)min(((unsigned)nq + idle - 1) / idle, (unsigned)kCandLanes);
+    }
+    unsigned lost = 0;
+    if (lane < lanes)
+      for (long long k = ((long long)(gridDim.x - 1 - blockIdx.x) * (kBlock / 32) + warp) * lanes + lane; k < nq;
+           k += (long long)gridDim.x * (kBlock / 32) * lanes)
+        candidate32(Pg, F, S, cnt, queue, qin[k], step, mode, true, n0, lost);
+    if (lost) atomicAdd(&cnt->lost, (unsigned long long)lost);
+  }
   // thread 0 claims the block's next chunk (index and window rows) a chunk
-  // ahead and has its state brought into L2 meanwhile; the first one before
-  // the candidates, so that it has their time to arrive
+  // ahead and has its state brought into L2 meanwhile
   long long next_ch = 0;
   int next_row0 = 0, next_rows = 0;
   if (threadIdx.x == 0) {
     next_ch = (long long)atomicAdd(&cnt->chunk_next, 1ull);
-    if (next_ch < nchunk) prefetch_chunk32(S, next_ch * chunk, min((next_ch + 1) * chunk, n0));
+    if (next_ch * chunk < n0) prefetch_chunk32(S, next_ch * chunk, min((next_ch + 1) * chunk, n0));
   }
-  if (mode != 1) {
-    const long long nq = (long long)cnt->n_cand[par ^ 1];
-    const int *qin = queue + (long long)(par ^ 1) * P.cap;
-    // kCandLanes candidates per warp, one per lane
-    unsigned lost = 0;
-    if (lane < kCandLanes)
-      for (long long k = ((long long)blockIdx.x * (kBlock / 32) + warp) * kCandLanes + lane; k < nq;
-           k += (long long)gridDim.x * (kBlock / 32) * kCandLanes)
-        candidate32(Pg, F, S, cnt, queue, qin[k], step, mode, true, n0, lost);
-    if (lost) atomicAdd(&cnt->lost, (unsigned long long)lost);
-  }
-  if (threadIdx.x == 0 && next_ch < nchunk) chunk_rows32(P, S, n0, chunk, next_ch, maxrows, next_row0, next_rows);
+  if (threadIdx.x == 0 && next_ch * chunk < n0)
+    chunk_rows32(P, S, n0, chunk, next_ch, maxrows, next_row0, next_rows);
   for (;;) {
     if (threadIdx.x == 0) {
       chunk_at = next_ch;
@@ -1717,7 +1727,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_pass32(SimParams P, State32 S, Fi
     }
     __syncthreads();
     const long long ch = chunk_at;
-    if (ch >= nchunk) break;
+    if (ch * chunk >= n0) break;
     // thread 0 claims the next chunk now; the claim's result is first used
     // after this chunk, so its round trip overlaps the chunk's work instead
     // of holding the block at the barrier above
@@ -1726,7 +1736,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_pass32(SimParams P, State32 S, Fi
     const int beg = (int)(ch * chunk), end = (int)min((long long)beg + chunk, n0);
     const Win32 w{win_rz, win_row0, win_rows, ws};
     chunk32<MODE>(P, S, F, cnt, queue, step, beg, end, w, &box_cmax);
-    if (threadIdx.x == 0 && next_ch < nchunk) {
+    if (threadIdx.x == 0 && next_ch * chunk < n0) {
       prefetch_chunk32(S, next_ch * chunk, min((next_ch + 1) * chunk, n0));
       chunk_rows32(P, S, n0, chunk, next_ch, maxrows, next_row0, next_rows);
     }
@@ -1763,18 +1773,28 @@ __global__ void __launch_bounds__(kBlock, 4) k_batch_pass32(const BatchCell32 *_
   __shared__ int win_row0, win_rows, box_cmax, cell_at;
   __shared__ long long chunk_at;
   __shared__ long long cand_pre[kMaxBatch + 1], chunk_pre[kMaxBatch + 1];
+  __shared__ int cell_chunk[kMaxBatch];
+  __shared__ unsigned long long total;
   __shared__ __align__(16) unsigned char sP_raw[sizeof(SimParams)];
   SimParams &sP = *reinterpret_cast<SimParams *>(sP_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < kWinNodes; i += kBlock) reinterpret_cast<int2 *>(win_rz)[i] = make_int2(0, 0);
+  if (threadIdx.x == 0) total = 0;
+  __syncthreads();
   // per-cell candidates (of the previous pass) and chunks, then prefix sums
   for (int c = threadIdx.x; c < ncell; c += kBlock) {
     const SimCounters *cc = cells[c].cnt;
     const long long step = cc->step;
     cand_pre[c + 1] = mode != 1 ? (long long)cc->n_cand[(int)(step & 1) ^ 1] : 0;
-    const long long n0 = (long long)cc->n_total;
-    const int chunk = cells[c].P[jb].chunk;
-    chunk_pre[c + 1] = (n0 + chunk - 1) / chunk;
+    chunk_pre[c + 1] = (long long)cc->n_total;
+    atomicAdd(&total, (unsigned long long)cc->n_total);
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < ncell; c += kBlock) {
+    const int fixed = cells[c].P[jb].chunk;
+    const int chunk = fixed ? fixed : even_chunk((unsigned)min(total, 0x7FFFFFFFull), gridDim.x, kChunkMax);
+    cell_chunk[c] = chunk;
+    chunk_pre[c + 1] = ((unsigned)chunk_pre[c + 1] + chunk - 1) / chunk;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -1797,8 +1817,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_batch_pass32(const BatchCell32 *_
       const SimParams &Pc = C.P[jb];
       const int ws = win_stride(Pc.nr), maxrows = min(kWinNodes / ws, Pc.nz);
       const long long n0c = (long long)C.cnt->n_total, chc = next - chunk_pre[next_c];
-      prefetch_chunk32(C.S[cur], chc * Pc.chunk, min((chc + 1) * Pc.chunk, n0c));
-      chunk_rows32(Pc, C.S[cur], n0c, Pc.chunk, chc, maxrows, next_row0, next_rows);
+      const int chunk = cell_chunk[next_c];
+      prefetch_chunk32(C.S[cur], chc * chunk, min((chc + 1) * chunk, n0c));
+      chunk_rows32(Pc, C.S[cur], n0c, chunk, chc, maxrows, next_row0, next_rows);
     }
   };
   if (threadIdx.x == 0) {
@@ -1844,7 +1865,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_batch_pass32(const BatchCell32 *_
     const BatchCell32 &C = cells[c];
     SimCounters *cc = C.cnt;
     const long long n0 = (long long)cc->n_total, step = cc->step;
-    const int chunk = sP.chunk;
+    const int chunk = cell_chunk[c];
     const long long ch = g - chunk_pre[c];
     const int beg = (int)(ch * chunk), end = (int)min((long long)beg + chunk, n0);
     const Win32 w{win_rz, win_row0, win_rows, win_stride(sP.nr)};
@@ -1924,6 +1945,7 @@ __device__ __forceinline__ void commit_pass32(SimCounters *cnt) {
   cnt->n_births = 0;
   cnt->n_cand[ns & 1] = 0;
   cnt->chunk_next = 0;
+  cnt->chunk = cnt->chunk_fixed ? cnt->chunk_fixed : even_chunk((unsigned)cnt->n_total, (unsigned)cnt->pass_blocks, kChunkMax);
   cnt->step = ns;
 }
 
@@ -2731,6 +2753,13 @@ int restart_steps(gasatt_sim *s, cudaStream_t st) {
   return GASATT_OK;
 }
 
+// the pass's chunk for the population in h (FP32; later the commits choose it)
+void set_chunk(const gasatt_sim *s, SimCounters &h) {
+  h.chunk_fixed = s->P.chunk;
+  h.pass_blocks = (int)s->pass_grid;
+  h.chunk = h.chunk_fixed ? h.chunk_fixed : even_chunk((unsigned)h.n_total, s->pass_grid, kChunkMax);
+}
+
 // A fresh population of n particles sits in state buffer 0: counters, current
 // buffers and the step bookkeeping start over.
 int sim_reset(gasatt_sim *s, int64_t n) {
@@ -2740,6 +2769,7 @@ int sim_reset(gasatt_sim *s, int64_t n) {
   zc.n_total = (unsigned long long)n;
   zc.step = -1;
   zc.cap = (unsigned long long)s->cfg.capacity;
+  set_chunk(s, zc);
   GASATT_CUDA(ctx, cudaMemcpyAsync(s->cnt, &zc, sizeof(zc), cudaMemcpyHostToDevice, st));
   for (int q = 0; q < 2; ++q) {
     GASATT_CUDA(ctx, cudaMemsetAsync(s->Jr[q], 0, jbytes(s), st));
@@ -3014,7 +3044,7 @@ int gasatt_sim_create(gasatt_ctx *ctx, const gasatt_sim_config *cfg, const gasat
   if (c.flags & ~(unsigned)(GASATT_Q_ER_END_COPY | GASATT_Q_EZ_AXIS_JSIGN | GASATT_Q_EZ_RSHIFT))
     return fail(ctx, GASATT_E_ARG, "the resident simulation accepts only the field quirk flags");
   if (c.pass_chunk < 0 || c.pass_chunk > kChunkMax || c.pass_chunk % kBlock)
-    return fail(ctx, GASATT_E_ARG, "pass_chunk: a multiple of 256 in [256, 1792] (0: 1792)");
+    return fail(ctx, GASATT_E_ARG, "pass_chunk: a multiple of 256 in [256, 1792] (0: by population)");
   if (c.fdtd_tile_rows < 0) return fail(ctx, GASATT_E_ARG, "fdtd_tile_rows: >= 0");
   if (c.gather < 0 || c.gather > 2) return fail(ctx, GASATT_E_ARG, "gather: 0 (auto), 1 (quads) or 2 (fields)");
   if (c.ion_capacity < 0 || (c.ion_capacity > 0 && (c.ion_subcycle < 1 || !(c.m_ion > 0) ||
@@ -3113,7 +3143,7 @@ int gasatt_sim_create(gasatt_ctx *ctx, const gasatt_sim_config *cfg, const gasat
   P.gas = nullptr;
   P.ion_sig = nullptr;
   P.Rp = nr * c.dr; P.Lp = nz * c.dz; P.kb = c.kb; P.m_ion = c.m_ion; P.T_gas = c.gas_temperature;
-  P.chunk = c.pass_chunk > 0 ? c.pass_chunk : kChunkMax;
+  P.chunk = c.pass_chunk;
   P.seed = c.seed; P.pk = philox_keys(c.seed); P.secondaries = c.secondaries; P.cap = cap;
   P.ion_cap = c.ion_capacity;
   P.ion_sigma = c.ion_capacity > 0 ? std::sqrt(c.kb * c.gas_temperature / c.m_ion) : 0.0;
@@ -3172,7 +3202,8 @@ int gasatt_sim_create(gasatt_ctx *ctx, const gasatt_sim_config *cfg, const gasat
   if (s->form == 1) {
     // FP32 blocks take chunks from a counter: no more blocks than chunks the
     // capacity can hold (small instances then leave the GPU to others)
-    const long long chunks = (cap + P.chunk - 1) / P.chunk;
+    const int least = P.chunk > 0 ? P.chunk : kBlock;
+    const long long chunks = (cap + least - 1) / least;
     if ((long long)s->pass_grid > chunks) s->pass_grid = (unsigned)(chunks > 0 ? chunks : 1);
   }
   // as many collision warps as fit on the device at once
@@ -3184,6 +3215,7 @@ int gasatt_sim_create(gasatt_ctx *ctx, const gasatt_sim_config *cfg, const gasat
   SimCounters z{};
   z.step = -1;
   z.cap = (unsigned long long)cap;
+  set_chunk(s, z);
   if (cudaMemcpy(s->cnt, &z, sizeof(z), cudaMemcpyHostToDevice) != cudaSuccess)
     return cleanup(fail(ctx, GASATT_E_CUDA, "counter init"));
   for (int k = 0; k < 2; ++k) {
@@ -3844,6 +3876,7 @@ int gasatt_sim_run_host(gasatt_sim *s, double *pos, double *vel, int64_t *n_io, 
   h.n_cand[0] = h.n_cand[1] = 0;
   h.uncommitted = 0;
   h.chunk_next = 0;
+  set_chunk(s, h);
   h.step += 1;                               // never reuse the last pass's step
   GASATT_CUDA(ctx, cudaMemcpyAsync(s->cnt, &h, sizeof(h), cudaMemcpyHostToDevice, st));
   for (int q = 0; q < 2; ++q) {

@@ -276,7 +276,9 @@ typedef struct gasatt_sim_config {
   int      fdtd_tile_rows;  /* rows of the field update's per-warp patch: 12, 16 or 20
                                (output 26 columns x rows - 6 per patch); default 12 */
   int      pass_chunk;      /* FP32 particle pass: particles per chunk a block takes,
-                               a multiple of 256 (256..1792); default 1792 */
+                               a multiple of 256 (256..1792); default: chosen every
+                               step so that the population fills all blocks evenly,
+                               at most 1792 */
   int      gather;          /* FP32 form, how the push reads E and H: 1 = packed 2 x 2
                                quads the field update writes beside the fields (three
                                16-byte loads per electron, 48 more bytes written per

@@ -57,3 +57,36 @@ def test_fp64_pass_matches_oracle(tables, nr, nz, n, spread):
     assert (d["n_ionizations"], d["n_elastic"], d["n_excitation"], d["n_null"], d["n_lost_wall"]) == \
         tuple(int(c) for c in orc.counters[:5])
     sim.close()
+
+
+# populations of one warp, around a block, around one chunk per block (592 x
+# 256 and 592 x 1792 electrons) and between; at 100 Torr 2% of the electrons are
+# collision candidates in each step, for idle and busy blocks alike
+@pytest.mark.parametrize("nr,nz,n", [(16, 20, 31), (16, 20, 257), (64, 64, 30_001), (64, 64, 151_553),
+                                     (64, 300, 400_000), (64, 300, 1_060_865)])
+def test_fp32_chunk_choice_changes_no_bit(nr, nz, n):
+    """The chunk chosen from the population and fixed chunks give the same state, fields and counts."""
+    parts = population(n, nr, nz, False, seed=n)
+    flds = grid_fields(nr, nz, np.random.default_rng(8), E0=3e6, H0=2e3)
+    flds[0][:, 0] = 0; flds[0][:, -1] = 0; flds[1][-1, :] = 0
+    ref = None
+    for chunk in (0, 256, 1792):
+        cfg = config(nr, nz, D, 1e-14, 100.0, precision=_lib.FP32_SPLIT, capacity=n + n // 4 + 100, seed=3,
+                     sort_period=3)
+        cfg.pass_chunk = chunk
+        sim = Sim(cfg)
+        sim.load(*parts)
+        sim.set_fields(*flds)
+        sim.step(7)
+        d, st = sim.diag(), sim.read()
+        a = st["r"] >= 0
+        o = np.argsort(st["id"][a], kind="stable")
+        got = [st[k][a][o] for k in ("id", "r", "z", "ur", "ut", "uz")] + list(sim.fields()) + list(sim.current())
+        got.append(np.array([d[k] for k in ("n_alive", "n_ionizations", "n_elastic", "n_excitation", "n_null",
+                                            "n_lost_wall", "collision_loss_ev")]))
+        sim.close()
+        if ref is None:
+            ref = got
+            assert d["n_alive"] > 0
+        for x, y in zip(got, ref):
+            np.testing.assert_array_equal(x, y)
