@@ -1452,79 +1452,65 @@ __device__ __forceinline__ void queue_one(SimCounters *cnt, int *queue, const Si
   queue[(long long)par * P.cap + (long long)k] = (int)p;
 }
 
-// A collision candidate of the previous step (FP32 form), taken by one lane:
+// A collision candidate of the previous step (FP32 form), taken by two lanes:
 // the MCC at the end of step `step` - 1 (FP64 test, branch, energy sharing;
-// float turn), the secondary's birth at the parent's position, then the push
-// of step `step` for both (push == true) with their current deposited by
-// global atomics and their own candidate test, or (push == false) nothing
-// more.  The chunk loop of the pass skips these particles (pending flag set,
+// float turn) by both, then the first lane goes on with the electron and the
+// second (kid) with its secondary, born at the parent's position.  PUSH: each
+// is pushed in step `step` (MODE as push32), its current deposited by global
+// atomics, with its own candidate test; otherwise nothing more.  The two pushes
+// share their instructions: one after the other in one lane, with the push of
+// every mode inlined, a pass whose chains are its critical path was 2 us
+// longer.  The chunk loop of the pass skips these particles (pending flag set,
 // or pushed-parity = this step's).
 // P: the launch's parameters in global memory (a reference to the kernel's
 // own parameter block would make every thread copy it to its stack).
+template <int MODE, bool PUSH>
 __device__ __noinline__ void candidate32(const SimParams *__restrict__ Pg, Fields<float> F,
                                          State32 S, SimCounters *cnt, int *queue, long long p,
-                                         long long step, int mode, bool push, long long n0,
-                                         unsigned &lost) {
+                                         long long step, bool kid, long long n0, unsigned &lost) {
   const SimParams &P = *Pg;
   const int par = (int)(step & 1);
-  const long long cstep = push ? step - 1 : step;      // step whose collision this is
+  const long long cstep = PUSH ? step - 1 : step;      // step whose collision this is
   const uint4 A = S.a[p];
   const float2 B = S.b[p];
-  const uint64_t id = S.id[p];
+  uint64_t id = S.id[p];
+  __syncwarp(3u << (threadIdx.x & 30));   // both lanes have read p before the first one writes it
   int ir = (int)(A.x & 0xFFFFu), iz = (int)(A.x >> 16);
   float fr = __uint_as_float(A.y & ~kSign), fz = __uint_as_float(A.z & ~kSign);
   double dux = (double)__uint_as_float(A.w) * P.c, duy = (double)B.x * P.c, duz = (double)B.y * P.c;
   Birth b;
   const int ev = mcc_event<true>(P, id, cstep, dux, duy, duz, b, gas_density(P, ir, iz));
-  count_event(cnt, ev, b);
-  if (ev == 2 && P.ion_cap > 0)
-    ion_birth(P.ion, P.ion_cap, ion_spread(P, ir, iz), P.seed, cnt, id, cstep, ((double)ir + (double)fr) * P.dr,
-              ((double)iz + (double)fz) * P.dz);
-  const int mark = push ? par : (int)(cstep & 1);
-  if (b.born) {
+  if (kid) {
+    if (!b.born) return;
     const unsigned long long kb = atomicAdd(&cnt->n_births, 1ull);
-    const long long slot = n0 + (long long)kb;
-    if (slot < P.cap) {
-      int cir = ir, ciz = iz;
-      float cfr = fr, cfz = fz;
-      float cur = (float)(b.ux / P.c), cut = (float)(b.uy / P.c), cuz = (float)(b.uz / P.c);
-      bool calive = true, cc = false;
-      const uint64_t cid = child_id(id, cstep);
-      if (push) {
-        float cig;
-        cc = mode == 0 ? push32<0>(P, F, cid, step, cir, ciz, cfr, cfz, cur, cut, cuz, calive, cig)
-           : mode == 1 ? push32<1>(P, F, cid, step, cir, ciz, cfr, cfz, cur, cut, cuz, calive, cig)
-                       : push32<2>(P, F, cid, step, cir, ciz, cfr, cfz, cur, cut, cuz, calive, cig);
-        if (calive && mode != 2) deposit_global32(P, cir, ciz, cfr, cfz, cur, cuz, cig);
-        if (!calive) {
-          lost++;
-          count_wall_loss(cnt, (double)cur * cur + (double)cut * cut + (double)cuz * cuz, P.me * P.c * P.c / P.qe);
-        }
-        if (cc) queue_one(cnt, queue, P, par, slot);
-      }
-      S.a[slot] = pack32(cir, ciz, cfr, cfz, cur, calive, cc, mark);
-      S.b[slot] = make_float2(cut, cuz);
-      S.id[slot] = cid;
-    } else {
+    p = n0 + (long long)kb;
+    if (p >= P.cap) {
       atomicAdd(&cnt->cap_overflow, 1ull);
+      return;
     }
+    id = child_id(id, cstep);
+    dux = b.ux; duy = b.uy; duz = b.uz;
+  } else {
+    count_event(cnt, ev, b);
+    if (ev == 2 && P.ion_cap > 0)
+      ion_birth(P.ion, P.ion_cap, ion_spread(P, ir, iz), P.seed, cnt, id, cstep, ((double)ir + (double)fr) * P.dr,
+                ((double)iz + (double)fz) * P.dz);
   }
   float ur = (float)(dux / P.c), ut = (float)(duy / P.c), uz = (float)(duz / P.c);
-  bool alive = true, pc = false;
-  if (push) {
-    float pig;
-    pc = mode == 0 ? push32<0>(P, F, id, step, ir, iz, fr, fz, ur, ut, uz, alive, pig)
-       : mode == 1 ? push32<1>(P, F, id, step, ir, iz, fr, fz, ur, ut, uz, alive, pig)
-                   : push32<2>(P, F, id, step, ir, iz, fr, fz, ur, ut, uz, alive, pig);
-    if (alive && mode != 2) deposit_global32(P, ir, iz, fr, fz, ur, uz, pig);
+  bool alive = true, cand = false;
+  if (PUSH) {
+    float ig;
+    cand = push32<MODE>(P, F, id, step, ir, iz, fr, fz, ur, ut, uz, alive, ig);
+    if (alive && MODE != 2) deposit_global32(P, ir, iz, fr, fz, ur, uz, ig);
     if (!alive) {
       lost++;
       count_wall_loss(cnt, (double)ur * ur + (double)ut * ut + (double)uz * uz, P.me * P.c * P.c / P.qe);
     }
-    if (pc) queue_one(cnt, queue, P, par, p);
+    if (cand) queue_one(cnt, queue, P, par, p);
   }
-  S.a[p] = pack32(ir, iz, fr, fz, ur, alive, pc, mark);
+  S.a[p] = pack32(ir, iz, fr, fz, ur, alive, cand, PUSH ? par : (int)(cstep & 1));
   S.b[p] = make_float2(ut, uz);
+  if (kid) S.id[p] = id;
 }
 
 // Window rows of chunk ch (particles [ch chunk, min(ch chunk + chunk, n0))):
@@ -1665,7 +1651,7 @@ constexpr int kCandLanes = 8;     // collision candidates a warp of the pass tak
 
 // FP32 particle pass of step `step` (modes as push32).  Its blocks first take
 // the collision candidates queued by the previous pass, kCandLanes per warp,
-// one per lane (a long serial chain each; a warp's chains share its issue but
+// two lanes each (a long serial chain; a warp's chains share its issue but
 // serialise their different collision branches, so a few per warp, not 32,
 // keep the longest warp short), then all other particles in chunks of
 // P.chunk handed out in order, so the blocks that ran candidates simply take
@@ -1690,7 +1676,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_pass32(SimParams P, State32 S, Fi
   const int maxrows = min(kWinNodes / ws, P.nz);
   const int chunk = max(cnt->chunk, kBlock);      // chosen with the commit (no division here)
   if (mode != 1) {
-    // The candidates go to the last blocks, kCandLanes per warp, one per lane;
+    // The candidates go to the last blocks, kCandLanes per warp, two lanes each;
     // where there are fewer chunks than blocks, to the warps of all blocks that
     // would otherwise be idle, fewer per warp.  A block takes its chunks after
     // its candidates.
@@ -1702,10 +1688,10 @@ __global__ void __launch_bounds__(kBlock, 4) k_pass32(SimParams P, State32 S, Fi
       lanes = (int)min(((unsigned)nq + idle - 1) / idle, (unsigned)kCandLanes);
     }
     unsigned lost = 0;
-    if (lane < lanes)
-      for (long long k = ((long long)(gridDim.x - 1 - blockIdx.x) * (kBlock / 32) + warp) * lanes + lane; k < nq;
+    if (lane < 2 * lanes)
+      for (long long k = ((long long)(gridDim.x - 1 - blockIdx.x) * (kBlock / 32) + warp) * lanes + (lane >> 1); k < nq;
            k += (long long)gridDim.x * (kBlock / 32) * lanes)
-        candidate32(Pg, F, S, cnt, queue, qin[k], step, mode, true, n0, lost);
+        candidate32<MODE, true>(Pg, F, S, cnt, queue, qin[k], step, lane & 1, n0, lost);
     if (lost) atomicAdd(&cnt->lost, (unsigned long long)lost);
   }
   // thread 0 claims the block's next chunk (index and window rows) a chunk
@@ -1827,17 +1813,17 @@ __global__ void __launch_bounds__(kBlock, 4) k_batch_pass32(const BatchCell32 *_
     resolve();
     cell_at = -1;
   }
-  // one candidate per lane (the chains of a warp share its instruction issue)
-  for (long long k = ((long long)blockIdx.x * (kBlock / 32) + warp) * 32 + lane; k < nq;
-       k += (long long)gridDim.x * kBlock) {
+  // one candidate per two lanes (the chains of a warp share its instruction issue)
+  for (long long k = (((long long)blockIdx.x * (kBlock / 32) + warp) * 32 + lane) >> 1; k < nq;
+       k += (long long)gridDim.x * (kBlock / 2)) {
     const int c = cell_of_item(cand_pre, ncell, k);
     const BatchCell32 &C = cells[c];
     SimCounters *cc = C.cnt;
     const long long step = cc->step;
     const int *qin = C.queue + (long long)((int)(step & 1) ^ 1) * C.P[jb].cap;
     unsigned lost = 0;
-    candidate32(&C.P[jb], C.F[jb], C.S[cur], cc, C.queue, qin[k - cand_pre[c]], step, mode, true,
-                (long long)cc->n_total, lost);
+    candidate32<mode, true>(&C.P[jb], C.F[jb], C.S[cur], cc, C.queue, qin[k - cand_pre[c]], step, lane & 1,
+                            (long long)cc->n_total, lost);
     if (lost) atomicAdd(&cc->lost, (unsigned long long)lost);
   }
   for (;;) {
@@ -1889,14 +1875,14 @@ __global__ void __launch_bounds__(kMccBlock) k_collide32(const SimParams *__rest
   const long long nq = (long long)cnt->n_cand[par];
   const int *qu = queue + (long long)par * P.cap;
   unsigned lost = 0;              // (no push here: nothing reaches the wall)
-  for (long long k = blockIdx.x * (long long)kMccBlock + threadIdx.x; k < nq;
-       k += (long long)gridDim.x * kMccBlock)
-    candidate32(Pg, F, S, cnt, queue, qu[k], step, 0, false, n0, lost);
+  for (long long k = (blockIdx.x * (long long)kMccBlock + threadIdx.x) >> 1; k < nq;
+       k += (long long)gridDim.x * (kMccBlock / 2))
+    candidate32<0, false>(Pg, F, S, cnt, queue, qu[k], step, threadIdx.x & 1, n0, lost);
 }
 
 // k_collide32 for every cell of a batch in one launch (before the batch's
-// sort): the cells' queued collisions in one range by prefix sums, one per
-// lane; each cell's are those its own k_collide32 would apply.
+// sort): the cells' queued collisions in one range by prefix sums, two lanes
+// each; each cell's are those its own k_collide32 would apply.
 __global__ void __launch_bounds__(kMccBlock) k_batch_collide32(const BatchCell32 *__restrict__ cells,
                                                                int ncell, int cur) {
   __shared__ long long pre[kMaxBatch + 1];
@@ -1911,16 +1897,16 @@ __global__ void __launch_bounds__(kMccBlock) k_batch_collide32(const BatchCell32
   }
   __syncthreads();
   const long long nq = pre[ncell];
-  for (long long k = blockIdx.x * (long long)kMccBlock + threadIdx.x; k < nq;
-       k += (long long)gridDim.x * kMccBlock) {
+  for (long long k = (blockIdx.x * (long long)kMccBlock + threadIdx.x) >> 1; k < nq;
+       k += (long long)gridDim.x * (kMccBlock / 2)) {
     const int c = cell_of_item(pre, ncell, k);
     const BatchCell32 &C = cells[c];
     SimCounters *cc = C.cnt;
     const long long step = cc->step;
     const int *qu = C.queue + (long long)(int)(step & 1) * C.P[0].cap;
     unsigned lost = 0;
-    candidate32(&C.P[0], C.F[0], C.S[cur], cc, C.queue, qu[k - pre[c]], step, 0, false,
-                (long long)cc->n_total, lost);
+    candidate32<0, false>(&C.P[0], C.F[0], C.S[cur], cc, C.queue, qu[k - pre[c]], step, threadIdx.x & 1,
+                          (long long)cc->n_total, lost);
   }
 }
 
