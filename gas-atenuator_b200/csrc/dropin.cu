@@ -2,7 +2,9 @@
 //   find_CS0, free_motion, particle_density, electricmagneticfield6
 //   (EM2 + EM7 + EM3_1 + EM3 + EM4), electron_collision (electron_transport).
 // Plain FP64 on the MATLAB column-major arrays; compiled with -fmad=false so
-// the arithmetic follows the reference expression by expression.
+// the arithmetic follows the reference expression by expression, but for
+// electricmagneticfield6, whose particle step multiplies by reciprocals and
+// uses explicit FMAs.
 #include <cub/device/device_scan.cuh>
 #include <cmath>
 #include <cstring>
@@ -203,6 +205,13 @@ int density_counts_on_device(gasatt_ctx *ctx, unsigned long long **out) {
 }
 
 // -------------------------------------------- electricmagneticfield6 path
+// Per particle step one field sub-cycle (k_em_fields) and one particle kernel
+// (k_em_push: kick and second half drift of the step, first half drift and
+// deposit of the next), where one launch per reference kernel took 26.  The
+// push multiplies by reciprocals and takes the sine and cosine of the azimuth
+// from x / r and y / r; its particles are not sorted, so it waits on scattered
+// gathers and global atomics.  100 x 500 cells, 260,000 particles: push 27 us,
+// fields 11 us; in 26 launches a step took 165 us.
 struct Species {
   double *pos[3], *vel[3];
   int64_t n[3];
@@ -210,110 +219,332 @@ struct Species {
 };
 
 struct EmState {
-  double *x, *y, *z, *vx, *vy, *vz, *r, *phi, *vr, *q, *m, *E;
+  double *x, *y, *z, *vx, *vy, *vz, *E;
   int *del;
+};
+
+struct EmParams {
+  double Rp, Lp, PHIp, cP, sP, hdt;       // hdt: half the particle step
+  double id, mu, c, ic2, FN, scale;       // id: 1 / cell size
+  double q[3], m[3], qm[3], qm_dt[3];     // per species: charge, mass, q/m, q/m x particle step
+  int nr, nz;
+  int wrap;                               // azimuth: 0 full ring, 1 wedge of at most pi/2, 2 any other wedge
+  bool atan_phi, euler, fast_fx;          // fast_fx: |fixed-point contribution| <= 2^50
+  unsigned long long *Jr, *Jz;            // deposit target
 };
 
 __device__ __forceinline__ int species_of(const Species &s, int64_t o) {
   return o >= s.start[2] ? 2 : (o >= s.start[1] ? 1 : 0);
 }
 
-// electricmagneticfield6.m:65-73, 113-118: concatenate the three species
-__global__ void k_em_load(Species sp, EmState st, int64_t N, double e, double m_e, double m_i,
-                          unsigned flags) {
-  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < N;
-       o += (int64_t)gridDim.x * blockDim.x) {
-    const int s = species_of(sp, o);
-    const int64_t i = o - sp.start[s], ld = sp.n[s];
-    const double p0 = sp.pos[s][i], p1 = sp.pos[s][ld + i], p2 = sp.pos[s][2 * ld + i];
-    if (flags & GASATT_POS_IN_CYL) { st.x[o] = p0 * cos(p1); st.y[o] = p0 * sin(p1); }
-    else { st.x[o] = p0; st.y[o] = p1; }
-    st.z[o] = p2;
-    st.vx[o] = sp.vel[s][i]; st.vy[o] = sp.vel[s][ld + i]; st.vz[o] = sp.vel[s][2 * ld + i];
-    st.q[o] = s == 0 ? -e : (s == 1 ? e : 2 * e);
-    st.m[o] = s == 0 ? m_e : m_i;
-    st.r[o] = 0; st.phi[o] = 0; st.vr[o] = 0; st.E[o] = 0;
-    st.del[o] = 0;
-  }
-}
-
-// EM2.cu:23-57 then EM7.cu:51-202 for the same particle (the deposit of a
-// particle needs only its own EM2 result)
-__global__ void k_em2_deposit(EmState st, int64_t N, double Rp, double Lp, double PHIp,
-                              double dt, int nr, int nz, double dr, double dz, double FN,
-                              double scale, unsigned long long *Jr, unsigned long long *Jz,
-                              unsigned flags) {
-  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < N;
-       o += (int64_t)gridDim.x * blockDim.x) {
-    if (st.del[o] == 1) continue;
-    double x = st.x[o], y = st.y[o], z = st.z[o], vx = st.vx[o], vy = st.vy[o], vz = st.vz[o];
-    double r, phi;
-    int del = 0;
-    halfdrift_cart(x, y, z, vx, vy, vz, vx, vy, vz, r, phi, del, Rp, Lp, PHIp, dt, flags);
-    const double vr = vx * cos(phi) + vy * sin(phi);
-    st.x[o] = x; st.y[o] = y; st.z[o] = z; st.vx[o] = vx; st.vy[o] = vy; st.vz[o] = vz;
-    st.r[o] = r; st.phi[o] = phi; st.vr[o] = vr;
-    if (del) { st.del[o] = 1; continue; }
-    int64_t a[4]; double b[4];
-    em7_weights(r, z, nr, nz, dr, dz, a, b);
-    const double q = st.q[o];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      fx_add(Jr, a[k], FN * b[k] * q * vr, scale);
-      fx_add(Jz, a[k], FN * b[k] * q * vz, scale);
+// EM2.cu:26-57 / EM4.cu:146-177: drift by half a step, delete beyond Rp, wrap
+// the azimuth into the wedge turning the velocity with it, reflect at z = 0
+// and Lp.  (c, s): cosine and sine of the new azimuth.  On a wedge of at most
+// pi/2 the tests phi < 0 and phi > PHIp are the signs of sin(phi) and
+// sin(phi - PHIp); atan(y/x) (atan_phi) is the azimuth of (|x|, y sign(x)).
+__device__ __forceinline__ void em_halfdrift(const EmParams &g, double &x, double &y, double &z, double &vx,
+                                             double &vy, double &vz, double &r, double &c, double &s,
+                                             bool &del) {
+  const double X = fma(g.hdt, vx, x), Y = fma(g.hdt, vy, y);
+  double Z = fma(g.hdt, vz, z);
+  r = sqrt(fma(X, X, Y * Y));
+  const double ir = 1 / r;
+  if (r > g.Rp) del = true;
+  if (g.wrap == 2) {
+    double phi = g.atan_phi ? atan(Y / X) : atan2(Y, X);
+    // bounded: a wrap count above 2^20 means phi is not finite-sized
+    for (int it = 0; phi < 0 && it < (1 << 20); ++it) {
+      phi = phi + g.PHIp;
+      const double w = vx * g.cP - vy * g.sP;
+      vy = vx * g.sP + vy * g.cP;
+      vx = w;
     }
-  }
-}
-
-// EM4.cu:33-177
-__global__ void k_em4(EmState st, int64_t N, const double *Er, const double *Ez, const double *H,
-                      double Rp, double Lp, double PHIp, int nr, int nz, double mu, double c,
-                      double dr, double dz, double dt, unsigned flags) {
-  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < N;
-       o += (int64_t)gridDim.x * blockDim.x) {
-    if (st.del[o] == 1) continue;
-    double Er0, Ez0, H0;
-    gather3<double>(Er, Ez, H, nr, nz, dr, dz, st.r[o], st.z[o], Er0, Ez0, H0);
-    const double vx = st.vx[o], vy = st.vy[o], vz = st.vz[o], q = st.q[o], m = st.m[o];
-    const double phi = st.phi[o];
-    double gamma = 1 / sqrt(1 - (vx * vx + vy * vy + vz * vz) / (c * c));
-    double ux, uy, uz;
-    if (flags & GASATT_Q_EULER_KICK) {
-      const double Fr = q * (Er0 + (-vz * H0 * mu));
-      const double Fz = q * (Ez0 + (st.vr[o] * H0 * mu));
-      const double Fx = Fr * cos(phi), Fy = Fr * sin(phi);
-      ux = gamma * vx + Fx / m * dt;
-      uy = gamma * vy + Fy / m * dt;
-      uz = gamma * vz + Fz / m * dt;
+    for (int it = 0; phi > g.PHIp && it < (1 << 20); ++it) {
+      phi = phi - g.PHIp;
+      const double w = vx * g.cP + vy * g.sP;
+      vy = -vx * g.sP + vy * g.cP;
+      vx = w;
+    }
+    sincos(phi, &s, &c);
+  } else {
+    if (g.atan_phi) {
+      c = fabs(X) * ir;
+      s = (signbit(X) ? -Y : Y) * ir;
     } else {
-      const double cp = cos(phi), sp = sin(phi);
-      ux = gamma * vx; uy = gamma * vy; uz = gamma * vz;
-      const double B = mu * H0;
-      boris(ux, uy, uz, Er0 * cp, Er0 * sp, Ez0, -B * sp, B * cp, 0.0, q / m * dt / 2, c);
+      c = r > 0 ? X * ir : 1.0;
+      s = r > 0 ? Y * ir : 0.0;
     }
-    gamma = sqrt(1 + (ux * ux + uy * uy + uz * uz) / (c * c));
-    st.E[o] = (gamma - 1) * m * c * c;
-    double nvx = ux / gamma, nvy = uy / gamma, nvz = uz / gamma;
-    double x = st.x[o], y = st.y[o], z = st.z[o], r, ph;
-    int del = 0;
-    halfdrift_cart(x, y, z, nvx, nvy, nvz, nvx, nvy, nvz, r, ph, del, Rp, Lp, PHIp, dt, flags);
+    if (g.wrap) {
+      for (int it = 0; s < 0 && it < (1 << 20); ++it) {
+        const double k = c * g.cP - s * g.sP;
+        s = c * g.sP + s * g.cP;
+        c = k;
+        const double w = vx * g.cP - vy * g.sP;
+        vy = vx * g.sP + vy * g.cP;
+        vx = w;
+      }
+      for (int it = 0; s * g.cP - c * g.sP > 0 && it < (1 << 20); ++it) {
+        const double k = c * g.cP + s * g.sP;
+        s = -c * g.sP + s * g.cP;
+        c = k;
+        const double w = vx * g.cP + vy * g.sP;
+        vy = -vx * g.sP + vy * g.cP;
+        vx = w;
+      }
+    }
+  }
+  x = r * c;
+  y = r * s;
+  if (Z > g.Lp) { Z = 2 * g.Lp - Z; vz = -vz; }
+  if (Z < 0) { Z = -Z; vz = -vz; }
+  z = Z;
+}
+
+// EM7.cu:51-202: q FN v w of a particle at (r, z) into its four nodes, in fixed point
+__device__ __forceinline__ void em_deposit(const EmParams &g, double r, double z, double vr, double vz,
+                                           double q) {
+  const Axis64 R = axis64(r * g.id, g.nr), Z = axis64(z * g.id, g.nz);
+  const double k = g.FN * q * g.scale, kr = k * vr, kz = k * vz;
+#pragma unroll
+  for (int n = 0; n < 4; ++n) {
+    const int64_t a = (n & 1 ? R.hi : R.lo) + (int64_t)(n & 2 ? Z.hi : Z.lo) * g.nr;
+    const double b = (n & 1 ? R.w : 1 - R.w) * (n & 2 ? Z.w : 1 - Z.w);
+    long long vr_fx, vz_fx;
+    if (g.fast_fx) {
+      vr_fx = __double_as_longlong(fma(kr, b, 6755399441055744.0)) - 0x4338000000000000LL;
+      vz_fx = __double_as_longlong(fma(kz, b, 6755399441055744.0)) - 0x4338000000000000LL;
+    } else {
+      vr_fx = __double2ll_rn(kr * b);
+      vz_fx = __double2ll_rn(kz * b);
+    }
+    if (vr_fx) atomicAdd(g.Jr + a, (unsigned long long)vr_fx);
+    if (vz_fx) atomicAdd(g.Jz + a, (unsigned long long)vz_fx);
+  }
+}
+
+// the first half drift of a step and its deposit (EM2.cu, EM7.cu)
+__device__ __forceinline__ void em_first_half(const EmParams &g, double &x, double &y, double &z, double &vx,
+                                              double &vy, double &vz, double q, bool &del) {
+  double r, c, s;
+  em_halfdrift(g, x, y, z, vx, vy, vz, r, c, s, del);
+  if (!del) em_deposit(g, r, z, fma(vx, c, vy * s), vz, q);
+}
+
+// electricmagneticfield6.m:65-73, 113-118: concatenate the three species; with
+// steps to take, the first half drift and deposit
+__global__ void k_em_load(Species sp, EmState st, EmParams g, int64_t N, bool cyl, bool steps) {
+  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < N;
+       o += (int64_t)gridDim.x * blockDim.x) {
+    const int k = species_of(sp, o);
+    const int64_t i = o - sp.start[k], ld = sp.n[k];
+    double x = sp.pos[k][i], y = sp.pos[k][ld + i], z = sp.pos[k][2 * ld + i];
+    if (cyl) {
+      double c, s;
+      sincos(y, &s, &c);
+      y = x * s;
+      x = x * c;
+    }
+    double vx = sp.vel[k][i], vy = sp.vel[k][ld + i], vz = sp.vel[k][2 * ld + i];
+    bool del = false;
+    if (steps) em_first_half(g, x, y, z, vx, vy, vz, g.q[k], del);
     st.x[o] = x; st.y[o] = y; st.z[o] = z;
-    st.vx[o] = nvx; st.vy[o] = nvy; st.vz[o] = nvz;
-    st.r[o] = r; st.phi[o] = ph;
+    st.vx[o] = vx; st.vy[o] = vy; st.vz[o] = vz;
+    st.E[o] = 0;
+    st.del[o] = del;
+  }
+}
+
+// EM4.cu:33-177, then (more steps to come) EM2.cu and EM7.cu of the next step
+template <bool LAST>
+__global__ void __launch_bounds__(kBlock) k_em_push(Species sp, EmState st, EmParams g, int64_t N,
+                                                    const double *__restrict__ Er,
+                                                    const double *__restrict__ Ez,
+                                                    const double *__restrict__ H) {
+  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < N;
+       o += (int64_t)gridDim.x * blockDim.x) {
+    if (st.del[o]) continue;
+    const int k = species_of(sp, o);
+    double x = st.x[o], y = st.y[o], z = st.z[o], vx = st.vx[o], vy = st.vy[o], vz = st.vz[o];
+    double r = sqrt(fma(x, x, y * y));
+    const double ir = 1 / r;
+    double c = x * ir, s = y * ir;
+    if (!g.atan_phi && !(r > 0)) { c = 1; s = 0; }
+    // the staggered bilinear gather (EM4.cu:41-122), one-sided at the edges
+    const Axis64 R = axis64(r * g.id, g.nr), Z = axis64(z * g.id, g.nz);
+    const double *e0 = Er + (int64_t)Z.i * g.nr, *e1 = e0 + g.nr;
+    const double *z0 = Ez + (int64_t)Z.lo * (g.nr + 1) + R.i, *z1 = Ez + (int64_t)Z.hi * (g.nr + 1) + R.i;
+    const double *h0 = H + (int64_t)Z.lo * g.nr, *h1 = H + (int64_t)Z.hi * g.nr;
+    const double Er0 = lerp64(lerp64(e0[R.lo], e0[R.hi], R.w), lerp64(e1[R.lo], e1[R.hi], R.w), Z.f);
+    const double Ez0 = lerp64(lerp64(z0[0], z0[1], R.f), lerp64(z1[0], z1[1], R.f), Z.w);
+    const double H0 = lerp64(lerp64(h0[R.lo], h0[R.hi], R.w), lerp64(h1[R.lo], h1[R.hi], R.w), Z.w);
+    const double g0 = rsqrt(1 - (vx * vx + vy * vy + vz * vz) * g.ic2);
+    double ux = g0 * vx, uy = g0 * vy, uz = g0 * vz;
+    if (g.euler) {
+      const double B = H0 * g.mu, vr = vx * c + vy * s;
+      const double fr = g.qm_dt[k] * (Er0 - vz * B);
+      ux = fma(fr, c, ux);
+      uy = fma(fr, s, uy);
+      uz = fma(g.qm_dt[k], Ez0 + vr * B, uz);
+    } else {
+      const double B = g.mu * H0;
+      boris(ux, uy, uz, Er0 * c, Er0 * s, Ez0, -B * s, B * c, 0.0, 0.5 * g.qm_dt[k], g.c);
+    }
+    const double u2 = 1 + (ux * ux + uy * uy + uz * uz) * g.ic2;
+    if (LAST) st.E[o] = (sqrt(u2) - 1) * g.m[k] * g.c * g.c;
+    const double ig = rsqrt(u2);
+    vx = ux * ig; vy = uy * ig; vz = uz * ig;
+    bool del = false;
+    em_halfdrift(g, x, y, z, vx, vy, vz, r, c, s, del);
+    if (!LAST && !del) em_first_half(g, x, y, z, vx, vy, vz, g.q[k], del);
+    st.x[o] = x; st.y[o] = y; st.z[o] = z;
+    st.vx[o] = vx; st.vy[o] = vy; st.vz[o] = vz;
     if (del) st.del[o] = 1;
   }
 }
 
-__global__ void k_keep_flags(const int *del, int64_t N, int *keep) {
-  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o <= N;
-       o += (int64_t)gridDim.x * blockDim.x)
-    keep[o] = (o < N && del[o] == 0) ? 1 : 0;
+// `pairs` H and E updates of the field sub-cycle (EM3_1.cu:2-17, EM3.cu:2-43;
+// electricmagneticfield6.m:146-151 calls ten pairs between a first and a last
+// H update of dt/4) in one launch, from one set of fields to another: a block
+// of kEmWarps warps owns a patch of 32 columns (a lane each) x kEmRows rows,
+// each warp kEmSeg consecutive rows in registers.  Horizontal neighbours are
+// shuffles, vertical ones registers, and between warps one row in shared
+// memory per update.  An E update reads one column and row below, an H update one above,
+// so `pairs` columns and rows on the low side and pairs + 1 on the high side of
+// a patch are recomputed by its neighbours instead of exchanged.  Points outside the grid
+// take the same expressions on zeros; no point inside reads them
+// (fdtd_warp_body has the same rules).  The first H update takes h_first, the
+// others dt/2; a last one takes h_last (0: none).
+constexpr int kEmWarps = 8, kEmSeg = 8, kEmRows = kEmWarps * kEmSeg;
+constexpr int kEmOneLaunch = 148;        // tiles of one launch at most (see gasatt_electricmagneticfield6)
+
+struct EmFields { const double *Er, *Ez, *H; double *oEr, *oEz, *oH; };
+
+struct EmFieldParams {
+  int nr, nz, pairs;
+  double delta, PHIp, inv_scale, dt_eps, dt_eps_dz, axis;
+  double h_first, h_mid, h_last;          // h / (mu delta)
+  bool endcopy, jsign, rshift;
+};
+
+__host__ __device__ inline int em_tile_cols(int pairs) { return 32 - 2 * pairs - 1; }
+__host__ __device__ inline int em_tile_rows(int pairs) { return kEmRows - 2 * pairs - 1; }
+
+__global__ void __launch_bounds__(32 * kEmWarps) k_em_fields(EmFields f, EmFieldParams P,
+                                                             const unsigned long long *__restrict__ Jr,
+                                                             const unsigned long long *__restrict__ Jz,
+                                                             unsigned long long *__restrict__ Jr_next,
+                                                             unsigned long long *__restrict__ Jz_next) {
+  constexpr unsigned FULL = 0xFFFFFFFFu;
+  constexpr int S = kEmSeg;
+  // the rows of a segment its neighbours read: first and last Er, last H
+  // (the Er rows in two buffers by turns: an E update reads one while others write the other)
+  __shared__ double s_first[2][kEmWarps][32], s_last[2][kEmWarps][32], s_h[kEmWarps][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int nr = P.nr, nz = P.nz;
+  const int col = (int)blockIdx.x * em_tile_cols(P.pairs) - P.pairs + lane;
+  const int y0 = (int)blockIdx.y * em_tile_rows(P.pairs) - P.pairs + w * S;     // the segment's first row
+  const bool in = col >= 0 && col < nr;
+  double iv = 0, ezp = 0, ezm = 0;        // coefficients of EM3.cu; Ez at column n_r stays as it is
+  if (in) {
+    iv = P.inv_scale / shell_volume(col, P.delta, P.delta, P.PHIp);
+    const double ri = (P.rshift ? col + 1 : col) * P.delta, id = 1 / P.delta;
+    ezp = col == 0 ? P.axis : P.dt_eps * (1 / (2 * ri) + id);
+    ezm = col == 0 ? 0.0 : P.dt_eps * (1 / (2 * ri) - id);
+  }
+  double er[S], ez[S], h[S], jr[S], jz[S];
+  {
+    auto current = [&](const unsigned long long *J, int j) {
+      return in && j >= 0 && j < nz ? (double)(long long)J[col + (int64_t)j * nr] * iv : 0.0;
+    };
+    double below = current(Jr, y0 - 1);
+#pragma unroll
+    for (int r = 0; r < S; ++r) {
+      const int j = y0 + r;
+      const bool row = j >= 0 && j < nz;
+      er[r] = in && j >= 0 && j <= nz ? f.Er[col + (int64_t)j * nr] : 0.0;
+      ez[r] = col >= 0 && col <= nr && row ? f.Ez[col + (int64_t)j * (nr + 1)] : 0.0;
+      h[r] = in && row ? f.H[col + (int64_t)j * nr] : 0.0;
+      const double a = current(Jr, j);
+      jr[r] = P.dt_eps * (below + a) / 2;
+      below = a;
+      jz[r] = current(Jz, j);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < S; ++r) {
+    const double left = __shfl_up_sync(FULL, jz[r], 1);
+    jz[r] = col == 0 ? (P.jsign ? -(P.dt_eps * jz[r]) : P.dt_eps * jz[r]) : in ? P.dt_eps * (left + jz[r]) / 2 : 0.0;
+  }
+  const int up = min(w + 1, kEmWarps - 1), dn = max(w - 1, 0);
+  const int r0 = -y0, rn = nz - y0;       // the end rows 0 and n_z of Er in this segment
+  auto publish_e = [&](int b) {
+    s_first[b][w][lane] = er[0];
+    s_last[b][w][lane] = er[S - 1];
+    __syncthreads();
+  };
+  auto h_update = [&](double k, int b) {
+    const double above = s_first[b][up][lane];
+#pragma unroll
+    for (int r = 0; r < S; ++r) {
+      const double right = __shfl_down_sync(FULL, ez[r], 1);
+      const double e1 = r + 1 < S ? er[r + 1 < S ? r + 1 : r] : above;
+      h[r] = fma(k, (right - ez[r]) - (e1 - er[r]), h[r]);
+    }
+  };
+  auto e_update = [&](int b) {
+    const double below = s_h[dn][lane], er_up = s_first[b][up][lane], er_dn = s_last[b][dn][lane];
+    double ne[S];
+#pragma unroll
+    for (int r = 0; r < S; ++r) {
+      const double left = __shfl_up_sync(FULL, h[r], 1), hl = col > 0 ? left : 0.0;
+      const double hb = r > 0 ? h[r > 0 ? r - 1 : 0] : below;
+      ne[r] = fma(-P.dt_eps_dz, h[r] - hb, er[r] - jr[r]);
+      if (in) ez[r] = fma(ezm, hl, fma(ezp, h[r], ez[r] - jz[r]));
+    }
+    if ((r0 >= 0 && r0 < S) || (rn >= 0 && rn < S)) {
+#pragma unroll
+      for (int r = 0; r < S; ++r) {
+        if (r == r0) ne[r] = P.endcopy ? (r + 1 < S ? er[r + 1 < S ? r + 1 : r] : er_up) : 0.0;
+        if (r == rn) ne[r] = P.endcopy ? (r > 0 ? er[r > 0 ? r - 1 : 0] : er_dn) : 0.0;
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < S; ++r) er[r] = ne[r];
+  };
+  publish_e(0);
+  for (int p = 0; p < P.pairs; ++p) {
+    h_update(p == 0 ? P.h_first : P.h_mid, p & 1);
+    s_h[w][lane] = h[S - 1];
+    __syncthreads();
+    e_update(p & 1);
+    publish_e((p & 1) ^ 1);
+  }
+  if (P.h_last != 0) h_update(P.h_last, P.pairs & 1);
+  // write the tile back, and clear it in the next deposit's current
+  if (lane < P.pairs || lane >= 32 - P.pairs - 1 || col > nr) return;
+#pragma unroll
+  for (int r = 0; r < S; ++r) {
+    const int j = y0 + r, pr = w * S + r;
+    if (pr < P.pairs || pr >= kEmRows - P.pairs - 1 || j > nz) continue;
+    const int64_t a = col + (int64_t)j * nr;
+    if (in) f.oEr[a] = er[r];
+    if (j < nz) {
+      f.oEz[col + (int64_t)j * (nr + 1)] = ez[r];
+      if (in) {
+        f.oH[a] = h[r];
+        Jr_next[a] = 0;
+        Jz_next[a] = 0;
+      }
+    }
+  }
 }
 
-// electricmagneticfield6.m:168-188 with each species compacted by its own
-// delete flags; pos[] is the exclusive scan of the keep flags (N+1 entries)
+// counts[0..3]: the scan at the species' starts and the end; electricmagneticfield6.m:168-188
+// with each species compacted by its own delete flags; pos[] is the exclusive
+// scan of the keep flags (N+1 entries)
 __global__ void k_em_store(Species sp, EmState st, int64_t N, const int *pos, double *kin,
-                           double e) {
+                           double e, int *counts) {
+  if (blockIdx.x == 0 && threadIdx.x < 4) counts[threadIdx.x] = pos[threadIdx.x < 3 ? sp.start[threadIdx.x] : N];
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < N;
        o += (int64_t)gridDim.x * blockDim.x) {
     if (st.del[o]) continue;
@@ -323,6 +554,12 @@ __global__ void k_em_store(Species sp, EmState st, int64_t N, const int *pos, do
     sp.vel[s][w] = st.vx[o]; sp.vel[s][ld + w] = st.vy[o]; sp.vel[s][2 * ld + w] = st.vz[o];
     if (s == 0 && kin) kin[w] = st.E[o] / (1000 * e);
   }
+}
+
+__global__ void k_keep_flags(const int *del, int64_t N, int *keep) {
+  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o <= N;
+       o += (int64_t)gridDim.x * blockDim.x)
+    keep[o] = (o < N && del[o] == 0) ? 1 : 0;
 }
 
 // ------------------------------------------------------- electron_collision
@@ -716,20 +953,24 @@ int gasatt_electricmagneticfield6(gasatt_ctx *ctx, double *e_pos, double *e_vel,
     return fail(ctx, GASATT_E_ARG, "electricmagneticfield6: grid must be Rp/delta x Lp/delta");
   GASATT_CUDA(ctx, cudaSetDevice(ctx->device));
   const int64_t N = n_e + n_i1 + n_i2;
-  const int64_t ncel = (int64_t)n_r * n_z;
+  const size_t ncel = (size_t)n_r * n_z, nEr = (size_t)n_r * (n_z + 1), nEz = (size_t)(n_r + 1) * n_z;
   const size_t sc = scan_tmp_bytes(N + 1);
-  const size_t bytes = 12 * align256((size_t)(N + 1) * 8) + 3 * align256((size_t)(N + 1) * 4) +
-                       2 * align256((size_t)ncel * 8) + align256(sc);
+  const size_t bytes = 7 * align256((size_t)(N + 1) * 8) + 3 * align256((size_t)(N + 1) * 4) +
+                       4 * align256(ncel * 8) + align256(nEr * 8) + align256(nEz * 8) + align256(ncel * 8) +
+                       align256(16) + align256(sc);
   void *buf;
   int st = scratch(ctx, bytes, &buf);
   if (st) return st;
   Carver cv{(char *)buf};
   EmState s;
-  double **f[12] = {&s.x, &s.y, &s.z, &s.vx, &s.vy, &s.vz, &s.r, &s.phi, &s.vr, &s.q, &s.m, &s.E};
-  for (int i = 0; i < 12; ++i) *f[i] = cv.take<double>(N + 1);
+  double **f[7] = {&s.x, &s.y, &s.z, &s.vx, &s.vy, &s.vz, &s.E};
+  for (int i = 0; i < 7; ++i) *f[i] = cv.take<double>(N + 1);
   s.del = cv.take<int>(N + 1);
   int *keep = cv.take<int>(N + 1), *scanned = cv.take<int>(N + 1);
-  unsigned long long *Jr = cv.take<unsigned long long>(ncel), *Jz = cv.take<unsigned long long>(ncel);
+  unsigned long long *J[2][2];                          // [buffer][r, z]
+  for (int i = 0; i < 4; ++i) J[i >> 1][i & 1] = cv.take<unsigned long long>(ncel);
+  double *Er2 = cv.take<double>(nEr), *Ez2 = cv.take<double>(nEz), *H2 = cv.take<double>(ncel);
+  int *counts = cv.take<int>(4);
   void *tmp = cv.take<char>(sc);
   Species sp;
   sp.pos[0] = e_pos; sp.pos[1] = i1_pos; sp.pos[2] = i2_pos;
@@ -738,48 +979,79 @@ int gasatt_electricmagneticfield6(gasatt_ctx *ctx, double *e_pos, double *e_vel,
   sp.start[0] = 0; sp.start[1] = n_e; sp.start[2] = n_e + n_i1;
   const double e = GASATT_EM_E, c = GASATT_EM_C, mu = GASATT_EM_MU, eps = GASATT_EM_EPS;
   const unsigned g = grid_for(N, kBlock);
-  if (N > 0) {
-    k_em_load<<<g, kBlock, 0, ctx->stream>>>(sp, s, N, e, GASATT_EM_ME, GASATT_EM_MION, flags);
-    GASATT_LAUNCHED(ctx);
-  }
   // fixed-point scale: |q FN v w| <= 2e FN c per particle, N particles per node at most
   const double bound = (double)(N > 0 ? N : 1) * 2 * e * std::fabs(FN) * c;
   const int S = (int)std::floor(std::log2(std::ldexp(1.0, 62) / bound));
-  const double scale = std::ldexp(1.0, S);
-  const int ratio = 5;
+  const int ratio = 5, steps = cycle_time / ratio;
   const double ddt = ratio * dt;                       // electricmagneticfield6.m:134-135
-  FdtdCoef fc;
-  fc.dr = delta; fc.dz = delta; fc.PHIp = PHIp; fc.inv_scale = std::ldexp(1.0, -S);
-  fc.dt_eps = (dt / 2) / eps;
-  fc.dt_eps_dz = (dt / 2) / (eps * delta);
-  fc.axis = 4 * (dt / 2) / (eps * delta);
-  const unsigned gh = grid_for(ncel, kBlock), ge = grid_for((int64_t)(n_r + 1) * (n_z + 1), kBlock);
-  for (int k = 0; k < cycle_time / ratio; ++k) {        // :138-166
-    GASATT_CUDA(ctx, cudaMemsetAsync(Jr, 0, (size_t)ncel * 8, ctx->stream));
-    GASATT_CUDA(ctx, cudaMemsetAsync(Jz, 0, (size_t)ncel * 8, ctx->stream));
-    if (N > 0) {
-      k_em2_deposit<<<g, kBlock, 0, ctx->stream>>>(s, N, Rp, Lp, PHIp, ddt, n_r, n_z, delta, delta,
-                                                   FN, scale, Jr, Jz, flags);
+  EmParams ep;
+  ep.Rp = Rp; ep.Lp = Lp; ep.PHIp = PHIp; ep.cP = std::cos(PHIp); ep.sP = std::sin(PHIp);
+  ep.hdt = 0.5 * ddt;
+  ep.id = 1 / delta; ep.mu = mu; ep.c = c; ep.ic2 = 1 / (c * c); ep.FN = FN; ep.scale = std::ldexp(1.0, S);
+  for (int k = 0; k < 3; ++k) {
+    ep.q[k] = k == 0 ? -e : k * e;
+    ep.m[k] = k == 0 ? GASATT_EM_ME : GASATT_EM_MION;
+    ep.qm[k] = ep.q[k] / ep.m[k];
+    ep.qm_dt[k] = ep.qm[k] * ddt;
+  }
+  ep.nr = n_r; ep.nz = n_z;
+  ep.atan_phi = (flags & GASATT_Q_ATAN_PHI) != 0;
+  ep.euler = (flags & GASATT_Q_EULER_KICK) != 0;
+  ep.fast_fx = N >= 4096;
+  ep.wrap = !ep.atan_phi && !(PHIp < 2 * GASATT_PI - 1e-12) ? 0 : PHIp > 0 && PHIp <= GASATT_PI / 2 ? 1 : 2;
+  EmFieldParams fp;
+  fp.nr = n_r; fp.nz = n_z; fp.delta = delta; fp.PHIp = PHIp; fp.inv_scale = std::ldexp(1.0, -S);
+  fp.dt_eps = (dt / 2) / eps;
+  fp.dt_eps_dz = (dt / 2) / (eps * delta);
+  fp.axis = 4 * (dt / 2) / (eps * delta);
+  fp.endcopy = (flags & GASATT_Q_ER_END_COPY) != 0;
+  fp.jsign = (flags & GASATT_Q_EZ_AXIS_JSIGN) != 0;
+  fp.rshift = (flags & GASATT_Q_EZ_RSHIFT) != 0;
+  fp.h_mid = (dt / 2) / (mu * delta);
+  // One launch of all ten pairs where its tiles (11 columns of 32) still fit
+  // the GPU at once, else two of five (21 columns of 32).  A call of 20 steps
+  // with one launch / two: 100 x 500 cells 1069 / 1188 us, 200 x 1000 cells
+  // 1956 / 1916, 400 x 2000 cells 2837 / 2574.
+  const int whole = 2 * ratio;
+  auto tiles = [&](int pairs) {
+    return dim3((n_r + em_tile_cols(pairs)) / em_tile_cols(pairs), (n_z + em_tile_rows(pairs)) / em_tile_rows(pairs));
+  };
+  const dim3 one = tiles(whole);
+  const bool single = (int64_t)one.x * one.y <= kEmOneLaunch;
+  const EmFields there{Er, Ez, Hphi, Er2, Ez2, H2}, back{Er2, Ez2, H2, Er, Ez, Hphi};
+  bool away = false;                                   // the fields are in the scratch set
+  auto launch_fields = [&](int pairs, bool first, bool last, int b) {
+    fp.pairs = pairs;
+    fp.h_first = first ? (dt / 4) / (mu * delta) : fp.h_mid;      // dt/2 after the -dt/4 that opens the sub-cycle
+    fp.h_last = last ? (dt / 4) / (mu * delta) : 0;
+    k_em_fields<<<tiles(pairs), 32 * kEmWarps, 0, ctx->stream>>>(away ? back : there, fp, J[b][0], J[b][1],
+                                                                 J[1 - b][0], J[1 - b][1]);
+    away = !away;
+  };
+  if (steps > 0)
+    for (int i = 0; i < (N > 0 ? 2 : 4); ++i)
+      GASATT_CUDA(ctx, cudaMemsetAsync(J[i >> 1][i & 1], 0, ncel * 8, ctx->stream));
+  if (N > 0) {
+    ep.Jr = J[0][0]; ep.Jz = J[0][1];
+    k_em_load<<<g, kBlock, 0, ctx->stream>>>(sp, s, ep, N, (flags & GASATT_POS_IN_CYL) != 0, steps > 0);
+    GASATT_LAUNCHED(ctx);
+  }
+  for (int k = 0; k < steps; ++k) {                    // :138-166
+    const int b = k & 1;
+    // (an odd number of single launches would leave the fields in the scratch set)
+    if (single && !(k == steps - 1 && !away)) {
+      launch_fields(whole, true, true, b);
+      GASATT_LAUNCHED(ctx);
+    } else {
+      launch_fields(ratio, true, false, b);
+      GASATT_LAUNCHED(ctx);
+      launch_fields(ratio, false, true, b);
       GASATT_LAUNCHED(ctx);
     }
-    const double hdt[3] = {-dt / 4, dt / 2, dt / 4};
-    auto hstep = [&](double h) {
-      k_fdtd_h<double><<<gh, kBlock, 0, ctx->stream>>>(Hphi, Er, Ez, n_r, n_z, h / (mu * delta),
-                                                      h / (mu * delta));
-    };
-    hstep(hdt[0]);
-    GASATT_LAUNCHED(ctx);
-    for (int i = 0; i < 2 * ratio; ++i) {
-      hstep(hdt[1]);
-      GASATT_LAUNCHED(ctx);
-      k_fdtd_e<double><<<ge, kBlock, 0, ctx->stream>>>(Er, Ez, Hphi, Jr, Jz, n_r, n_z, fc, flags);
-      GASATT_LAUNCHED(ctx);
-    }
-    hstep(hdt[2]);
-    GASATT_LAUNCHED(ctx);
     if (N > 0) {
-      k_em4<<<g, kBlock, 0, ctx->stream>>>(s, N, Er, Ez, Hphi, Rp, Lp, PHIp, n_r, n_z, mu, c, delta,
-                                           delta, ddt, flags);
+      ep.Jr = J[1 - b][0]; ep.Jz = J[1 - b][1];
+      auto push = k == steps - 1 ? k_em_push<true> : k_em_push<false>;
+      push<<<g, kBlock, 0, ctx->stream>>>(sp, s, ep, N, away ? Er2 : Er, away ? Ez2 : Ez, away ? H2 : Hphi);
       GASATT_LAUNCHED(ctx);
     }
   }
@@ -789,13 +1061,10 @@ int gasatt_electricmagneticfield6(gasatt_ctx *ctx, double *e_pos, double *e_vel,
     GASATT_LAUNCHED(ctx);
     st = exclusive_scan(ctx, keep, scanned, N + 1, tmp, sc);
     if (st) return st;
-    k_em_store<<<g, kBlock, 0, ctx->stream>>>(sp, s, N, scanned, electron_kinetic, e);
+    k_em_store<<<g, kBlock, 0, ctx->stream>>>(sp, s, N, scanned, electron_kinetic, e, counts);
     GASATT_LAUNCHED(ctx);
     int h[4];
-    const int64_t idx[4] = {0, n_e, n_e + n_i1, N};
-    for (int i = 0; i < 4; ++i)
-      GASATT_CUDA(ctx, cudaMemcpyAsync((int *)ctx->pinned + i, scanned + idx[i], 4,
-                                       cudaMemcpyDeviceToHost, ctx->stream));
+    GASATT_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, counts, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     GASATT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     std::memcpy(h, ctx->pinned, sizeof(h));
     outs[0] = h[1] - h[0]; outs[1] = h[2] - h[1]; outs[2] = h[3] - h[2];

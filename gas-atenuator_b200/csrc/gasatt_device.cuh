@@ -136,14 +136,34 @@ __device__ __forceinline__ void gather3s(const T *__restrict__ Er, const T *__re
   }
 }
 
-// the reference's dense column-major grids (EM4.cu:41-122)
-template <typename T>
-__device__ __forceinline__ void gather3(const T *__restrict__ Er, const T *__restrict__ Ez,
-                                        const T *__restrict__ H, int nr, int nz, double dr,
-                                        double dz, double r0, double z0, double &E_r,
-                                        double &E_z, double &Hp) {
-  gather3s<T>(Er, Ez, H, nr, nz, nr, nr + 1, nr, dr, dz, r0, z0, E_r, E_z, Hp);
+// ------------------------------------------------------------ grid axis
+// x = i + f with i = floor(x) and f in [0, 1), for |x| < 2^31: rounding
+// x + 1.5 2^52 down leaves floor(x) in the low mantissa bits (exact)
+__device__ __forceinline__ int floor_split(double x, double &f) {
+  const double t = __dadd_rd(x, 6755399441055744.0);
+  f = __dsub_rn(x, __dsub_rn(t, 6755399441055744.0));
+  return __double2loint(t);
 }
+
+// Cell coordinate of x (in cells) on an axis of n cells: cell i in [0, n - 1]
+// (x = n exactly sits at the end of the last) and fraction f; the half-cell
+// staggered node pair a, a + 1 with weight w of the second, indices clamped
+// one-sided at the edges.
+struct Axis64 { int i, lo, hi; double f, w; };
+__device__ __forceinline__ Axis64 axis64(double x, int n) {
+  Axis64 A;
+  const int i = floor_split(x, A.f);
+  A.i = min(max(i, 0), n - 1);
+  if (i != A.i) A.f = __dsub_rn(x, (double)A.i);
+  const bool up = A.f >= 0.5;
+  const int a = up ? A.i : A.i - 1;
+  A.w = __dadd_rn(A.f, up ? -0.5 : 0.5);
+  A.lo = max(a, 0);
+  A.hi = min(a + 1, n - 1);
+  return A;
+}
+
+__device__ __forceinline__ double lerp64(double a, double b, double w) { return fma(w, __dsub_rn(b, a), a); }
 
 // ------------------------------------------------------ deposit weights
 // EM7.cu:56-162: the four cell-centred nodes around (r0, z0) and their
@@ -192,64 +212,9 @@ __device__ __forceinline__ int em7_weights_ld(double r0, double z0, int nr, int 
   return ar;
 }
 
-// the reference's dense n_r x n_z grid (EM7.cu:56-162)
-__device__ __forceinline__ int em7_weights(double r0, double z0, int nr, int nz, double dr,
-                                           double dz, int64_t a[4], double b[4]) {
-  return em7_weights_ld(r0, z0, nr, nz, nr, dr, dz, a, b);
-}
-
-// fixed-point current: value * 2^S rounded to nearest, added with a 64-bit
-// integer atomic (associative, so the grid is bit-identical run to run)
-__device__ __forceinline__ void fx_add(unsigned long long *J, int64_t idx, double v, double scale) {
-  const long long q = __double2ll_rn(v * scale);
-  if (q != 0) atomicAdd(J + idx, (unsigned long long)q);
-}
-
 // shell volume of node column i (EM7.cu:175-176)
 __host__ __device__ __forceinline__ double shell_volume(int i, double dr, double dz, double PHIp) {
   return PHIp / 2 * ((((i + 1) * dr) * ((i + 1) * dr) - (i * dr) * (i * dr)) * dz);
-}
-
-// ----------------------------------------------------------- half drift
-// EM2.cu:26-57 / EM4.cu:146-177 in Cartesian form: drift by v dt/2, (r, phi),
-// delete beyond Rp, wedge wrap that rotates the velocity-like vector w, and
-// specular reflection at z = 0, Lp.  Corrected mode uses atan2 and skips the
-// wrap for a full ring (PHIp >= 2 pi).
-__device__ __forceinline__ void halfdrift_cart(double &x, double &y, double &z, double &wx,
-                                               double &wy, double &wz, double vx, double vy,
-                                               double vz, double &r_o, double &phi_o, int &del,
-                                               double Rp, double Lp, double PHIp, double dt,
-                                               unsigned flags) {
-  double X = x + 0.5 * vx * dt;
-  double Y = y + 0.5 * vy * dt;
-  double Z = z + 0.5 * vz * dt;
-  const double r = sqrt(X * X + Y * Y);
-  double phi = (flags & GASATT_Q_ATAN_PHI) ? atan(Y / X) : atan2(Y, X);
-  if (r > Rp) del = 1;
-  const bool wrap = (flags & GASATT_Q_ATAN_PHI) || PHIp < 2 * GASATT_PI - 1e-12;
-  if (wrap) {
-    const double cp = cos(PHIp), sp = sin(PHIp);
-    double w1;
-    // bounded: a wrap count above 2^20 means phi is not finite-sized
-    for (int it = 0; phi < 0 && it < (1 << 20); ++it) {
-      phi = phi + PHIp;
-      w1 = wx * cp - wy * sp;
-      wy = wx * sp + wy * cp;
-      wx = w1;
-    }
-    for (int it = 0; phi > PHIp && it < (1 << 20); ++it) {
-      phi = phi - PHIp;
-      w1 = wx * cp + wy * sp;
-      wy = -wx * sp + wy * cp;
-      wx = w1;
-    }
-  }
-  X = r * cos(phi);
-  Y = r * sin(phi);
-  if (Z > Lp) { Z = 2 * Lp - Z; wz = -wz; }
-  if (Z < 0) { Z = -Z; wz = -wz; }
-  x = X; y = Y; z = Z;
-  r_o = r; phi_o = phi;
 }
 
 // ------------------------------------------------------------- rotation

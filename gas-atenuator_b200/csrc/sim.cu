@@ -515,34 +515,6 @@ __device__ __forceinline__ void deposit_values64(const SimParams &P, double r, d
 // longer.  Chunks of up to 4608 particles: 1024 / 1536 / 2560 are 5 / 2 / 1 us
 // longer (more flushes).
 
-// x = i + f with i = floor(x) and f in [0, 1), for |x| < 2^31: rounding
-// x + 1.5 2^52 down leaves floor(x) in the low mantissa bits (exact)
-__device__ __forceinline__ int floor_split(double x, double &f) {
-  const double t = __dadd_rd(x, 6755399441055744.0);
-  f = __dsub_rn(x, __dsub_rn(t, 6755399441055744.0));
-  return __double2loint(t);
-}
-
-// Cell coordinate of x (in cells) on an axis of n cells: cell i in [0, n - 1]
-// (x = n exactly sits at the end of the last) and fraction f; the half-cell
-// staggered node pair a, a + 1 with weight w of the second, indices clamped
-// one-sided at the edges.
-struct Axis64 { int i, lo, hi; double f, w; };
-__device__ __forceinline__ Axis64 axis64(double x, int n) {
-  Axis64 A;
-  const int i = floor_split(x, A.f);
-  A.i = min(max(i, 0), n - 1);
-  if (i != A.i) A.f = __dsub_rn(x, (double)A.i);
-  const bool up = A.f >= 0.5;
-  const int a = up ? A.i : A.i - 1;
-  A.w = __dadd_rn(A.f, up ? -0.5 : 0.5);
-  A.lo = max(a, 0);
-  A.hi = min(a + 1, n - 1);
-  return A;
-}
-
-__device__ __forceinline__ double lerp64(double a, double b, double w) { return fma(w, __dsub_rn(b, a), a); }
-
 // Boris kick in E = (Er, 0, Ez), B = (0, mu0 H, 0) with the fields of the
 // staggered bilinear gather (EM4.cu:41-122).
 __device__ __forceinline__ void kick64(const SimParams &P, const Fields<double> &F, double r,
