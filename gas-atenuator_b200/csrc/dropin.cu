@@ -45,6 +45,18 @@ __device__ double d_loglog(const double *x, int sx, const double *y, int sy, int
   return y1 * pow(xq / x1, s);
 }
 
+// x^e; the excitation table's exponents are 1, 3 and 3/4, whose powers need no
+// logarithm (200,000 energies: 53 us with pow throughout, 18 us so)
+__device__ __forceinline__ double pow_table(double x, double e) {
+  if (e == 1) return x;
+  if (e == 3) return x * x * x;
+  if (e == 0.75) {
+    const double r = sqrt(x);
+    return r * sqrt(r);
+  }
+  return pow(x, e);
+}
+
 // find_CS0.m:100-146 on one energy E [keV]
 __global__ void k_find_cs0(XsRaw t, const double *__restrict__ E, int64_t n, double *se,
                            double *si, double *sx, unsigned flags) {
@@ -76,8 +88,8 @@ __global__ void k_find_cs0(XsRaw t, const double *__restrict__ E, int64_t n, dou
       const double nu = t.t_exc[3 * t.n_exc + i], ga = t.t_exc[4 * t.n_exc + i];
       if (!faithful && !(T > k)) continue;
       const double a = GASATT_CS_Q0 * A / (k * k);
-      const double b = pow(k / T, om);
-      const double c = pow(1 - pow(k / T, ga), nu);
+      const double b = pow_table(k / T, om);
+      const double c = pow_table(1 - pow_table(k / T, ga), nu);
       s = s + a * b * c;
     }
     sx[p] = s * 1e-4;
@@ -563,6 +575,12 @@ __global__ void k_keep_flags(const int *del, int64_t N, int *keep) {
 }
 
 // ------------------------------------------------------- electron_collision
+// The table set-up, the test of every electron
+// (k_collision_select: density cell, collision test, branch), and the
+// collisions alone (k_collision_elastic, k_collision_other), compacted by branch.  One thread per
+// electron that ran whatever befell it took 461 us for 200,000 electrons: an
+// elastic angle evaluates the 181-angle PDF up to three times, and most lanes
+// of a warp wait for the few that collide.
 struct MccTables {
   const double *xI, *yI, *V;  int ne;
   const double *exc;  int n_exc;     // n_exc x 5 column-major
@@ -570,68 +588,26 @@ struct MccTables {
   const double *density, *temperature; int64_t ncell;
 };
 
-__device__ __forceinline__ double pdf_k(const double *V, int ne, int i, int k, double a0,
-                                        double b0, double TCS, double pi) {
-  int64_t i1 = (int64_t)i * 181 + k, i2 = (int64_t)(i + 1) * 181 + k;
-  const int64_t last = (int64_t)ne * 181 - 1;
-  if (i1 > last) i1 = last;
-  if (i2 > last) i2 = last;
-  const double vI = a0 * V[i1] + b0 * V[i2];
-  double D = exp(vI);
-  D = 2 * pi * sin(k * pi / 180) * D * 2;
-  return 1 / TCS * D;
-}
+// the raw tables packed in one upload (offsets in doubles)
+struct MccRaw {
+  const double *sel1, *el, *sdel, *del;
+  int n_sel1, n_el, sdel_cols, del_cols;
+};
 
-// electron_transport.cu:88-121 (GASATT_Q_CDF_NEXTBIN) or get_ElasticSc_sub1.m
-__device__ double elastic_theta(double energy, const MccTables &t, double U, double pi,
-                                unsigned flags) {
-  const double *xI = t.xI;
-  const int ne = t.ne;
-  double Ee = (flags & GASATT_Q_XS_LINEAR_E) ? energy : log(energy);
-  if (!(flags & GASATT_Q_XS_LINEAR_E)) {
-    if (Ee < xI[0]) Ee = xI[0];
-    if (Ee > xI[ne - 1]) Ee = xI[ne - 1];
-  }
-  int i = 0;
-  while (i < ne - 2 && Ee > xI[i + 1]) i++;
-  const double a0 = (xI[i + 1] - Ee) / (xI[i + 1] - xI[i]);
-  const double b0 = (Ee - xI[i]) / (xI[i + 1] - xI[i]);
-  const double TCS = (a0 * t.yI[i] + b0 * t.yI[i + 1]) * 2;
-  if (flags & GASATT_Q_CDF_NEXTBIN) {
-    double imax = 0;
-    for (int k = 0; k <= 180; ++k) imax = imax + pdf_k(t.V, ne, i, k, a0, b0, TCS, pi) * pi / 180;
-    const double rnd = U * imax;
-    double i1 = 0;
-    int k = 0;
-    while (rnd > i1 && k < 181) {
-      i1 = i1 + pdf_k(t.V, ne, i, k, a0, b0, TCS, pi) * pi / 180;
-      k++;
-    }
-    const double i2 = i1 + pdf_k(t.V, ne, i, k, a0, b0, TCS, pi) * pi / 180;
-    const double aa = (i2 - rnd) / (i2 - i1), bb = (rnd - i1) / (i2 - i1);
-    return (aa * (k - 1) + bb * k) * pi / 180;
-  }
-  // trapezoid CDF and linear inverse (cumtrapz + interp1)
-  const double h = pi / 180;
-  double C = 0, prev = pdf_k(t.V, ne, i, 0, a0, b0, TCS, pi);
-  double tot = 0;
-  {
-    double p0 = prev;
-    for (int k = 1; k <= 180; ++k) {
-      const double pk = pdf_k(t.V, ne, i, k, a0, b0, TCS, pi);
-      tot = tot + (p0 + pk) / 2 * h;
-      p0 = pk;
+// electron_collision.m:12-33 as build_elastic_tables (tables.cpp): combined
+// cross-sections and the logarithms of the energies and DCS columns
+__global__ void k_collision_tables(MccRaw t, double *xI, double *yI, double *V) {
+  const int m1 = t.n_sel1 - 1, ns = t.sdel_cols - 1, ne = ns + t.del_cols - 1;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ne * 182; i += gridDim.x * blockDim.x) {
+    const int c = i / 182, k = i - c * 182;
+    const double v = log(c < ns ? t.sdel[(int64_t)(c + 1) * 182 + k] : t.del[(int64_t)(c - ns + 1) * 182 + k]);
+    if (k == 0) {
+      xI[c] = v;
+      yI[c] = c < m1 ? t.sel1[t.n_sel1 + c] * 1e-20 / GASATT_A0SQ / 2 : t.el[2 * (c - m1) + 1];
+    } else {
+      V[(int64_t)c * 181 + k - 1] = v;
     }
   }
-  const double rn = U * tot;
-  for (int k = 1; k <= 180; ++k) {
-    const double pk = pdf_k(t.V, ne, i, k, a0, b0, TCS, pi);
-    const double Cn = C + (prev + pk) / 2 * h;
-    if (Cn > rn || k == 180) return ((k - 1) + (rn - C) / (Cn - C)) * h;
-    C = Cn;
-    prev = pk;
-  }
-  return pi;
 }
 
 __device__ __forceinline__ double pow_sel(double a, double b, unsigned flags) {
@@ -640,138 +616,313 @@ __device__ __forceinline__ double pow_sel(double a, double b, unsigned flags) {
 }
 
 struct MccOut {
-  uint8_t *sec;
+  int *sec;                          // 1: a secondary is born (n + 1 entries, the last 0)
   double *svx, *svy, *svz, *sample, *ivx, *ivy, *ivz;
 };
 
-// electron_transport.cu:39-229; positions/velocities column-major (ld = cap)
-__global__ void k_electron_transport(double *pos, double *vel, int64_t cap, int64_t n,
-                                     const double *sig_el, const double *sig_ion,
-                                     const double *sig_exc, const double *energy, MccTables t,
-                                     MccOut out, double dr, double dz, double dt,
-                                     const double *draws, uint64_t seed, int64_t call,
-                                     unsigned flags) {
-  const double e = GASATT_MCC_E, c = GASATT_MCC_C, m = GASATT_MCC_ME, m_ion = GASATT_MCC_MION;
-  const double kb = GASATT_MCC_KB, E_e = m * c * c / e;
-  const double pi = (flags & GASATT_Q_PI7) ? GASATT_MCC_PI7 : GASATT_PI;
+// colliding electrons by branch: elastic ones, and the others (an ionization
+// as ~index); n[0], n[1]: how many
+struct MccLists { int *elastic, *other; unsigned *n; };
+
+__device__ __forceinline__ void list_push(bool want, int v, unsigned *n, int *list) {
+  const unsigned m = __ballot_sync(0xFFFFFFFFu, want);
+  if (!m) return;
+  const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+  unsigned base = 0;
+  if (lane == leader) base = atomicAdd(n, (unsigned)__popc(m));
+  base = __shfl_sync(0xFFFFFFFFu, base, leader);
+  if (want) list[base + __popc(m & ((1u << lane) - 1))] = v;
+}
+
+// electron_transport.cu:64-87, 127-128, 139: the density cell, the collision
+// test and the branch of every electron
+__global__ void k_collision_select(const double *__restrict__ pos, const double *__restrict__ vel, int64_t cap,
+                                   int64_t n, const double *__restrict__ sig_el,
+                                   const double *__restrict__ sig_ion, const double *__restrict__ sig_exc,
+                                   const double *__restrict__ energy, MccTables t, MccOut out, MccLists ls,
+                                   double dr, double dz, double dt, const double *__restrict__ draws,
+                                   uint64_t seed, int64_t call, unsigned flags) {
   const double I = GASATT_ION_I_EV;
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
-       p += (int64_t)gridDim.x * blockDim.x) {
-    out.sec[p] = 0;
-    double U[GASATT_MCC_NDRAW];
-    if (draws) {
-#pragma unroll
-      for (int k = 0; k < GASATT_MCC_NDRAW; ++k) U[k] = draws[p * GASATT_MCC_NDRAW + k];
-    } else {
-      U2 a = draw2(seed, (uint64_t)p, call, 0), b = draw2(seed, (uint64_t)p, call, 1);
-      U2 g1 = draw2(seed, (uint64_t)p, call, 2), g2 = draw2(seed, (uint64_t)p, call, 3);
-      U[0] = a.a; U[1] = a.b; U[2] = b.a; U[3] = b.b;
-      const double rad1 = sqrt(-2 * log(g1.a)), rad2 = sqrt(-2 * log(g2.a));
-      U[4] = rad1 * cos(2 * GASATT_PI * g1.b);
-      U[5] = rad1 * sin(2 * GASATT_PI * g1.b);
-      U[6] = rad2 * cos(2 * GASATT_PI * g2.b);
-      U[7] = 0;
-    }
-    double vx = vel[p], vy = vel[cap + p], vz = vel[2 * cap + p];
-    const double x = pos[p], y = pos[cap + p], z = pos[2 * cap + p];
-    const double v_e = sqrt(vx * vx + vy * vy + vz * vz);
-    const double dx = v_e * dt;
-    const double r = sqrt(x * x + y * y);
-    const double phi = atan(y / x);
-    int iz = (int)floor(z / dz), ir = (int)floor(r / dr);
-    if (ir > t.rmax - 1) ir = t.rmax - 1;
-    if (ir < 0) ir = 0;
-    int iphi = (int)floor(phi / t.dphi[ir]);
-    const int nphi = t.sum_cell0[ir + 1] - t.sum_cell0[ir];
-    if (iphi > nphi - 1) iphi = nphi - 1;
-    if (iphi < 0) iphi = 0;
-    int64_t index = (int64_t)iz * t.cellnumxy + t.sum_cell0[ir] + iphi;
-    if (index < 0) index = 0;
-    if (index > t.ncell - 1) index = t.ncell - 1;
-    const double p_el = dx * t.density[index] * sig_el[p];
-    const double p_io = dx * t.density[index] * sig_ion[p];
-    const double p_ex = dx * t.density[index] * sig_exc[p];
-    double p_tot = p_el + p_io + p_ex;
-    const double a = p_el / p_tot;
-    const double b = a + p_io / p_tot;
-    if (!(flags & GASATT_Q_COLL_LINEAR_P)) p_tot = -expm1(-p_tot);
-    if (!(U[0] < p_tot)) continue;
-    const double en = energy[p];
-    if (U[1] < a) {
-      const double th = elastic_theta(en, t, U[2], pi, flags);
-      const double ph = 2 * pi * U[3];
-      rotate_v(vx, vy, vz, th, ph, true);
-    } else if (U[1] < b && en > I / 1000) {
-      const double T = en * 1000;
-      const double T_a = 1000, T_b = 2 * I, t_b = I, T_s = 4.17, t_s = 13.8;
-      const double T_0 = T_s - T_a / (T + T_b);
-      const double tt = t_s * T / (T + t_b);
-      const double T_m = (T - I) / 2;
-      const double k_1 = atan((T_m - T_0) / tt);
-      const double k_2 = atan(T_0 / tt);
-      const double k0 = T_0 + tt * tan(U[2] * (k_1 + k_2) - k_2);
-      const double E_1 = k0, E_2 = T - E_1 - I;
-      double E_p, E_s;
-      if (E_2 > E_1) { E_p = E_2; E_s = E_1; } else { E_p = E_1; E_s = E_2; }
-      const double kk = (flags & GASATT_Q_SEC_LAB_FRAME) ? k0 : E_s;
-      E_p = E_p * e;
-      E_s = E_s * e;
-      const double phi_p = 2 * pi * U[3];
-      const double phi_s = phi_p - pi;
-      const double th_p = asin(sqrt((kk / T) / ((1 - kk / T) * T / (2 * E_e) + 1)));
-      const double th_s = asin(sqrt((1 - kk / T) / (1 + kk / (2 * E_e))));
-      const double ix = vx / v_e, iy = vy / v_e, iz_ = vz / v_e;
-      double gamma = 1 + E_p / (m * c * c);
-      const double v_p = c * sqrt(1 - 1 / (gamma * gamma));
-      const double ratio = v_p / v_e;
-      vx = ratio * vx; vy = ratio * vy; vz = ratio * vz;
-      rotate_v(vx, vy, vz, th_p, phi_p, true);
-      gamma = 1 + E_s / (m * c * c);
-      const double v_s = c * sqrt(1 - 1 / (gamma * gamma));
-      out.sec[p] = 1;
-      if (flags & GASATT_Q_SEC_LAB_FRAME) {
-        out.svx[p] = v_s * sin(th_s) * cos(phi_s);
-        out.svy[p] = v_s * sin(th_s) * sin(phi_s);
-        out.svz[p] = v_s * cos(th_s);
+  const int lane = threadIdx.x & 31;
+  for (int64_t base = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); base <= n;
+       base += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = base + lane;
+    bool elastic = false, other = false, ion = false;
+    if (p <= n) out.sec[p] = 0;
+    if (p < n) {
+      double U0, U1;
+      if (draws) {
+        U0 = draws[p * GASATT_MCC_NDRAW];
+        U1 = draws[p * GASATT_MCC_NDRAW + 1];
       } else {
-        double sx = ix * v_s, sy = iy * v_s, sz = iz_ * v_s;
-        rotate_v(sx, sy, sz, th_s, phi_s, true);
-        out.svx[p] = sx; out.svy[p] = sy; out.svz[p] = sz;
+        const U2 a = draw2(seed, (uint64_t)p, call, 0);
+        U0 = a.a; U1 = a.b;
       }
-      out.sample[p] = (double)index;
-      const double sd = sqrt(m_ion / (kb * t.temperature[index]));
-      out.ivx[p] = (double)(float)U[4] / sd;
-      out.ivy[p] = (double)(float)U[5] / sd;
-      out.ivz[p] = (double)(float)U[6] / sd;
-    } else {
-      const double T = en * 1000;
-      double k1 = 0, k2 = 0;
-      for (int i = 0; i < t.n_exc; ++i) {
-        const double k = t.exc[i], A = t.exc[t.n_exc + i], om = t.exc[2 * t.n_exc + i];
-        const double nu = t.exc[3 * t.n_exc + i], ga = t.exc[4 * t.n_exc + i];
-        if (!(flags & GASATT_Q_EXC_POWF) && !(T > k)) continue;
-        const double aE = GASATT_MCC_Q0 * A / (k * k);
-        const double bE = pow_sel(k / T, om, flags);
-        const double cE = pow_sel(pow_sel(1 - k / T, ga, flags), nu, flags);
-        k1 = k1 + aE * bE * cE * k;
-        k2 = k2 + aE * bE * cE;
+      const double vx = vel[p], vy = vel[cap + p], vz = vel[2 * cap + p];
+      const double x = pos[p], y = pos[cap + p], z = pos[2 * cap + p];
+      const double v_e = sqrt(vx * vx + vy * vy + vz * vz);
+      const double dx = v_e * dt;
+      const double r = sqrt(x * x + y * y);
+      const double phi = atan(y / x);
+      int iz = (int)floor(z / dz), ir = (int)floor(r / dr);
+      if (ir > t.rmax - 1) ir = t.rmax - 1;
+      if (ir < 0) ir = 0;
+      int iphi = (int)floor(phi / t.dphi[ir]);
+      const int nphi = t.sum_cell0[ir + 1] - t.sum_cell0[ir];
+      if (iphi > nphi - 1) iphi = nphi - 1;
+      if (iphi < 0) iphi = 0;
+      int64_t index = (int64_t)iz * t.cellnumxy + t.sum_cell0[ir] + iphi;
+      if (index < 0) index = 0;
+      if (index > t.ncell - 1) index = t.ncell - 1;
+      const double den = t.density[index];
+      const double p_el = dx * den * sig_el[p];
+      const double p_io = dx * den * sig_ion[p];
+      const double p_ex = dx * den * sig_exc[p];
+      double p_tot = p_el + p_io + p_ex;
+      const double a = p_el / p_tot;
+      const double b = a + p_io / p_tot;
+      if (!(flags & GASATT_Q_COLL_LINEAR_P)) p_tot = -expm1(-p_tot);
+      if (U0 < p_tot) {
+        elastic = U1 < a;
+        other = !elastic;
+        ion = other && U1 < b && energy[p] > I / 1000;
+        if (ion) out.sample[p] = (double)index;
       }
-      if (k2 == 0) continue;
-      const double E_dep = k1 / k2;
-      const double E_p = T - E_dep;
-      const double gamma = 1 + E_p * e / (m * c * c);
-      const double v_p = c * sqrt(1 - 1 / (gamma * gamma));
-      const double ratio = v_p / v_e;
-      vx = ratio * vx; vy = ratio * vy; vz = ratio * vz;
     }
-    vel[p] = vx; vel[cap + p] = vy; vel[2 * cap + p] = vz;
+    list_push(elastic, (int)p, ls.n, ls.elastic);
+    list_push(other, ion ? ~(int)p : (int)p, ls.n + 1, ls.other);
   }
 }
 
-__global__ void k_u8_to_int(const uint8_t *a, int64_t n, int *b) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    b[i] = i < n ? (int)a[i] : 0;
+// Elastic angles, kElGroup electrons per block: its warps evaluate the PDF of
+// each at the 181 angles, a lane per angle, into shared memory; then a lane
+// per electron forms the CDF in the reference's order and inverts it.  Bound
+// by instruction issue (the exponentials: 181 an electron); 107,000 elastic
+// collisions take 97 us.
+constexpr int kElGroup = 32, kElThreads = 256;
+constexpr int kElSmem = (kElGroup + 1) * 181 * 8;    // the PDFs (181 apart: no bank conflicts), and the sines
+
+struct ElasticAt { int i; double a0, b0, inv_tcs; };
+
+// electron_transport.cu:88-102: the energy columns around an electron's energy
+// (by a whole warp: the first column whose upper end is not below it)
+__device__ __forceinline__ ElasticAt elastic_at(double energy, const MccTables &t, unsigned flags) {
+  const double *xI = t.xI;
+  double Ee = (flags & GASATT_Q_XS_LINEAR_E) ? energy : log(energy);
+  if (!(flags & GASATT_Q_XS_LINEAR_E)) {
+    if (Ee < xI[0]) Ee = xI[0];
+    if (Ee > xI[t.ne - 1]) Ee = xI[t.ne - 1];
+  }
+  ElasticAt e;
+  const int lane = threadIdx.x & 31;
+  e.i = t.ne - 2;
+  for (int k = 0; k < t.ne - 2; k += 32) {
+    const unsigned stop = __ballot_sync(0xFFFFFFFFu, k + lane < t.ne - 2 && !(Ee > xI[k + lane + 1]));
+    if (stop) { e.i = k + __ffs(stop) - 1; break; }
+  }
+  e.a0 = (xI[e.i + 1] - Ee) / (xI[e.i + 1] - xI[e.i]);
+  e.b0 = (Ee - xI[e.i]) / (xI[e.i + 1] - xI[e.i]);
+  e.inv_tcs = 1 / ((e.a0 * t.yI[e.i] + e.b0 * t.yI[e.i + 1]) * 2);
+  return e;
+}
+
+// The angle from f[k] = PDF(k degrees) pi / 180, k = 0..180 (the rectangles of
+// the reference's CDF): electron_transport.cu:103-121 (GASATT_Q_CDF_NEXTBIN) or
+// get_ElasticSc_sub1.m.  The running sums, added in the reference's order,
+// replace f, and its walk up the CDF becomes a bisection (it stops at once
+// where the sums are not above 0, else they rise).
+__device__ double elastic_theta(double *f, const ElasticAt &e, const MccTables &t, double U, double pi,
+                                unsigned flags) {
+  double sum = 0, last = f[0];
+  if (flags & GASATT_Q_CDF_NEXTBIN) {
+#pragma unroll 8
+    for (int k = 0; k <= 180; ++k) {
+      sum = sum + f[k];
+      f[k] = sum;                          // the first k + 1 rectangles
+    }
+    const double rnd = U * sum;
+    int k = 0;                             // the first k with rnd <= the first k rectangles
+    if (rnd > 0) {
+      int lo = 0, hi = 181;
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (rnd > f[mid - 1]) lo = mid; else hi = mid;
+      }
+      k = hi;
+    }
+    const double i1 = k > 0 ? f[k - 1] : 0.0;
+    double i2;
+    if (k < 181) {
+      i2 = f[k];
+    } else {             // the reference goes on into the next column (clamped to the table)
+      const int64_t end = (int64_t)t.ne * 181 - 1, i1k = (int64_t)e.i * 181 + k, i2k = i1k + 181;
+      const double vI = e.a0 * t.V[i1k < end ? i1k : end] + e.b0 * t.V[i2k < end ? i2k : end];
+      i2 = i1 + e.inv_tcs * (2 * pi * sin(k * pi / 180) * exp(vI) * 2) * pi / 180;
+    }
+    const double aa = (i2 - rnd) / (i2 - i1), bb = (rnd - i1) / (i2 - i1);
+    return (aa * (k - 1) + bb * k) * pi / 180;
+  }
+  // trapezoid CDF and linear inverse (cumtrapz + interp1)
+  f[0] = 0;
+#pragma unroll 4
+  for (int k = 1; k <= 180; ++k) {
+    const double fk = f[k];
+    sum = sum + (last + fk) / 2;
+    f[k] = sum;
+    last = fk;
+  }
+  const double rn = U * sum;
+  int lo = 0, hi = 180;                    // the first k with CDF(k) > rn, at most 180
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (f[mid] > rn) hi = mid; else lo = mid;
+  }
+  return ((hi - 1) + (rn - f[hi - 1]) / (f[hi] - f[hi - 1])) * (pi / 180);
+}
+
+__device__ __forceinline__ void late_draws(const double *draws, int64_t p, uint64_t seed, int64_t call, double &u2,
+                                           double &u3) {
+  if (draws) {
+    u2 = draws[p * GASATT_MCC_NDRAW + 2];
+    u3 = draws[p * GASATT_MCC_NDRAW + 3];
+  } else {
+    const U2 b = draw2(seed, (uint64_t)p, call, 1);
+    u2 = b.a; u3 = b.b;
+  }
+}
+
+// An ionization or excitation of electron p (electron_transport.cu:139-227)
+__device__ __forceinline__ void collide_other(int64_t p, bool ion, double *vel, int64_t cap, double en,
+                                              const MccTables &t, const MccOut &out, const double *draws,
+                                              uint64_t seed, int64_t call, double pi, unsigned flags) {
+  const double e = GASATT_MCC_E, c = GASATT_MCC_C, m = GASATT_MCC_ME, m_ion = GASATT_MCC_MION;
+  const double kb = GASATT_MCC_KB, E_e = m * c * c / e, I = GASATT_ION_I_EV;
+  double vx = vel[p], vy = vel[cap + p], vz = vel[2 * cap + p];
+  const double v_e = sqrt(vx * vx + vy * vy + vz * vz);
+  const double T = en * 1000;
+  if (ion) {
+    double u2, u3;
+    late_draws(draws, p, seed, call, u2, u3);
+    const double T_a = 1000, T_b = 2 * I, t_b = I, T_s = 4.17, t_s = 13.8;
+    const double T_0 = T_s - T_a / (T + T_b);
+    const double tt = t_s * T / (T + t_b);
+    const double T_m = (T - I) / 2;
+    const double k_1 = atan((T_m - T_0) / tt);
+    const double k_2 = atan(T_0 / tt);
+    const double k0 = T_0 + tt * tan(u2 * (k_1 + k_2) - k_2);
+    const double E_1 = k0, E_2 = T - E_1 - I;
+    double E_p, E_s;
+    if (E_2 > E_1) { E_p = E_2; E_s = E_1; } else { E_p = E_1; E_s = E_2; }
+    const double kk = (flags & GASATT_Q_SEC_LAB_FRAME) ? k0 : E_s;
+    E_p = E_p * e;
+    E_s = E_s * e;
+    const double phi_p = 2 * pi * u3;
+    const double phi_s = phi_p - pi;
+    const double th_p = asin(sqrt((kk / T) / ((1 - kk / T) * T / (2 * E_e) + 1)));
+    const double th_s = asin(sqrt((1 - kk / T) / (1 + kk / (2 * E_e))));
+    const double ix = vx / v_e, iy = vy / v_e, iz_ = vz / v_e;
+    double gamma = 1 + E_p / (m * c * c);
+    const double v_p = c * sqrt(1 - 1 / (gamma * gamma));
+    const double ratio = v_p / v_e;
+    vx = ratio * vx; vy = ratio * vy; vz = ratio * vz;
+    rotate_v(vx, vy, vz, th_p, phi_p, true);
+    gamma = 1 + E_s / (m * c * c);
+    const double v_s = c * sqrt(1 - 1 / (gamma * gamma));
+    out.sec[p] = 1;
+    if (flags & GASATT_Q_SEC_LAB_FRAME) {
+      out.svx[p] = v_s * sin(th_s) * cos(phi_s);
+      out.svy[p] = v_s * sin(th_s) * sin(phi_s);
+      out.svz[p] = v_s * cos(th_s);
+    } else {
+      double sx = ix * v_s, sy = iy * v_s, sz = iz_ * v_s;
+      rotate_v(sx, sy, sz, th_s, phi_s, true);
+      out.svx[p] = sx; out.svy[p] = sy; out.svz[p] = sz;
+    }
+    double g[3];
+    if (draws) {
+      for (int k = 0; k < 3; ++k) g[k] = draws[p * GASATT_MCC_NDRAW + 4 + k];
+    } else {
+      const U2 g1 = draw2(seed, (uint64_t)p, call, 2), g2 = draw2(seed, (uint64_t)p, call, 3);
+      const double rad1 = sqrt(-2 * log(g1.a)), rad2 = sqrt(-2 * log(g2.a));
+      g[0] = rad1 * cos(2 * GASATT_PI * g1.b);
+      g[1] = rad1 * sin(2 * GASATT_PI * g1.b);
+      g[2] = rad2 * cos(2 * GASATT_PI * g2.b);
+    }
+    const double sd = sqrt(m_ion / (kb * t.temperature[(int64_t)out.sample[p]]));
+    out.ivx[p] = (double)(float)g[0] / sd;
+    out.ivy[p] = (double)(float)g[1] / sd;
+    out.ivz[p] = (double)(float)g[2] / sd;
+  } else {
+    double k1 = 0, k2 = 0;
+    for (int i = 0; i < t.n_exc; ++i) {
+      const double k = t.exc[i], A = t.exc[t.n_exc + i], om = t.exc[2 * t.n_exc + i];
+      const double nu = t.exc[3 * t.n_exc + i], ga = t.exc[4 * t.n_exc + i];
+      if (!(flags & GASATT_Q_EXC_POWF) && !(T > k)) continue;
+      const double aE = GASATT_MCC_Q0 * A / (k * k);
+      const double bE = pow_sel(k / T, om, flags);
+      const double cE = pow_sel(pow_sel(1 - k / T, ga, flags), nu, flags);
+      k1 = k1 + aE * bE * cE * k;
+      k2 = k2 + aE * bE * cE;
+    }
+    if (k2 == 0) return;
+    const double E_dep = k1 / k2;
+    const double E_p = T - E_dep;
+    const double gamma = 1 + E_p * e / (m * c * c);
+    const double v_p = c * sqrt(1 - 1 / (gamma * gamma));
+    const double ratio = v_p / v_e;
+    vx = ratio * vx; vy = ratio * vy; vz = ratio * vz;
+  }
+  vel[p] = vx; vel[cap + p] = vy; vel[2 * cap + p] = vz;
+}
+
+// the ionizations and excitations (electron_transport.cu:139-227), one per thread
+__global__ void k_collision_other(double *vel, int64_t cap, const double *__restrict__ energy, MccTables t,
+                                  MccOut out, MccLists ls, const double *__restrict__ draws, uint64_t seed,
+                                  int64_t call, unsigned flags) {
+  const double pi = (flags & GASATT_Q_PI7) ? GASATT_MCC_PI7 : GASATT_PI;
+  const unsigned n = ls.n[1];
+  for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const int v = ls.other[k], p = v < 0 ? ~v : v;
+    collide_other(p, v < 0, vel, cap, energy[p], t, out, draws, seed, call, pi, flags);
+  }
+}
+
+// the elastic collisions (electron_transport.cu:88-135), in groups
+__global__ void __launch_bounds__(kElThreads) k_collision_elastic(double *vel, int64_t cap,
+                                                                  const double *__restrict__ energy, MccTables t,
+                                                                  MccLists ls, const double *__restrict__ draws,
+                                                                  uint64_t seed, int64_t call, unsigned flags) {
+  extern __shared__ double el_smem[];
+  __shared__ ElasticAt at[kElGroup];
+  const double pi = (flags & GASATT_Q_PI7) ? GASATT_MCC_PI7 : GASATT_PI;
+  const unsigned n = ls.n[0];
+  double *sines = el_smem + kElGroup * 181;
+  for (int k = threadIdx.x; k < 181; k += kElThreads) sines[k] = 4 * pi * sin(k * pi / 180) * (pi / 180);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (unsigned g = blockIdx.x * kElGroup; g < n; g += gridDim.x * kElGroup) {
+    const int m = min(n - g, (unsigned)kElGroup);
+    __syncthreads();                      // the last group's PDFs are no longer read
+    for (int j = warp; j < m; j += kElThreads / 32) {
+      const ElasticAt e = elastic_at(energy[ls.elastic[g + j]], t, flags);
+      if (lane == 0) at[j] = e;
+      // electron_transport.cu:103-109
+      const double *V = t.V + e.i * 181 + lane;
+      double *f = el_smem + j * 181 + lane;
+#pragma unroll
+      for (int k = 0; k < 181; k += 32)
+        if (k + lane < 181) f[k] = e.inv_tcs * sines[k + lane] * exp(e.a0 * V[k] + e.b0 * V[k + 181]);
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < m) {
+      const int64_t p = ls.elastic[g + threadIdx.x];
+      double u2, u3;
+      late_draws(draws, p, seed, call, u2, u3);
+      const double th = elastic_theta(el_smem + threadIdx.x * 181, at[threadIdx.x], t, u2, pi, flags);
+      double vx = vel[p], vy = vel[cap + p], vz = vel[2 * cap + p];
+      rotate_v(vx, vy, vz, th, 2 * pi * u3, true);
+      vel[p] = vx; vel[cap + p] = vy; vel[2 * cap + p] = vz;
+    }
+  }
 }
 
 // electron_collision.m:63-75: append secondaries and ions in parent order
@@ -837,16 +988,17 @@ int gasatt_find_CS0(gasatt_ctx *ctx, const gasatt_tables *tab, const double *E_k
   const size_t ne = 2 * (size_t)tab->n_el, ns = 2 * (size_t)tab->n_sel, ni = 2 * (size_t)tab->n_ion,
                nx = 5 * (size_t)tab->n_exc;
   void *buf;
-  st = scratch(ctx, align256(ne * 8) + align256(ns * 8) + align256(ni * 8) + align256(nx * 8), &buf);
+  st = scratch(ctx, (ne + ns + ni + nx) * 8, &buf);
   if (st) return st;
-  Carver cv{(char *)buf};
-  double *d_el = cv.take<double>(ne), *d_sel = cv.take<double>(ns), *d_ion = cv.take<double>(ni),
-         *d_exc = cv.take<double>(nx);
-  GASATT_CUDA(ctx, cudaMemcpyAsync(d_el, tab->t_el, ne * 8, cudaMemcpyHostToDevice, ctx->stream));
-  GASATT_CUDA(ctx, cudaMemcpyAsync(d_sel, tab->t_sel, ns * 8, cudaMemcpyHostToDevice, ctx->stream));
-  GASATT_CUDA(ctx, cudaMemcpyAsync(d_ion, tab->t_ion, ni * 8, cudaMemcpyHostToDevice, ctx->stream));
-  GASATT_CUDA(ctx, cudaMemcpyAsync(d_exc, tab->t_exc, nx * 8, cudaMemcpyHostToDevice, ctx->stream));
-  XsRaw t{d_el, tab->n_el, d_sel, tab->n_sel, d_ion, tab->n_ion, d_exc, tab->n_exc};
+  // one upload of the four tables
+  std::vector<double> host(ne + ns + ni + nx);
+  std::memcpy(host.data(), tab->t_el, ne * 8);
+  std::memcpy(host.data() + ne, tab->t_sel, ns * 8);
+  std::memcpy(host.data() + ne + ns, tab->t_ion, ni * 8);
+  std::memcpy(host.data() + ne + ns + ni, tab->t_exc, nx * 8);
+  const double *d = (const double *)buf;
+  GASATT_CUDA(ctx, cudaMemcpyAsync(buf, host.data(), host.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
+  XsRaw t{d, tab->n_el, d + ne, tab->n_sel, d + ne + ns, tab->n_ion, d + ne + ns + ni, tab->n_exc};
   k_find_cs0<<<grid_for(n, kBlock), kBlock, 0, ctx->stream>>>(t, E_keV, n, sig_el, sig_ion, sig_exc, flags);
   GASATT_LAUNCHED(ctx);
   GASATT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1089,54 +1241,72 @@ int gasatt_electron_collision(gasatt_ctx *ctx, double *e_pos, double *e_vel, int
   if (!ctx) return GASATT_E_ARG;
   if (n_e < 0 || cap_e < n_e || n_i1 < 0 || cap_i1 < n_i1 || rmax < 1 || cellnumxy < 1 || ncell < 1)
     return fail(ctx, GASATT_E_ARG, "electron_collision: bad sizes");
-  ElasticTables el;
   std::string err;
-  int st = build_elastic_tables(tab, el, err);
+  int st = check_tables(tab, err);
   if (st) return fail(ctx, st, err);
   GASATT_CUDA(ctx, cudaSetDevice(ctx->device));
-  std::vector<int> sc0(rmax + 1);
-  std::vector<double> dphi(rmax);
-  sc0[0] = 0;                                           // electron_collision.m:53-54
-  for (int i = 0; i < rmax; ++i) { sc0[i + 1] = (int)sum_cell[i]; dphi[i] = PHIp * 1 / phimax[i]; }
   const int64_t n = n_e;
+  const int ne = tab->n_sel1 - 1 + tab->n_el;
+  // one upload: the raw tables, the azimuthal cell widths and the rings' first
+  // cells (electron_collision.m:53-54)
+  const size_t len[6] = {2 * (size_t)tab->n_sel1, 2 * (size_t)tab->n_el, 182 * (size_t)tab->sdel_cols,
+                         182 * (size_t)tab->del_cols, 5 * (size_t)tab->n_exc, (size_t)rmax};
+  size_t off[7] = {0};
+  for (int i = 0; i < 6; ++i) off[i + 1] = off[i] + len[i];
+  std::vector<double> host(off[6] + (size_t)(rmax + 2) / 2);
+  const double *src[5] = {tab->t_sel_1, tab->t_el, tab->t_sdel, tab->t_del, tab->t_exc};
+  for (int i = 0; i < 5; ++i) std::memcpy(host.data() + off[i], src[i], len[i] * 8);
+  int *sc0 = reinterpret_cast<int *>(host.data() + off[6]);
+  sc0[0] = 0;
+  for (int i = 0; i < rmax; ++i) {
+    sc0[i + 1] = (int)sum_cell[i];
+    host[off[5] + i] = PHIp * 1 / phimax[i];
+  }
   const size_t sc = scan_tmp_bytes(n + 1);
-  const size_t bytes = align256(el.xInterp.size() * 8) * 2 + align256(el.V.size() * 8) +
-                       align256((size_t)5 * tab->n_exc * 8) + align256((size_t)rmax * 8) +
-                       align256((size_t)(rmax + 1) * 4) + align256((size_t)(n + 1)) +
-                       7 * align256((size_t)(n + 1) * 8) + 2 * align256((size_t)(n + 1) * 4) +
+  const size_t bytes = align256(host.size() * 8) + 2 * align256((size_t)ne * 8) + align256((size_t)ne * 181 * 8) +
+                       align256(8) + 7 * align256((size_t)(n + 1) * 8) + 4 * align256((size_t)(n + 1) * 4) +
                        align256(sc);
   void *buf;
   st = scratch(ctx, bytes, &buf);
   if (st) return st;
   Carver cv{(char *)buf};
-  double *d_xI = cv.take<double>(el.ne), *d_yI = cv.take<double>(el.ne), *d_V = cv.take<double>(el.V.size());
-  double *d_exc = cv.take<double>(5 * tab->n_exc), *d_dphi = cv.take<double>(rmax);
-  int *d_sc0 = cv.take<int>(rmax + 1);
+  double *d_host = cv.take<double>(host.size());
+  double *d_xI = cv.take<double>(ne), *d_yI = cv.take<double>(ne), *d_V = cv.take<double>((size_t)ne * 181);
+  MccLists ls;
+  ls.n = cv.take<unsigned>(2);
   MccOut out;
-  out.sec = cv.take<uint8_t>(n + 1);
   double **o7[7] = {&out.svx, &out.svy, &out.svz, &out.sample, &out.ivx, &out.ivy, &out.ivz};
   for (int i = 0; i < 7; ++i) *o7[i] = cv.take<double>(n + 1);
-  int *flag_i = cv.take<int>(n + 1), *posb = cv.take<int>(n + 1);
+  out.sec = cv.take<int>(n + 1);
+  int *posb = cv.take<int>(n + 1);
+  ls.elastic = cv.take<int>(n + 1);
+  ls.other = cv.take<int>(n + 1);
   void *tmp = cv.take<char>(sc);
   cudaStream_t s = ctx->stream;
-  GASATT_CUDA(ctx, cudaMemcpyAsync(d_xI, el.xInterp.data(), el.ne * 8, cudaMemcpyHostToDevice, s));
-  GASATT_CUDA(ctx, cudaMemcpyAsync(d_yI, el.yInterp.data(), el.ne * 8, cudaMemcpyHostToDevice, s));
-  GASATT_CUDA(ctx, cudaMemcpyAsync(d_V, el.V.data(), el.V.size() * 8, cudaMemcpyHostToDevice, s));
-  GASATT_CUDA(ctx, cudaMemcpyAsync(d_exc, tab->t_exc, (size_t)5 * tab->n_exc * 8, cudaMemcpyHostToDevice, s));
-  GASATT_CUDA(ctx, cudaMemcpyAsync(d_dphi, dphi.data(), (size_t)rmax * 8, cudaMemcpyHostToDevice, s));
-  GASATT_CUDA(ctx, cudaMemcpyAsync(d_sc0, sc0.data(), (size_t)(rmax + 1) * 4, cudaMemcpyHostToDevice, s));
-  MccTables t{d_xI, d_yI, d_V, el.ne, d_exc, tab->n_exc, d_dphi, d_sc0, rmax, cellnumxy,
-              density, temperature, ncell};
+  GASATT_CUDA(ctx, cudaMemcpyAsync(d_host, host.data(), host.size() * 8, cudaMemcpyHostToDevice, s));
+  GASATT_CUDA(ctx, cudaMemsetAsync(ls.n, 0, 8, s));
+  MccTables t{d_xI, d_yI, d_V, ne, d_host + off[4], tab->n_exc, d_host + off[5],
+              reinterpret_cast<const int *>(d_host + off[6]), rmax, cellnumxy, density, temperature, ncell};
   const int64_t call = ctx->mcc_calls++;
   if (n > 0) {
-    k_electron_transport<<<grid_for(n, kBlock), kBlock, 0, s>>>(
-        e_pos, e_vel, cap_e, n, sig_el, sig_ion, sig_exc, electron_kinetic, t, out, dr, dz,
-        dt_transport, draws, ctx->seed, call, flags);
+    k_collision_tables<<<(ne * 182 + kBlock - 1) / kBlock, kBlock, 0, s>>>(
+        MccRaw{d_host, d_host + off[1], d_host + off[2], d_host + off[3], tab->n_sel1, tab->n_el, tab->sdel_cols,
+               tab->del_cols}, d_xI, d_yI, d_V);
     GASATT_LAUNCHED(ctx);
+    k_collision_select<<<grid_for(n + 1, kBlock), kBlock, 0, s>>>(
+        e_pos, e_vel, cap_e, n, sig_el, sig_ion, sig_exc, electron_kinetic, t, out, ls, dr, dz, dt_transport, draws,
+        ctx->seed, call, flags);
+    GASATT_LAUNCHED(ctx);
+    k_collision_other<<<grid_for(n, kElThreads), kElThreads, 0, s>>>(e_vel, cap_e, electron_kinetic, t, out, ls, draws,
+                                                                    ctx->seed, call, flags);
+    GASATT_LAUNCHED(ctx);
+    k_collision_elastic<<<grid_for(n, kElGroup, 4u * 148u), kElThreads, kElSmem, s>>>(
+        e_vel, cap_e, electron_kinetic, t, ls, draws, ctx->seed, call, flags);
+    GASATT_LAUNCHED(ctx);
+  } else {
+    GASATT_CUDA(ctx, cudaMemsetAsync(out.sec, 0, 4, s));
   }
-  k_u8_to_int<<<grid_for(n + 1, kBlock), kBlock, 0, s>>>(out.sec, n, flag_i);
-  GASATT_LAUNCHED(ctx);
-  st = exclusive_scan(ctx, flag_i, posb, n + 1, tmp, sc);
+  st = exclusive_scan(ctx, out.sec, posb, n + 1, tmp, sc);
   if (st) return st;
   GASATT_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, posb + n, 4, cudaMemcpyDeviceToHost, s));
   GASATT_CUDA(ctx, cudaStreamSynchronize(s));
