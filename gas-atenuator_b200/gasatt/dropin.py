@@ -82,11 +82,8 @@ def _p(t):
 
 
 def _tables(**override):
-    base = N2Tables()
-    if override:
-        return N2Tables(**{k: np.asarray(v.cpu() if torch.is_tensor(v) else v, dtype=np.float64)
-                           for k, v in override.items()})
-    return base
+    return N2Tables(**{k: np.asarray(v.cpu() if torch.is_tensor(v) else v, dtype=np.float64)
+                       for k, v in override.items()})
 
 
 def find_CS0(t_el, t_sel, t_ion, t_exc, E_PE, *, flags=FAITHFUL, device=0):

@@ -10,15 +10,28 @@ DATA = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
                     "n2_tables.npz")
 
 
+_packaged = {}      # the packaged file's arrays, read once per process
+
+
+def _raw(path):
+    if path != DATA:
+        return np.load(path)
+    if not _packaged:
+        with np.load(DATA) as z:
+            _packaged.update({k: z[k] for k in z.files})
+    return _packaged
+
+
 class N2Tables:
-    """Holds the seven raw tables in Fortran order and a gasatt_tables view."""
+    """Holds the seven raw tables in Fortran order and a gasatt_tables view
+    (each object has its own copy of the packaged tables)."""
 
     NAMES = ("t_el", "t_sel", "t_sel_1", "t_del", "t_sdel", "t_ion", "t_exc")
 
     def __init__(self, path=DATA, **override):
-        z = np.load(path)
-        self.arrays = {k: np.asfortranarray(override.get(k, z[k]), dtype=np.float64)
-                       for k in self.NAMES}
+        z = _raw(path)
+        self.arrays = {k: np.asfortranarray(override[k], dtype=np.float64) if k in override else
+                       np.array(z[k], dtype=np.float64, order="F") for k in self.NAMES}
         a = self.arrays
         p = lambda k: a[k].ctypes.data_as(ctypes.c_void_p)
         self.struct = Tables(p("t_el"), a["t_el"].shape[1], p("t_sel"), a["t_sel"].shape[0],
