@@ -571,7 +571,7 @@ __device__ __forceinline__ void drift64(const SimParams &P, double dt, double &r
 // 3 x 3 nodes around a warp's particles are in nine.
 constexpr int kWin64Nodes = 3072;
 constexpr int kWin64Bytes = kWin64Nodes * 16;
-constexpr int kWin64Cols = 256;           // columns of the box at most (wide grids)
+constexpr int kWinCols = 256;             // columns of a deposit box at most (wide grids)
 constexpr int kChunk64 = 4608;            // particles per chunk at most
 
 struct Win64 {
@@ -579,8 +579,8 @@ struct Win64 {
   int row0, rows, col0, cols, ws;
 };
 
-__host__ __device__ inline int win64_cols(int nr) { return nr < kWin64Cols ? nr : kWin64Cols; }
-__host__ __device__ inline int win64_stride(int cols) { return cols + ((3 - cols % 32) + 32) % 32; }
+__host__ __device__ inline int win_cols(int nr) { return nr < kWinCols ? nr : kWinCols; }
+__host__ __device__ inline int win_stride(int cols) { return cols + ((3 - cols % 32) + 32) % 32; }
 
 // Box of a chunk: the rows of its first and last live particles (row_lo..row_hi;
 // row_hi < 0: none live) plus up to three rows either side for the drift
@@ -611,7 +611,7 @@ __device__ __forceinline__ void box64(const SimParams &P, const State64 &S, long
     lo = min(lo, k);
     hi = max(hi, k);
   }
-  chunk_box(P.nr, P.nz, win64_cols(P.nr), maxrows, lo, hi, col, row0, rows, col0);
+  chunk_box(P.nr, P.nz, win_cols(P.nr), maxrows, lo, hi, col, row0, rows, col0);
 }
 
 __device__ __forceinline__ void win64_add(unsigned *w, double v) {
@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_pass64(SimParams P, State64 S, Fi
   const long long step = cnt->step;
   if (blockIdx.x == 0 && threadIdx.x == 0) cnt->uncommitted = 1;
   const int chunk = even_chunk((unsigned)n0, gridDim.x, kChunk64);
-  const int cols = win64_cols(P.nr), ws = win64_stride(cols), maxrows = min(kWin64Nodes / ws, P.nz);
+  const int cols = win_cols(P.nr), ws = win_stride(cols), maxrows = min(kWin64Nodes / ws, P.nz);
   // the window starts zeroed; each chunk's flush leaves it zeroed again
   for (int i = threadIdx.x; i < kWin64Nodes; i += kBlock) reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0, 0, 0, 0);
   // the blocks take the chunks in turn, so neighbouring blocks work on
@@ -935,7 +935,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_batch_pass64(const BatchCell64 *_
     span(next, C, beg, end);
     const SimParams &Pc = C->P[jb];
     prefetch_chunk64(C->S[cur], beg, end);
-    box64(Pc, C->S[cur], beg, end, min(kWin64Nodes / win64_stride(win64_cols(Pc.nr)), Pc.nz), next_row0,
+    box64(Pc, C->S[cur], beg, end, min(kWin64Nodes / win_stride(win_cols(Pc.nr)), Pc.nz), next_row0,
           next_rows, next_col0);
   };
   if (threadIdx.x == 0) {
@@ -965,8 +965,8 @@ __global__ void __launch_bounds__(kBlock, 3) k_batch_pass64(const BatchCell64 *_
       __syncthreads();
       if (threadIdx.x == 0) cell_at = c;
     }
-    const int cols = win64_cols(sP.nr);
-    const Win64 w{reinterpret_cast<unsigned *>(smem), box_row0, box_rows, box_col0, cols, win64_stride(cols)};
+    const int cols = win_cols(sP.nr);
+    const Win64 w{reinterpret_cast<unsigned *>(smem), box_row0, box_rows, box_col0, cols, win_stride(cols)};
     chunk64<0>(sP, C->S[cur], C->F[jb], C->cnt, C->queue, q, C->cnt->step, (int)beg, (int)end, w, &box_cmax);
     if (threadIdx.x == 0) resolve();
     __syncthreads();
@@ -1261,28 +1261,22 @@ __device__ __forceinline__ void drift32(int &ir, int &iz, float &fr, float &fz, 
   reflect_z(iz, fz, uz, P.nz);
 }
 
-// The four deposit nodes (columns ca, cb; rows ra, rb; clamped one-sided at
-// the edges as EM7.cu:56-202) and the fixed-point contributions.  perm (0..3)
-// permutes the node order: bit 0 swaps the columns, bit 1 the rows, so the
-// order is (c0,r0), (c1,r0), (c0,r1), (c1,r1) with (c0, c1) = (ca, cb) or
-// (cb, ca) and likewise rows; each node's integer is the same whatever the
-// order (its weight is the same product of the same two factors).  The
+// The fixed-point contributions to the four deposit nodes (columns ar, ar + 1,
+// rows az, az + 1; clamped one-sided at the edges as EM7.cu:56-202, see
+// clamp_nodes).  perm (0..3) permutes the node order: bit 0 swaps the columns,
+// bit 1 the rows, so the order is (c0,r0), (c1,r0), (c0,r1), (c1,r1) with (c0,
+// c1) = (ar, ar + 1) or (ar + 1, ar) and likewise rows; each node's integer is the same
+// whatever the order (its weight is the same product of the same two factors).  The
 // weights sum to 1, so one particle adds at most 2^20 in magnitude to any
 // node, even where clamped nodes merge.  ig: 1/gamma of u (the drift's,
 // which turns u without changing |u|).
-__device__ __forceinline__ void deposit_nodes32(const SimParams &P, int ir, int iz, float fr,
-                                                float fz, float ur, float uz, float ig, int perm,
-                                                int &c0, int &c1, int &r0, int &r1, int vr[4],
-                                                int vz[4]) {
-  int ar, az;
+__device__ __forceinline__ void deposit_values32(const SimParams &P, int ir, int iz, float fr, float fz,
+                                                 float ur, float uz, float ig, int perm, int &ar, int &az,
+                                                 int vr[4], int vz[4]) {
   float wr, wz;
   half_shift(ir, fr, ar, wr);
   half_shift(iz, fz, az, wz);
-  const int ca = max(ar, 0), cb = min(ar + 1, P.nr - 1);
-  const int ra = max(az, 0), rb = min(az + 1, P.nz - 1);
   const bool sc = perm & 1, sr = perm & 2;
-  c0 = sc ? cb : ca; c1 = sc ? ca : cb;
-  r0 = sr ? rb : ra; r1 = sr ? ra : rb;
   const float2 om = __fadd2_rn(f2(1.f), f2(-wr, -wz));        // (1 - wr, 1 - wz)
   const float2 A = sc ? f2(wr, om.x) : f2(om.x, wr);         // column factors of c0, c1
   const float B0 = sr ? wz : om.y, B1 = sr ? om.y : wz;       // row factors of r0, r1
@@ -1297,28 +1291,42 @@ __device__ __forceinline__ void deposit_nodes32(const SimParams &P, int ir, int 
   vr[3] = __float_as_int(v3.x) - 0x4B400000; vz[3] = __float_as_int(v3.y) - 0x4B400000;
 }
 
-// FP32-form deposit window: int32 sums of one chunk of particles on the grid
-// rows [row0, row0 + rows) in shared memory.  A chunk holds at most kChunkMax
+__device__ __forceinline__ void clamp_nodes(const SimParams &P, int ar, int az, int perm, int &c0, int &c1,
+                                            int &r0, int &r1) {
+  const int ca = max(ar, 0), cb = min(ar + 1, P.nr - 1);
+  const int ra = max(az, 0), rb = min(az + 1, P.nz - 1);
+  const bool sc = perm & 1, sr = perm & 2;
+  c0 = sc ? cb : ca; c1 = sc ? ca : cb;
+  r0 = sr ? rb : ra; r1 = sr ? ra : rb;
+}
+
+// FP32-form deposit window: int32 sums of one chunk of particles on a box of
+// the grid in shared memory (chunk_box).  A chunk holds at most kChunkMax
 // particles, so a node's window sum stays below kChunkMax * 2^20 < 2^31.  A
 // node's two sums (r, z) are adjacent words, so one address serves both
-// atomics; rows are ws >= nr nodes apart with ws = 3 (mod 32), so the 3 x 3
+// atomics; rows are ws >= cols nodes apart with ws = 3 (mod 32), so the 3 x 3
 // nodes around a warp's particles sit in 9 different bank pairs.  Nodes
 // outside the window go straight to the grid with 64-bit atomics; the window
 // is added to the grid with one 64-bit atomic per touched node.
+// WIDE: the grid has more than kWinCols columns and the box only a part of
+// them, but 15 rows.  With all columns a 1024-wide grid had 3 rows, which the
+// electrons leave between two sorts: 16M electrons, step 495 us, now 423.  A
+// box of all columns needs no column test (on 256 columns the test and the
+// register for the box's first column cost 0.7 us of 55).
 constexpr int kWinNodes = 4096;           // nodes (two int32 sums each)
+constexpr int64_t kQuadCells = 1300000;   // cells of a grid with gather quads at most: 62 MB, half of L2
 
 struct Win32 {
   int *rz;                  // node k: r at rz[2k], z at rz[2k + 1]
-  int row0, rows, ws;
+  int row0, rows, col0, cols, ws;
 };
 
-__host__ __device__ inline int win_stride(int nr) { return nr + ((3 - nr % 32) + 32) % 32; }
-
+template <bool WIDE>
 __device__ __forceinline__ void win_node(const Win32 &w, const SimParams &P, int col, int row,
                                          int vr, int vz) {
-  const unsigned lr = (unsigned)(row - w.row0);
-  if (lr < (unsigned)w.rows) {
-    const int k = (int)lr * w.ws + col;
+  const unsigned lr = (unsigned)(row - w.row0), lc = (unsigned)(col - w.col0);
+  if (lr < (unsigned)w.rows && (!WIDE || lc < (unsigned)w.cols)) {
+    const int k = (int)lr * w.ws + (int)lc;
     atomicAdd(w.rz + 2 * k, vr);
     atomicAdd(w.rz + 2 * k + 1, vz);
   } else {
@@ -1411,8 +1419,9 @@ __device__ __forceinline__ bool push32(const SimParams &P, const Fields<float> &
 // the same integers whichever path pushed it
 __device__ __forceinline__ void deposit_global32(const SimParams &P, int ir, int iz, float fr,
                                                  float fz, float ur, float uz, float ig) {
-  int ca, cb, ra, rb, vr[4], vz[4];
-  deposit_nodes32(P, ir, iz, fr, fz, ur, uz, ig, 0, ca, cb, ra, rb, vr, vz);
+  int ar, az, ca, cb, ra, rb, vr[4], vz[4];
+  deposit_values32(P, ir, iz, fr, fz, ur, uz, ig, 0, ar, az, vr, vz);
+  clamp_nodes(P, ar, az, 0, ca, cb, ra, rb);
   const int64_t a[4] = {ca + (int64_t)ra * P.ldj, cb + (int64_t)ra * P.ldj,
                         ca + (int64_t)rb * P.ldj, cb + (int64_t)rb * P.ldj};
   deposit_atomic<int>(a, vr, vz, P.Jr, P.Jz);
@@ -1485,28 +1494,15 @@ __device__ __noinline__ void candidate32(const SimParams *__restrict__ Pg, Field
   if (kid) S.id[p] = id;
 }
 
-// Window rows of chunk ch (particles [ch chunk, min(ch chunk + chunk, n0))):
-// the node rows of its first and last particles, with a margin for the drift
-// since the last sort.  maxrows: rows the window holds for this grid.
-__device__ __forceinline__ void chunk_rows32(const SimParams &P, const State32 &S, long long n0,
-                                             int chunk, long long ch, int maxrows, int &row0,
-                                             int &rows) {
-  const long long beg = ch * chunk, end = min(beg + chunk, n0);
+// Box of the particles [beg, end) (chunk_box) from the cells of the first and last one
+__device__ __forceinline__ void box32(const SimParams &P, const State32 &S, long long beg, long long end,
+                                      int cols, int maxrows, int &row0, int &rows, int &col0) {
   const uint32_t k0 = reinterpret_cast<const uint32_t *>(S.a + beg)[0];
   const uint32_t k1 = reinterpret_cast<const uint32_t *>(S.a + end - 1)[0];
-  int lo = P.nz, hi = -1;
-  if (k0 != kDead) { lo = min(lo, (int)(k0 >> 16)); hi = max(hi, (int)(k0 >> 16)); }
+  int lo = P.nz, hi = -1, col = 0;
+  if (k0 != kDead) { lo = hi = (int)(k0 >> 16); col = (int)(k0 & 0xFFFFu); }
   if (k1 != kDead) { lo = min(lo, (int)(k1 >> 16)); hi = max(hi, (int)(k1 >> 16)); }
-  row0 = 0; rows = maxrows;
-  if (hi >= 0) {
-    // the chunk's own deposit rows lo-1 .. hi+1 first, then up to three
-    // rows either side for the drift since the last sort (a wide grid
-    // leaves room for few rows)
-    const int core = hi - lo + 3;
-    const int below = maxrows >= core + 6 ? 3 : max(1, 1 + (maxrows - core) / 2);
-    row0 = min(max(0, lo - below), P.nz - maxrows);
-    rows = min(maxrows, hi + 4 - row0);
-  }
+  chunk_box(P.nr, P.nz, cols, maxrows, lo, hi, col, row0, rows, col0);
 }
 
 __device__ __forceinline__ void prefetch_chunk32(const State32 &S, long long beg, long long end) {
@@ -1521,7 +1517,7 @@ __device__ __forceinline__ void prefetch_chunk32(const State32 &S, long long beg
 // push (push32), collision candidates queued, deposit into the window w
 // (nodes outside the window straight to the grid).  The highest window column touched is merged
 // into *box_cmax; electrons absorbed at the wall are counted into cnt.
-template <int MODE>
+template <int MODE, bool WIDE>
 __device__ __forceinline__ void chunk32(const SimParams &P, const State32 &S, const Fields<float> &F,
                                         SimCounters *cnt, int *queue, long long step,
                                         int beg, int end, const Win32 &w, int *box_cmax) {
@@ -1573,30 +1569,32 @@ __device__ __forceinline__ void chunk32(const SimParams &P, const State32 &S, co
     // nodes in each atomic.  (Summing the lanes of a quad first with
     // match.any / redux.sync made this pass two to four times slower on B200.)
     if (act) {
-      int c0, c1, r0, r1, vr[4], vz[4];
-      deposit_nodes32(P, ir, iz, fr, fz, ur, uz, ig, lane & 3, c0, c1, r0, r1, vr, vz);
-      const unsigned l0 = (unsigned)(r0 - w.row0), l1 = (unsigned)(r1 - w.row0);
-      if (l0 < (unsigned)w.rows && l1 < (unsigned)w.rows) {
-        const int k0 = (int)l0 * w.ws, k1 = (int)l1 * w.ws;
-        int *n00 = w.rz + 2 * (k0 + c0), *n10 = w.rz + 2 * (k0 + c1);
-        int *n01 = w.rz + 2 * (k1 + c0), *n11 = w.rz + 2 * (k1 + c1);
-        atomicAdd(n00, vr[0]); atomicAdd(n00 + 1, vz[0]);
-        atomicAdd(n10, vr[1]); atomicAdd(n10 + 1, vz[1]);
-        atomicAdd(n01, vr[2]); atomicAdd(n01 + 1, vz[2]);
-        atomicAdd(n11, vr[3]); atomicAdd(n11 + 1, vz[3]);
+      int ar, az, vr[4], vz[4];
+      deposit_values32(P, ir, iz, fr, fz, ur, uz, ig, lane & 3, ar, az, vr, vz);
+      const int a = ar - (WIDE ? w.col0 : 0), b = az - w.row0;
+      int c0, c1, r0, r1;
+      if ((unsigned)a < (unsigned)(w.cols - 1) && (unsigned)b < (unsigned)(w.rows - 1)) {
+        // all four nodes in the box and on the grid (no clamping)
+        const int dc = lane & 1, dr = lane & 2 ? w.ws : 0;
+        int *n0 = w.rz + 2 * (b * w.ws + a + dr), *n1 = w.rz + 2 * (b * w.ws + a + w.ws - dr);
+        atomicAdd(n0 + 2 * dc, vr[0]); atomicAdd(n0 + 2 * dc + 1, vz[0]);
+        atomicAdd(n0 + 2 - 2 * dc, vr[1]); atomicAdd(n0 + 3 - 2 * dc, vz[1]);
+        atomicAdd(n1 + 2 * dc, vr[2]); atomicAdd(n1 + 2 * dc + 1, vz[2]);
+        atomicAdd(n1 + 2 - 2 * dc, vr[3]); atomicAdd(n1 + 3 - 2 * dc, vz[3]);
       } else {
-        win_node(w, P, c0, r0, vr[0], vz[0]);
-        win_node(w, P, c1, r0, vr[1], vz[1]);
-        win_node(w, P, c0, r1, vr[2], vz[2]);
-        win_node(w, P, c1, r1, vr[3], vz[3]);
+        clamp_nodes(P, ar, az, lane & 3, c0, c1, r0, r1);
+        win_node<WIDE>(w, P, c0, r0, vr[0], vz[0]);
+        win_node<WIDE>(w, P, c1, r0, vr[1], vz[1]);
+        win_node<WIDE>(w, P, c0, r1, vr[2], vz[2]);
+        win_node<WIDE>(w, P, c1, r1, vr[3], vz[3]);
       }
-      wc_max = max(wc_max, max(c0, c1));   // (win_node may use the window for one row)
+      wc_max = max(wc_max, a + 1);   // (win_node may use the window for one row or column)
     }
   }
   // the window columns this warp touched, merged into the block's; the wall
   // losses of the warp
   wc_max = __reduce_max_sync(0xFFFFFFFFu, wc_max);
-  if (lane == 0 && wc_max >= 0) atomicMax(box_cmax, wc_max);
+  if (lane == 0 && wc_max >= 0) atomicMax(box_cmax, min(wc_max, w.cols - 1));
   lost = __reduce_add_sync(0xFFFFFFFFu, lost);
   if (lane == 0 && lost) atomicAdd(&cnt->lost, (unsigned long long)lost);
 }
@@ -1611,7 +1609,7 @@ __device__ __forceinline__ void flush32(const SimParams &P, const Win32 &w, int 
     const int2 v = reinterpret_cast<const int2 *>(w.rz)[k];
     const int vr = v.x, vz = v.y;
     if (vr | vz) {
-      const int64_t g = (int64_t)(w.row0 + row) * P.ldj + col;
+      const int64_t g = (int64_t)(w.row0 + row) * P.ldj + w.col0 + col;
       if (vr) atomicAdd(P.Jr + g, (unsigned long long)(long long)vr);
       if (vz) atomicAdd(P.Jz + g, (unsigned long long)(long long)vz);
       reinterpret_cast<int2 *>(w.rz)[k] = make_int2(0, 0);
@@ -1629,13 +1627,13 @@ constexpr int kCandLanes = 8;     // collision candidates a warp of the pass tak
 // P.chunk handed out in order, so the blocks that ran candidates simply take
 // fewer chunks.  Counters are committed by the field
 // kernel of the next step.
-template <int MODE>
+template <int MODE, bool WIDE>
 __global__ void __launch_bounds__(kBlock, 4) k_pass32(SimParams P, State32 S, Fields<float> F,
                                                       SimCounters *cnt, int *queue,
                                                       const SimParams *__restrict__ Pg) {
   constexpr int mode = MODE;
   __shared__ __align__(16) int win_rz[2 * kWinNodes];
-  __shared__ int win_row0, win_rows;
+  __shared__ int win_row0, win_rows, win_col0;
   __shared__ int box_cmax;                       // highest window column the chunk touched
   __shared__ long long chunk_at;
   const long long n0 = (long long)cnt->n_total;   // births of this pass land beyond
@@ -1644,7 +1642,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_pass32(SimParams P, State32 S, Fi
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // the window starts zeroed; each chunk's flush leaves it zeroed again
   for (int i = threadIdx.x; i < kWinNodes; i += kBlock) reinterpret_cast<int2 *>(win_rz)[i] = make_int2(0, 0);
-  const int ws = win_stride(P.nr);
+  const int cols = win_cols(P.nr), ws = win_stride(cols);
   const int maxrows = min(kWinNodes / ws, P.nz);
   const int chunk = max(cnt->chunk, kBlock);      // chosen with the commit (no division here)
   if (mode != 1) {
@@ -1669,18 +1667,19 @@ __global__ void __launch_bounds__(kBlock, 4) k_pass32(SimParams P, State32 S, Fi
   // thread 0 claims the block's next chunk (index and window rows) a chunk
   // ahead and has its state brought into L2 meanwhile
   long long next_ch = 0;
-  int next_row0 = 0, next_rows = 0;
+  int next_row0 = 0, next_rows = 0, next_col0 = 0;
   if (threadIdx.x == 0) {
     next_ch = (long long)atomicAdd(&cnt->chunk_next, 1ull);
     if (next_ch * chunk < n0) prefetch_chunk32(S, next_ch * chunk, min((next_ch + 1) * chunk, n0));
   }
   if (threadIdx.x == 0 && next_ch * chunk < n0)
-    chunk_rows32(P, S, n0, chunk, next_ch, maxrows, next_row0, next_rows);
+    box32(P, S, next_ch * chunk, min((next_ch + 1) * chunk, n0), cols, maxrows, next_row0, next_rows, next_col0);
   for (;;) {
     if (threadIdx.x == 0) {
       chunk_at = next_ch;
       win_row0 = next_row0;
       win_rows = next_rows;
+      if (WIDE) win_col0 = next_col0;
       box_cmax = -1;
     }
     __syncthreads();
@@ -1692,11 +1691,11 @@ __global__ void __launch_bounds__(kBlock, 4) k_pass32(SimParams P, State32 S, Fi
     if (threadIdx.x == 0) next_ch = (long long)atomicAdd(&cnt->chunk_next, 1ull);
     // 32-bit slot indices: the capacity is below 2^31
     const int beg = (int)(ch * chunk), end = (int)min((long long)beg + chunk, n0);
-    const Win32 w{win_rz, win_row0, win_rows, ws};
-    chunk32<MODE>(P, S, F, cnt, queue, step, beg, end, w, &box_cmax);
+    const Win32 w{win_rz, win_row0, win_rows, WIDE ? win_col0 : 0, WIDE ? cols : P.nr, ws};
+    chunk32<MODE, WIDE>(P, S, F, cnt, queue, step, beg, end, w, &box_cmax);
     if (threadIdx.x == 0 && next_ch * chunk < n0) {
       prefetch_chunk32(S, next_ch * chunk, min((next_ch + 1) * chunk, n0));
-      chunk_rows32(P, S, n0, chunk, next_ch, maxrows, next_row0, next_rows);
+      box32(P, S, next_ch * chunk, min((next_ch + 1) * chunk, n0), cols, maxrows, next_row0, next_rows, next_col0);
     }
     __syncthreads();
     flush32(P, w, box_cmax + 1);
@@ -1723,12 +1722,13 @@ struct BatchCell32 {
 // (*chunk_next, zeroed before the launch), copying the cell's parameters into
 // shared memory when the cell changes.  Every cell gives what its own
 // k_pass32 gives.
+template <bool WIDE>
 __global__ void __launch_bounds__(kBlock, 4) k_batch_pass32(const BatchCell32 *__restrict__ cells,
                                                             int ncell, int cur, int jb,
                                                             unsigned long long *chunk_next) {
   constexpr int mode = 0;        // a batch only takes whole steps
   __shared__ __align__(16) int win_rz[2 * kWinNodes];
-  __shared__ int win_row0, win_rows, box_cmax, cell_at;
+  __shared__ int win_row0, win_rows, win_col0, box_cmax, cell_at;
   __shared__ long long chunk_at;
   __shared__ long long cand_pre[kMaxBatch + 1], chunk_pre[kMaxBatch + 1];
   __shared__ int cell_chunk[kMaxBatch];
@@ -1767,17 +1767,17 @@ __global__ void __launch_bounds__(kBlock, 4) k_batch_pass32(const BatchCell32 *_
   // (cell, chunk) work items; the block's first one is claimed (and its state
   // brought into L2) before the candidates
   long long next = 0;
-  int next_c = -1, next_row0 = 0, next_rows = 0;
+  int next_c = -1, next_row0 = 0, next_rows = 0, next_col0 = 0;
   auto resolve = [&]() {         // thread 0: the cell and window rows of the claimed item
     if (next < nchunk) {
       next_c = cell_of_item(chunk_pre, ncell, next);
       const BatchCell32 &C = cells[next_c];
       const SimParams &Pc = C.P[jb];
-      const int ws = win_stride(Pc.nr), maxrows = min(kWinNodes / ws, Pc.nz);
+      const int cols = win_cols(Pc.nr), maxrows = min(kWinNodes / win_stride(cols), Pc.nz);
       const long long n0c = (long long)C.cnt->n_total, chc = next - chunk_pre[next_c];
       const int chunk = cell_chunk[next_c];
       prefetch_chunk32(C.S[cur], chc * chunk, min((chc + 1) * chunk, n0c));
-      chunk_rows32(Pc, C.S[cur], n0c, chunk, chc, maxrows, next_row0, next_rows);
+      box32(Pc, C.S[cur], chc * chunk, min((chc + 1) * chunk, n0c), cols, maxrows, next_row0, next_rows, next_col0);
     }
   };
   if (threadIdx.x == 0) {
@@ -1804,6 +1804,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_batch_pass32(const BatchCell32 *_
       chunk_at = next;
       win_row0 = next_row0;
       win_rows = next_rows;
+      win_col0 = next_col0;
       box_cmax = -1;
     }
     __syncthreads();
@@ -1826,8 +1827,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_batch_pass32(const BatchCell32 *_
     const int chunk = cell_chunk[c];
     const long long ch = g - chunk_pre[c];
     const int beg = (int)(ch * chunk), end = (int)min((long long)beg + chunk, n0);
-    const Win32 w{win_rz, win_row0, win_rows, win_stride(sP.nr)};
-    chunk32<0>(sP, C.S[cur], C.F[jb], cc, C.queue, step, beg, end, w, &box_cmax);
+    const int cols = WIDE ? win_cols(sP.nr) : sP.nr;
+    const Win32 w{win_rz, win_row0, win_rows, WIDE ? win_col0 : 0, cols, win_stride(cols)};
+    chunk32<0, WIDE>(sP, C.S[cur], C.F[jb], cc, C.queue, step, beg, end, w, &box_cmax);
     if (threadIdx.x == 0) resolve();
     __syncthreads();
     flush32(sP, w, box_cmax + 1);
@@ -2550,7 +2552,9 @@ int launch_pass(gasatt_sim *s, cudaStream_t st, int mode, int jb, int q, int fb)
   }
   else
   {
-    auto kern = mode == 0 ? k_pass32<0> : mode == 1 ? k_pass32<1> : k_pass32<2>;
+    auto kern = win_cols(P.nr) < P.nr
+                    ? (mode == 0 ? k_pass32<0, true> : mode == 1 ? k_pass32<1, true> : k_pass32<2, true>)
+                    : (mode == 0 ? k_pass32<0, false> : mode == 1 ? k_pass32<1, false> : k_pass32<2, false>);
     kern<<<s->pass_grid, kBlock, 0, st>>>(P, s->s32[b], fields_of<float>(s, fb), s->cnt, s->queue,
                                           s->d_P + jb);
   }
@@ -3068,8 +3072,12 @@ int gasatt_sim_create(gasatt_ctx *ctx, const gasatt_sim_config *cfg, const gasat
     return cleanup(rc);
   // FP32 gather quads: 48 bytes more per cell written by every field update,
   // against nine fewer loads per electron; worth it where electrons are dense
+  // and the quads stay in L2 between the field update and the pass.  256 x 1024
+  // cells, 2M electrons: step 56.7 us with quads, 58.2 with the fields; 1024 x
+  // 4096 cells (200 MB of quads), 16M electrons: 525 and 493.
   const bool quads = s->form == 1 &&
-                     (c.gather == 1 || (c.gather == 0 && c.capacity >= 4 * (int64_t)(nr + 1) * (nz + 1)));
+                     (c.gather == 1 || (c.gather == 0 && (int64_t)(nr + 1) * (nz + 1) <= kQuadCells &&
+                                        c.capacity >= 4 * (int64_t)(nr + 1) * (nz + 1)));
   if (quads) {
     if ((rc = sim_alloc(s, &s->quads.er, (size_t)(nr + 1) * nz)) ||
         (rc = sim_alloc(s, &s->quads.ez, (size_t)nr * (nz + 1))) ||
@@ -3155,7 +3163,7 @@ int gasatt_sim_create(gasatt_ctx *ctx, const gasatt_sim_config *cfg, const gasat
         return cleanup(fail(ctx, GASATT_E_CUDA, "FP64 pass: shared memory"));
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pass64<0>, kBlock, kWin64Bytes);
   }
-  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pass32<0>, kBlock, 0);
+  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (k_pass32<0, false>), kBlock, 0);
   s->pass_grid = (unsigned)(nsm * (occ > 0 ? occ : 1));
   if (s->form == 1) {
     // FP32 blocks take chunks from a counter: no more blocks than chunks the
@@ -3904,6 +3912,7 @@ struct BatchGroup {
   unsigned long long *chunk_next = nullptr;
   unsigned fdtd_grid = 0, pass_grid = 0, mcc_grid = 0;
   size_t fdtd_smem = 0;
+  bool wide = false;                     // a cell's grid is wider than a deposit box
 };
 
 struct gasatt_batch {
@@ -4010,7 +4019,8 @@ int batch_group_setup(gasatt_batch *b, BatchGroup &G) {
   const long long fblocks = (G.nitems + kTmaWarps - 1) / kTmaWarps;
   G.fdtd_grid = (unsigned)(fslots < fblocks ? fslots : (fblocks > 0 ? fblocks : 1));
   occ = 1;
-  if (G.form == 1) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_pass32, kBlock, 0);
+  for (const gasatt_sim *s : G.sims) G.wide = G.wide || win_cols(s->cfg.n_r) < s->cfg.n_r;
+  if (G.form == 1) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_pass32<true>, kBlock, 0);
   else {
     GASATT_CUDA(ctx, cudaFuncSetAttribute(k_batch_pass64, cudaFuncAttributeMaxDynamicSharedMemorySize, kWin64Bytes));
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_pass64, kBlock, kWin64Bytes);
@@ -4034,8 +4044,8 @@ int batch_group_launch(gasatt_batch *b, BatchGroup &G, cudaStream_t cs, cudaStre
                                                                         G.commit, n);
     GASATT_CUDA(ctx, cudaGetLastError());
     GASATT_CUDA(ctx, cudaMemsetAsync(G.chunk_next, 0, 8, cs));
-    k_batch_pass32<<<G.pass_grid, kBlock, 0, cs>>>((const BatchCell32 *)G.cells, n, cur, 1 - q,
-                                                   G.chunk_next);
+    (G.wide ? k_batch_pass32<true> : k_batch_pass32<false>)<<<G.pass_grid, kBlock, 0, cs>>>(
+        (const BatchCell32 *)G.cells, n, cur, 1 - q, G.chunk_next);
     GASATT_CUDA(ctx, cudaGetLastError());
     return GASATT_OK;
   }

@@ -62,11 +62,14 @@ def test_fp64_pass_matches_oracle(tables, nr, nz, n, spread):
 # populations of one warp, around a block, around one chunk per block (592 x
 # 256 and 592 x 1792 electrons) and between; at 100 Torr 2% of the electrons are
 # collision candidates in each step, for idle and busy blocks alike
-@pytest.mark.parametrize("nr,nz,n", [(16, 20, 31), (16, 20, 257), (64, 64, 30_001), (64, 64, 151_553),
-                                     (64, 300, 400_000), (64, 300, 1_060_865)])
-def test_fp32_chunk_choice_changes_no_bit(nr, nz, n):
+@pytest.mark.parametrize("nr,nz,n,spread", [
+    (16, 20, 31, False), (16, 20, 257, False), (64, 64, 30_001, False), (64, 64, 151_553, False),
+    (64, 300, 400_000, False), (64, 300, 1_060_865, False),
+    # grids wider than a box: near its columns, one row per chunk, many rows per chunk
+    (257, 9, 20_001, True), (600, 6, 120_000, False), (600, 60, 30_000, True), (1100, 20, 300_000, True)])
+def test_fp32_chunk_choice_changes_no_bit(nr, nz, n, spread):
     """The chunk chosen from the population and fixed chunks give the same state, fields and counts."""
-    parts = population(n, nr, nz, False, seed=n)
+    parts = population(n, nr, nz, spread, seed=n)
     flds = grid_fields(nr, nz, np.random.default_rng(8), E0=3e6, H0=2e3)
     flds[0][:, 0] = 0; flds[0][:, -1] = 0; flds[1][-1, :] = 0
     ref = None
