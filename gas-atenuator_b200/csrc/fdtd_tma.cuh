@@ -1,28 +1,30 @@
 // fdtd_tma.cuh - the field sub-cycle of the resident simulation (fdtd_ratio 1):
-// one warp per patch, the patch staged by TMA, the sub-cycle in registers.
+// one block per patch, the patch staged by TMA, the sub-cycle in registers.
 //
 // One launch advances the fields by one particle step: H(dt/4), E(dt/2),
 // H(dt/2), E(dt/2), H(dt/4) (EM3_1.cu:2-17 and EM3.cu:2-43, called as the
 // sub-cycle of electricmagneticfield6.m:146-151), with the same arithmetic as
-// the reference-layout kernels of fdtd.cuh.
+// the general kernel of fdtd.cuh.
 //
 // Work: the grid (n_r + 1 columns x n_z + 1 rows of Yee points) is cut into
-// tiles of 26 columns x (R - 6) rows.  A warp owns a patch of 32 columns x R
+// tiles of 26 columns x (R - 6) rows.  A block owns a patch of 32 columns x R
 // rows around its tile (3 halo columns and rows on each side: the five
 // sub-updates need two on the low side and three on the high side, and one
-// more on the low side lets the warp assemble every gather quad of its tile
-// from values it computed).  Lane l holds column l of the patch - Er, Ez, H
-// and the two current terms of all R rows - in registers: vertical
-// neighbours are registers, horizontal ones are warp shuffles, so the warps
-// never wait on one another (no block barrier) and the halo is recomputed by
-// each warp instead of exchanged.
+// more on the low side lets it assemble every gather quad of its tile
+// from values it computed).  Each of its warps holds a segment of S
+// consecutive rows in registers - lane l column l: Er, Ez, H and the two
+// current terms - so vertical neighbours are registers and horizontal ones
+// shuffles; between segments one row of Er or H goes through shared memory per
+// update.  The halo is recomputed by each block instead of exchanged: 1.35 times
+// the points at R = 64.  (A warp per patch of 32 x 12 recomputed 2.5 times the
+// points: 1024 x 4096 cells in 59 us, 31M warp instructions.)
 //
-// Staging: one lane of each warp issues five 2D tensor copies (Er, Ez, H as
-// stored, Jr, Jz as 64-bit fixed point) of its patch into the warp's own
-// staging area, completing on the warp's mbarrier.  Once the lanes hold the
-// patch in registers the area is free, and the copies of the warp's next
-// patch go out before the current one is computed.  Warps walk the work items
-// warp-stride.  The tiles are written to a second set of fields: a patch
+// Staging: one thread of each block issues five 2D tensor copies (Er, Ez, H as
+// stored, Jr, Jz as 64-bit fixed point) of its patch into the block's staging
+// area, completing on its mbarrier.  Once the registers hold the patch the area
+// is free, and the copies of the block's next patch go out before the current
+// one is computed.  Blocks walk the work items grid-stride.  The tiles are
+// written to a second set of fields: a patch
 // staged after its neighbours' tiles were written still reads the old fields
 // in its halo.
 //
@@ -32,7 +34,7 @@
 // from there; a lane reads its column at that offset.  Points outside the
 // grid (negative or beyond the extent) arrive as zeros and are never updated.
 //
-// Every wait on an mbarrier is bounded; a warp whose copy has not completed
+// Every wait on an mbarrier is bounded; a block whose copy has not completed
 // after the bound sets the cell's *err, waits (bounded) once more for that
 // copy and returns.
 #pragma once
@@ -44,8 +46,25 @@ namespace gasatt {
 constexpr int kTmaTileW = 26;                 // output columns per tile
 constexpr int kTmaPatchW = 32;                // patch columns (one per lane)
 constexpr int kTmaHalo = 3;                   // halo columns / rows on each side
-constexpr int kTmaWarps = 1;                  // warps per block (each on its own patches)
 constexpr unsigned kTmaWaitLimit = 1u << 22;  // try_wait rounds before giving up
+
+// The patch of knob value K (fdtd_tile_rows): W warps of S rows each, and how
+// many blocks an SM is to hold.
+template <int K> struct TmaShape;
+template <> struct TmaShape<12> { static constexpr int W = 4, S = 4; };
+template <> struct TmaShape<16> { static constexpr int W = 8, S = 4; };
+template <> struct TmaShape<20> { static constexpr int W = 8, S = 8; };
+__host__ __device__ constexpr int tma_warps(int k) { return k == 12 ? 4 : 8; }
+__host__ __device__ constexpr int tma_rows(int k) { return k == 12 ? 16 : k == 16 ? 32 : 64; }
+__host__ __device__ constexpr int tma_blocks(int k) { return k == 12 ? 8 : k == 16 ? 4 : 2; }
+__host__ __device__ constexpr bool tma_rows_ok(int k) { return k == 12 || k == 16 || k == 20; }
+
+// tiles of a grid of n_r x n_z cells
+inline int tma_tiles_x(int nr) { return (nr + kTmaTileW) / kTmaTileW; }
+inline int tma_tiles(int k, int nr, int nz) {
+  const int h = tma_rows(k) - 2 * kTmaHalo;
+  return tma_tiles_x(nr) * ((nz + h) / h);
+}
 
 // staging box widths (elements): 32 columns from an aligned start below the
 // patch's first column
@@ -95,16 +114,15 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
 }
 
 // ------------------------------------------------------------ layout
-// One warp's staging area for R patch rows (Er, Ez, H in T, Jr, Jz in 64 bits;
-// each 128-byte aligned).  A block holds kTmaWarps areas, then one mbarrier
-// per warp.
+// A block's staging area for R patch rows (Er, Ez, H in T, Jr, Jz in 64 bits;
+// each 128-byte aligned), then its mbarrier.
 template <typename T, int R>
 struct TmaStage {
   static constexpr size_t up(size_t b) { return (b + 127) & ~(size_t)127; }
   static constexpr size_t field_bytes = up((size_t)TmaBox<T>::w * R * sizeof(T));
   static constexpr size_t cur_bytes = up((size_t)34 * R * 8);
   static constexpr size_t bytes = 3 * field_bytes + 2 * cur_bytes;
-  static constexpr size_t block_bytes = kTmaWarps * bytes + 128;
+  static constexpr size_t block_bytes = bytes + 128;
   // bytes one patch's five copies deliver (whole boxes, out-of-bounds fill included)
   static constexpr uint32_t tx_bytes =
       (uint32_t)(3 * (size_t)TmaBox<T>::w * R * sizeof(T) + 2 * (size_t)34 * R * 8);
@@ -159,7 +177,7 @@ __device__ __forceinline__ void tma_patch_origin(int t, int tiles_x, int rows, i
   y0 = ty * (rows - 2 * kTmaHalo) - kTmaHalo;
 }
 
-// issue the copies of work item t into a warp's staging area (one lane)
+// issue the copies of work item t into the staging area (one thread)
 template <typename T, int R>
 __device__ __forceinline__ void tma_issue_item(const FdtdWork &W, int t, unsigned char *stage,
                                                uint64_t *bar) {
@@ -179,32 +197,37 @@ __device__ __forceinline__ void tma_issue_item(const FdtdWork &W, int t, unsigne
 }
 
 // The sub-cycle on the work items of W (cells on the padded layout: row
-// strides ldf for the fields, ldj for the currents), R patch rows per warp.
+// strides ldf for the fields, ldj for the currents), patches of shape K.
 // The field arithmetic is that of fdtd_tiled (fdtd.cuh); the per-column
 // coefficients come from the cell's table, the current terms of the two E
 // updates are formed once per patch.
-template <typename T, int R>
-__device__ __forceinline__ void fdtd_warp_body(const FdtdWork &W) {
-  using S = TmaStage<T, R>;
-  static_assert(R > 2 * kTmaHalo && R <= 32, "patch rows");
+template <typename T, int K>
+__device__ __forceinline__ void fdtd_block_body(const FdtdWork &W) {
+  constexpr int NW = TmaShape<K>::W, S = TmaShape<K>::S, R = NW * S;
+  using St = TmaStage<T, R>;
+  static_assert(R == tma_rows(K) && NW == tma_warps(K) && S > kTmaHalo, "patch shape");
   constexpr int BW = TmaBox<T>::w, al = 16 / (int)sizeof(T);
   constexpr unsigned FULL = 0xFFFFFFFFu;
   extern __shared__ __align__(128) unsigned char smem[];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  unsigned char *stage = smem + wib * S::bytes;
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smem + kTmaWarps * S::bytes) + wib;
-  const int ntiles = W.ntiles, stride = gridDim.x * kTmaWarps;
-  int t = blockIdx.x * kTmaWarps + wib;
-  if (lane == 0) {
+  // the rows of a segment that its neighbours read: first and last Er (in two
+  // buffers by turns: an E update reads one while others write the other),
+  // last H and Ez
+  __shared__ double s_first[2][NW][32], s_last[2][NW][32], s_h[NW][32], s_ez[NW][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem + St::bytes);
+  const int ntiles = W.ntiles, stride = gridDim.x;
+  int t = blockIdx.x;
+  if (threadIdx.x == 0) {
     mbar_init(bar, 1);
     mbar_fence_init();
   }
-  __syncwarp();
-  if (lane == 0 && t < ntiles) tma_issue_item<T, R>(W, t, stage, bar);
+  __syncthreads();
+  if (threadIdx.x == 0 && t < ntiles) tma_issue_item<T, R>(W, t, smem, bar);
   for (int k = 0; t < ntiles; t += stride, ++k) {
     int lt, x0, y0;
     const FdtdInst &I = W.at(t, lt);
     tma_patch_origin(lt, I.tiles_x, R, x0, y0);
+    y0 += w * S;                           // the segment's first row
     const int nr = I.nr, nz = I.nz;
     const unsigned flags = I.flags;
     const bool endcopy = (flags & GASATT_Q_ER_END_COPY) != 0;
@@ -226,166 +249,166 @@ __device__ __forceinline__ void fdtd_warp_body(const FdtdWork &W) {
       ezp = col == 0 ? axis : I.colc[3 * col + 1];
       ezm = I.colc[3 * col + 2];            // 0 on the axis
     }
-    const bool ok = __all_sync(FULL, mbar_wait(bar, (uint32_t)(k & 1)));
+    const bool ok = __syncthreads_and(mbar_wait(bar, (uint32_t)(k & 1)));
     if (!ok) {
-      if (lane == 0) {
+      if (threadIdx.x == 0) {
         atomicOr(I.err, 1u);
         mbar_wait(bar, (uint32_t)(k & 1));          // the copy still owns the area
       }
       break;
     }
-    // the column's patch: fields, and the current terms of the E updates
+    // the column's segment: fields, and the current terms of the E updates
     // (jr: dt/eps (J_r(j-1) + J_r(j)) / 2; jz: the same over columns i-1, i,
     // or on the axis minus the signed dt/eps J_z term)
-    double er[R], ez[R], h[R], jr[R], jz[R];
+    double er[S], ez[S], h[S], jr[S], jz[S];
     {
-      const T *gEr = reinterpret_cast<const T *>(stage);
-      const T *gEz = reinterpret_cast<const T *>(stage + S::field_bytes);
-      const T *gH = reinterpret_cast<const T *>(stage + 2 * S::field_bytes);
-      const long long *gJr = reinterpret_cast<const long long *>(stage + 3 * S::field_bytes);
-      const long long *gJz = reinterpret_cast<const long long *>(stage + 3 * S::field_bytes + S::cur_bytes);
+      const T *gEr = reinterpret_cast<const T *>(smem);
+      const T *gEz = reinterpret_cast<const T *>(smem + St::field_bytes);
+      const T *gH = reinterpret_cast<const T *>(smem + 2 * St::field_bytes);
+      const long long *gJr = reinterpret_cast<const long long *>(smem + 3 * St::field_bytes);
+      const long long *gJz = reinterpret_cast<const long long *>(smem + 3 * St::field_bytes + St::cur_bytes);
       const ExtraCurrent xj = I.xj;
-      double below = 0.0;
-      if (xj.Jr) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int sf = lane + of + r * BW, sj = lane + oj + r * 34, row = y0 + r;
-          er[r] = (double)gEr[sf];
-          ez[r] = (double)gEz[sf];
-          h[r] = (double)gH[sf];
-          double a = (double)gJr[sj], b = (double)gJz[sj];
-          if (colH && row >= 0 && row < nz) {
-            const int64_t g = col + (int64_t)row * I.ldj;
-            a = a + (double)(long long)xj.Jr[g] * xj.rel;
-            b = b + (double)(long long)xj.Jz[g] * xj.rel;
-          }
-          a = a * iv;
-          b = b * iv;
-          jr[r] = dt_eps * (below + a) / 2;
-          below = a;
-          jz[r] = b;
+      // row r of the segment (r = -1: the row below it)
+      auto current = [&](const long long *g, const unsigned long long *x, int r) {
+        double a = (double)g[lane + oj + (w * S + r) * 34];
+        if (x) {
+          const int row = y0 + r;
+          if (colH && row >= 0 && row < nz) a = a + (double)(long long)x[col + (int64_t)row * I.ldj] * xj.rel;
         }
-      } else {
+        return a * iv;
+      };
+      double below = w > 0 ? current(gJr, xj.Jr, -1) : 0.0;
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int sf = lane + of + r * BW, sj = lane + oj + r * 34;
-          er[r] = (double)gEr[sf];
-          ez[r] = (double)gEz[sf];
-          h[r] = (double)gH[sf];
-          const double a = (double)gJr[sj] * iv;
-          jr[r] = dt_eps * (below + a) / 2;
-          below = a;
-          jz[r] = (double)gJz[sj] * iv;
-        }
+      for (int r = 0; r < S; ++r) {
+        const int sf = lane + of + (w * S + r) * BW;
+        er[r] = (double)gEr[sf];
+        ez[r] = (double)gEz[sf];
+        h[r] = (double)gH[sf];
+        const double a = current(gJr, xj.Jr, r);
+        jr[r] = dt_eps * (below + a) / 2;
+        below = a;
+        jz[r] = current(gJz, xj.Jz, r);
       }
     }
-    __syncwarp();
-    // the area is free: the warp's next patch is fetched while this one is computed
-    if (lane == 0 && t + stride < ntiles) {
+    __syncthreads();
+    // the area is free: the block's next patch is fetched while this one is computed
+    if (threadIdx.x == 0 && t + stride < ntiles) {
       fence_proxy_async_smem();
-      tma_issue_item<T, R>(W, t + stride, stage, bar);
+      tma_issue_item<T, R>(W, t + stride, smem, bar);
     }
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
+    for (int r = 0; r < S; ++r) {
       const double left = __shfl_up_sync(FULL, jz[r], 1);
       const double jt = jsign ? dt_eps * jz[r] : -(dt_eps * jz[r]);
       jz[r] = col == 0 ? -jt : (colH ? dt_eps * (left + jz[r]) / 2 : 0.0);
     }
-    // patch rows of grid rows 0 and n_z (Er there: zero, or the end copies)
+    // segment rows of grid rows 0 and n_z (Er there: zero, or the end copies)
     const int r0 = -y0, rn = nz - y0;
-    const bool edge_rows = (r0 >= 0 && r0 < R) || (rn >= 0 && rn < R);
-    auto h_update = [&](double chr, double chz) {
+    const bool edge_rows = (r0 >= 0 && r0 < S) || (rn >= 0 && rn < S);
+    // the segments above and below (the patch's first and last read their own
+    // row instead: halo points, whose values do not matter)
+    const int up = w + 1 < NW ? w + 1 : w, dn = w > 0 ? w - 1 : 0;
+    auto publish_e = [&](int b) {
+      s_first[b][w][lane] = er[0];
+      s_last[b][w][lane] = er[S - 1];
+      __syncthreads();
+    };
+    auto h_update = [&](double chr, double chz, int b) {
+      const double above = s_first[b][up][lane];
 #pragma unroll
-      for (int r = 0; r + 1 < R; ++r) {
+      for (int r = 0; r < S; ++r) {
         const double ezr = __shfl_down_sync(FULL, ez[r], 1);
-        h[r] = h[r] + (chr * (ezr - ez[r]) - chz * (er[r + 1] - er[r]));
+        const double e1 = r + 1 < S ? er[r + 1 < S ? r + 1 : r] : above;
+        h[r] = h[r] + (chr * (ezr - ez[r]) - chz * (e1 - er[r]));
       }
     };
-    auto e_update = [&]() {
-      double ne[R];
+    auto e_update = [&](int b) {
+      s_h[w][lane] = h[S - 1];
+      __syncthreads();
+      const double hb = s_h[dn][lane];
+      double ne[S];
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int rm = r > 0 ? r - 1 : 0;
+      for (int r = 0; r < S; ++r) {
         const double hl = __shfl_up_sync(FULL, h[r], 1);
-        ne[r] = er[r] - jr[r] - dt_eps_dz * (h[r] - h[rm]);
+        ne[r] = er[r] - jr[r] - dt_eps_dz * (h[r] - (r > 0 ? h[r > 0 ? r - 1 : 0] : hb));
         ez[r] = ez[r] - jz[r] + ezp * h[r] + ezm * hl;
       }
       if (edge_rows) {
+        const double eu = s_first[b][up][lane], ed = s_last[b][dn][lane];
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int rm = r > 0 ? r - 1 : r, rp = r + 1 < R ? r + 1 : r;
-          if (r == r0) ne[r] = endcopy ? er[rp] : 0.0;
-          if (r == rn) ne[r] = endcopy ? er[rm] : 0.0;
+        for (int r = 0; r < S; ++r) {
+          if (r == r0) ne[r] = endcopy ? (r + 1 < S ? er[r + 1 < S ? r + 1 : r] : eu) : 0.0;
+          if (r == rn) ne[r] = endcopy ? (r > 0 ? er[r > 0 ? r - 1 : 0] : ed) : 0.0;
         }
       }
 #pragma unroll
-      for (int r = 0; r < R; ++r) er[r] = ne[r];
+      for (int r = 0; r < S; ++r) er[r] = ne[r];
     };
-    h_update(I.chr4, I.chz4);
-    e_update();
-    h_update(I.chr2, I.chz2);
-    e_update();
-    h_update(I.chr4, I.chz4);
+    publish_e(0);
+    h_update(I.chr4, I.chz4, 0);
+    e_update(0);
+    publish_e(1);
+    h_update(I.chr2, I.chz2, 1);
+    e_update(1);
+    publish_e(0);
+    h_update(I.chr4, I.chz4, 0);
     // write back the tile: columns [3, 29) and rows [3, R - 3) of the patch
     T *Er = reinterpret_cast<T *>(I.Er), *Ez = reinterpret_cast<T *>(I.Ez), *H = reinterpret_cast<T *>(I.H);
     unsigned long long *Jr_next = I.Jr_next, *Jz_next = I.Jz_next;
     const int ldf = I.ldf, ldj = I.ldj;
     const bool out_col = lane >= kTmaHalo && lane < kTmaHalo + kTmaTileW && col <= nr;
-    if (sizeof(T) == 4) {
-      // FP32 form: the fields rounded to float once; whole gather quads (when
-      // the cell has them) from those floats, corner columns from the lane
-      // below by shuffle
-      const FieldQuads q = I.q;
-      float fe[R], fz[R], fh[R];
 #pragma unroll
-      for (int r = kTmaHalo - 1; r <= R - kTmaHalo; ++r) {
+    for (int r = 0; r < S; ++r) {
+      const int row = y0 + r, pr = w * S + r;
+      if (pr < kTmaHalo || pr >= R - kTmaHalo || row > nz) continue;
+      if (!out_col) continue;
+      if (col < nr) Er[col + (int64_t)row * ldf] = (T)er[r];
+      if (row < nz) Ez[col + (int64_t)row * ldf] = (T)ez[r];
+      if (col < nr && row < nz) {
+        H[col + (int64_t)row * ldf] = (T)h[r];
+        const int64_t g = col + (int64_t)row * ldj;
+        Jr_next[g] = 0;
+        Jz_next[g] = 0;
+      }
+    }
+    if (sizeof(T) == 4 && I.q.er) {
+      // FP32 form: whole gather quads from the fields rounded to float, corner
+      // columns from the lane below by shuffle, corner rows from the segments
+      // above and below
+      const FieldQuads q = I.q;
+      s_h[w][lane] = h[S - 1];
+      s_ez[w][lane] = ez[S - 1];
+      __syncthreads();
+      const float e_up = (float)s_first[0][up][lane], z_dn = (float)s_ez[dn][lane], h_dn = (float)s_h[dn][lane];
+      float fe[S + 1], fz[S + 1], fh[S + 1];     // fe[r]: row r; fz[r], fh[r]: row r - 1
+      fe[S] = e_up; fz[0] = z_dn; fh[0] = h_dn;
+#pragma unroll
+      for (int r = 0; r < S; ++r) {
         fe[r] = (float)er[r];
-        fz[r] = (float)ez[r];
-        fh[r] = (float)h[r];
+        fz[r + 1] = (float)ez[r];
+        fh[r + 1] = (float)h[r];
       }
       const bool lo0 = col > 0, hi0 = col > nr - 1;   // corner column c0 = col - 1, c1 = col - 1
 #pragma unroll
-      for (int r = kTmaHalo; r < R - kTmaHalo; ++r) {
-        const int row = y0 + r;
+      for (int r = 0; r < S; ++r) {
+        const int row = y0 + r, pr = w * S + r;
+        if (pr < kTmaHalo || pr >= R - kTmaHalo || row > nz) continue;     // (the same for the whole warp)
         const float eu0 = __shfl_up_sync(FULL, fe[r], 1), eu1 = __shfl_up_sync(FULL, fe[r + 1], 1);
-        const float zd0 = __shfl_down_sync(FULL, fz[r - 1], 1), zd1 = __shfl_down_sync(FULL, fz[r], 1);
-        const float hu0 = __shfl_up_sync(FULL, fh[r - 1], 1), hu1 = __shfl_up_sync(FULL, fh[r], 1);
-        if (!out_col || row > nz) continue;
-        if (col < nr) reinterpret_cast<float *>(Er)[col + (int64_t)row * ldf] = fe[r];
-        if (row < nz) reinterpret_cast<float *>(Ez)[col + (int64_t)row * ldf] = fz[r];
-        if (col < nr && row < nz) {
-          reinterpret_cast<float *>(H)[col + (int64_t)row * ldf] = fh[r];
-          const int64_t g = col + (int64_t)row * ldj;
-          Jr_next[g] = 0;
-          Jz_next[g] = 0;
-        }
-        if (!q.er) continue;                                 // no gather quads in this cell
+        const float zd0 = __shfl_down_sync(FULL, fz[r], 1), zd1 = __shfl_down_sync(FULL, fz[r + 1], 1);
+        const float hu0 = __shfl_up_sync(FULL, fh[r], 1), hu1 = __shfl_up_sync(FULL, fh[r + 1], 1);
+        if (!out_col) continue;
         const bool ra_lo = row > 0, rb_lo = row > nz - 1;   // quad rows ra = row - 1, rb = row - 1
         if (row < nz)
           q.er[col + (int64_t)row * (nr + 1)] =
               make_float4(lo0 ? eu0 : fe[r], hi0 ? eu0 : fe[r], lo0 ? eu1 : fe[r + 1], hi0 ? eu1 : fe[r + 1]);
         if (col < nr)
           q.ez[col + (int64_t)row * nr] =
-              make_float4(ra_lo ? fz[r - 1] : fz[r], ra_lo ? zd0 : zd1, rb_lo ? fz[r - 1] : fz[r],
+              make_float4(ra_lo ? fz[r] : fz[r + 1], ra_lo ? zd0 : zd1, rb_lo ? fz[r] : fz[r + 1],
                           rb_lo ? zd0 : zd1);
-        const float ha0 = ra_lo ? hu0 : hu1, ha = ra_lo ? fh[r - 1] : fh[r];
-        const float hb0 = rb_lo ? hu0 : hu1, hb = rb_lo ? fh[r - 1] : fh[r];
+        const float ha0 = ra_lo ? hu0 : hu1, ha = ra_lo ? fh[r] : fh[r + 1];
+        const float hb0 = rb_lo ? hu0 : hu1, hb = rb_lo ? fh[r] : fh[r + 1];
         q.h[col + (int64_t)row * (nr + 1)] =
             make_float4(lo0 ? ha0 : ha, hi0 ? ha0 : ha, lo0 ? hb0 : hb, hi0 ? hb0 : hb);
-      }
-    } else if (out_col) {
-#pragma unroll
-      for (int r = kTmaHalo; r < R - kTmaHalo; ++r) {
-        const int row = y0 + r;
-        if (row > nz) continue;
-        if (col < nr) Er[col + (int64_t)row * ldf] = (T)er[r];
-        if (row < nz) Ez[col + (int64_t)row * ldf] = (T)ez[r];
-        if (col < nr && row < nz) {
-          H[col + (int64_t)row * ldf] = (T)h[r];
-          const int64_t g = col + (int64_t)row * ldj;
-          Jr_next[g] = 0;
-          Jz_next[g] = 0;
-        }
       }
     }
   }

@@ -1916,35 +1916,30 @@ __device__ __forceinline__ void commit_pass32(SimCounters *cnt) {
   cnt->step = ns;
 }
 
-// The field sub-cycle of one step for fdtd_ratio 1: one warp per patch of R
-// rows (fdtd_tma.cuh).
-template <typename T, int R>
-__global__ void __launch_bounds__(32 * kTmaWarps, 2) k_sim_fdtd_tma(const __grid_constant__ FdtdInst I,
-                                                                SimCounters *cnt) {
+// The field sub-cycle of one step for fdtd_ratio 1: one block per patch of
+// shape K (fdtd_tma.cuh).
+template <typename T, int K>
+__global__ void __launch_bounds__(32 * tma_warps(K), tma_blocks(K)) k_sim_fdtd_tma(
+    const __grid_constant__ FdtdInst I, SimCounters *cnt) {
   if (cnt && blockIdx.x == 0 && threadIdx.x == 0) commit_pass32(cnt);
-  fdtd_warp_body<T, R>(FdtdWork{&I, nullptr, I.ntiles});
+  fdtd_block_body<T, K>(FdtdWork{&I, nullptr, I.ntiles});
 }
 
-// The field update of every cell of a batch in one launch: the warps walk a
-// table of (cell, tile) work items; FP32 form (commit given): the blocks first
+// The field update of every cell of a batch in one launch: the blocks walk a
+// table of (cell, tile) work items; FP32 form (commit given): they first
 // commit the previous pass of every cell.
-template <typename T, int R>
-__global__ void __launch_bounds__(32 * kTmaWarps, 2) k_batch_fdtd_tma(const FdtdInst *insts,
-                                                                  const int2 *table, int nitems,
-                                                                  SimCounters *const *commit,
-                                                                  int ninst) {
+template <typename T, int K>
+__global__ void __launch_bounds__(32 * tma_warps(K), tma_blocks(K)) k_batch_fdtd_tma(
+    const FdtdInst *insts, const int2 *table, int nitems, SimCounters *const *commit, int ninst) {
   if (commit && threadIdx.x == 0)
     for (int i = blockIdx.x; i < ninst; i += gridDim.x) commit_pass32(commit[i]);
-  fdtd_warp_body<T, R>(FdtdWork{insts, table, nitems});
+  fdtd_block_body<T, K>(FdtdWork{insts, table, nitems});
 }
 
 using SimFdtdTmaFn = void (*)(const FdtdInst, SimCounters *);
 using BatchFdtdTmaFn = void (*)(const FdtdInst *, const int2 *, int, SimCounters *const *, int);
 
-// the patch heights (rows) the field update is built for
-__host__ __device__ constexpr bool tma_rows_ok(int rows) { return rows == 12 || rows == 16 || rows == 20; }
-
-// the instance of each kernel, and its dynamic shared memory, for `rows`
+// the instance of each kernel, and its dynamic shared memory, for knob value `rows`
 template <typename T>
 SimFdtdTmaFn sim_fdtd_tma_fn(int rows) {
   return rows == 12 ? k_sim_fdtd_tma<T, 12> : rows == 20 ? k_sim_fdtd_tma<T, 20> : k_sim_fdtd_tma<T, 16>;
@@ -1955,8 +1950,8 @@ BatchFdtdTmaFn batch_fdtd_tma_fn(int rows) {
 }
 template <typename T>
 size_t tma_block_bytes(int rows) {
-  return rows == 12 ? TmaStage<T, 12>::block_bytes
-                    : rows == 20 ? TmaStage<T, 20>::block_bytes : TmaStage<T, 16>::block_bytes;
+  return rows == 12 ? TmaStage<T, tma_rows(12)>::block_bytes
+                    : rows == 20 ? TmaStage<T, tma_rows(20)>::block_bytes : TmaStage<T, tma_rows(16)>::block_bytes;
 }
 
 // The general sub-cycle (fdtd_ratio > 1): one 32 x 32 patch per block
@@ -2515,7 +2510,7 @@ int launch_fdtd(gasatt_sim *s, cudaStream_t st, int q) {
   // the held ion current, in the electron current's fixed-point units
   const ExtraCurrent ion{s->Jir, s->Jiz, s->scale / s->ion_scale};
   if (R == 1) {
-    const dim3 block(32 * kTmaWarps);
+    const dim3 block(32 * tma_warps(s->tma_rows));
     if (s->form == 0)
       sim_fdtd_tma_fn<double>(s->tma_rows)<<<s->tma_grid, block, s->tma_smem, st>>>(s->fdtd_inst[q], nullptr);
     else
@@ -2801,56 +2796,70 @@ int encode_map(gasatt_sim *s, CUtensorMap *m, CUtensorMapDataType type, void *ba
   return GASATT_OK;
 }
 
-// The field update of fdtd_ratio 1: patch rows, tiles, grid, shared memory
-// and the tensor maps of the fields and of both current buffers.
+// The patch shape for cells of the given numbers of tiles in the three shapes
+// (fdtd_tile_rows 0): the smallest patches (short segments, so the shortest
+// chain) while they leave half of the GPU's block slots free, the middle ones
+// while their tiles are one wave of blocks, beyond that the tallest (the least
+// halo recomputed).  FP32 step with shape 12 / 16 / 20: 32 x 64 cells 18.4 / 19.2
+// / 21.2 us; 256 x 1024 54.3 / 54.4 / 56.7 (FP64 79.7 / 78.5 / 78.4); 1024 x
+// 4096 423 / 417 / 405; 16 batched cells 328 / 314 / 301.
+int tma_auto(long long tiles12, long long tiles16) { return tiles12 <= 4 * 148 ? 12 : tiles16 <= 4 * 148 ? 16 : 20; }
+
+// The field update's descriptor of a cell for the steps of parity q with patch
+// shape k: tensor maps of the fields and of the current read, where the
+// tiles are written.
 template <typename T>
-int setup_fdtd_tma(gasatt_sim *s, int nsm) {
+int fdtd_inst_of(gasatt_sim *s, int k, int q, FdtdInst &I) {
   const auto &c = s->cfg;
-  const int ph = c.fdtd_tile_rows > 0 ? c.fdtd_tile_rows : 12;
-  if (!tma_rows_ok(ph)) return fail(s->ctx, GASATT_E_ARG, "fdtd_tile_rows: 12, 16 or 20");
-  s->tma_rows = ph;
-  s->tma_smem = tma_block_bytes<T>(ph);
-  const int tiles_x = (c.n_r + 1 + kTmaTileW - 1) / kTmaTileW;
-  const int tiles_y = (c.n_z + 1 + (ph - 2 * kTmaHalo) - 1) / (ph - 2 * kTmaHalo);
-  const int ntiles = tiles_x * tiles_y;
-  const SimFdtdTmaFn kern = sim_fdtd_tma_fn<T>(ph);
-  GASATT_CUDA(s->ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)s->tma_smem));
-  int occ = 0;
-  GASATT_CUDA(s->ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * kTmaWarps,
-                                                                    s->tma_smem));
-  if (occ < 1) return fail(s->ctx, GASATT_E_ARG, "field update: patch does not fit in shared memory");
-  const long long slots = (long long)nsm * occ, blocks = (ntiles + kTmaWarps - 1) / kTmaWarps;
-  s->tma_grid = (unsigned)(slots < blocks ? slots : blocks);
+  const int rows = tma_rows(k);
   const CUtensorMapDataType ft = sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
   const size_t ldb = (size_t)s->ldf * sizeof(T), ldjb = (size_t)s->ldj * 8;
   const int bw = TmaBox<T>::w;
-  for (int q = 0; q < 2; ++q) {
-    FdtdInst &I = s->fdtd_inst[q];
-    std::memset(&I, 0, sizeof(I));
-    TmaMaps &M = I.maps;
-    SIM_TRY(encode_map(s, &M.er, ft, s->Er[q], c.n_r, c.n_z + 1, ldb, bw, ph));
-    SIM_TRY(encode_map(s, &M.ez, ft, s->Ez[q], c.n_r + 1, c.n_z, ldb, bw, ph));
-    SIM_TRY(encode_map(s, &M.h, ft, s->H[q], c.n_r, c.n_z, ldb, bw, ph));
-    SIM_TRY(encode_map(s, &M.jr, CU_TENSOR_MAP_DATA_TYPE_INT64, s->Jr[q], c.n_r, c.n_z, ldjb, 34, ph));
-    SIM_TRY(encode_map(s, &M.jz, CU_TENSOR_MAP_DATA_TYPE_INT64, s->Jz[q], c.n_r, c.n_z, ldjb, 34, ph));
-    I.Er = s->Er[1 - q]; I.Ez = s->Ez[1 - q]; I.H = s->H[1 - q];
-    I.Jr_next = s->Jr[1 - q]; I.Jz_next = s->Jz[1 - q];
-    I.colc = s->fdtd_colc;
-    I.xj = ExtraCurrent{s->Jir, s->Jiz, s->scale / s->ion_scale};
-    I.q = sizeof(T) == 4 ? s->quads : FieldQuads{};
-    I.c = fdtd_coef(s);
-    const double h4 = c.dt / 4, h2 = c.dt / 2;
-    I.chr4 = h4 / (c.mu0 * I.c.dr);
-    I.chz4 = h4 / (c.mu0 * I.c.dz);
-    I.chr2 = h2 / (c.mu0 * I.c.dr);
-    I.chz2 = h2 / (c.mu0 * I.c.dz);
-    I.nr = c.n_r; I.nz = c.n_z; I.ldf = s->ldf; I.ldj = s->ldj;
-    I.flags = c.flags;
-    I.tiles_x = tiles_x;
-    I.ntiles = ntiles;
-    I.err = &s->cnt->fdtd_err;
-  }
+  std::memset(&I, 0, sizeof(I));
+  TmaMaps &M = I.maps;
+  SIM_TRY(encode_map(s, &M.er, ft, s->Er[q], c.n_r, c.n_z + 1, ldb, bw, rows));
+  SIM_TRY(encode_map(s, &M.ez, ft, s->Ez[q], c.n_r + 1, c.n_z, ldb, bw, rows));
+  SIM_TRY(encode_map(s, &M.h, ft, s->H[q], c.n_r, c.n_z, ldb, bw, rows));
+  SIM_TRY(encode_map(s, &M.jr, CU_TENSOR_MAP_DATA_TYPE_INT64, s->Jr[q], c.n_r, c.n_z, ldjb, 34, rows));
+  SIM_TRY(encode_map(s, &M.jz, CU_TENSOR_MAP_DATA_TYPE_INT64, s->Jz[q], c.n_r, c.n_z, ldjb, 34, rows));
+  I.Er = s->Er[1 - q]; I.Ez = s->Ez[1 - q]; I.H = s->H[1 - q];
+  I.Jr_next = s->Jr[1 - q]; I.Jz_next = s->Jz[1 - q];
+  I.colc = s->fdtd_colc;
+  I.xj = ExtraCurrent{s->Jir, s->Jiz, s->scale / s->ion_scale};
+  I.q = sizeof(T) == 4 ? s->quads : FieldQuads{};
+  I.c = fdtd_coef(s);
+  const double h4 = c.dt / 4, h2 = c.dt / 2;
+  I.chr4 = h4 / (c.mu0 * I.c.dr);
+  I.chz4 = h4 / (c.mu0 * I.c.dz);
+  I.chr2 = h2 / (c.mu0 * I.c.dr);
+  I.chz2 = h2 / (c.mu0 * I.c.dz);
+  I.nr = c.n_r; I.nz = c.n_z; I.ldf = s->ldf; I.ldj = s->ldj;
+  I.flags = c.flags;
+  I.tiles_x = tma_tiles_x(c.n_r);
+  I.ntiles = tma_tiles(k, c.n_r, c.n_z);
+  I.err = &s->cnt->fdtd_err;
+  return GASATT_OK;
+}
+
+// The field update of fdtd_ratio 1: patch shape, descriptors, grid and shared memory.
+template <typename T>
+int setup_fdtd_tma(gasatt_sim *s, int nsm) {
+  const auto &c = s->cfg;
+  const int k = c.fdtd_tile_rows > 0 ? c.fdtd_tile_rows
+                                     : tma_auto(tma_tiles(12, c.n_r, c.n_z), tma_tiles(16, c.n_r, c.n_z));
+  if (!tma_rows_ok(k)) return fail(s->ctx, GASATT_E_ARG, "fdtd_tile_rows: 12, 16 or 20");
+  s->tma_rows = k;
+  s->tma_smem = tma_block_bytes<T>(k);
+  const int ntiles = tma_tiles(k, c.n_r, c.n_z);
+  const SimFdtdTmaFn kern = sim_fdtd_tma_fn<T>(k);
+  GASATT_CUDA(s->ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)s->tma_smem));
+  int occ = 0;
+  GASATT_CUDA(s->ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * tma_warps(k), s->tma_smem));
+  if (occ < 1) return fail(s->ctx, GASATT_E_ARG, "field update: patch does not fit in shared memory");
+  const long long slots = (long long)nsm * occ;
+  s->tma_grid = (unsigned)(slots < ntiles ? slots : ntiles);
+  for (int q = 0; q < 2; ++q) SIM_TRY(fdtd_inst_of<T>(s, k, q, s->fdtd_inst[q]));
   return GASATT_OK;
 }
 
@@ -3909,7 +3918,7 @@ int gasatt_sim_run_host(gasatt_sim *s, double *pos, double *vel, int64_t *n_io, 
 // ever out of step (stepped on its own in between), the batch steps each
 // cell with its own graph.
 struct BatchGroup {
-  int form = 0, ph = 0;
+  int form = 0, ph = 0;                  // ph: patch shape (0 until set up: chosen for the group)
   std::vector<gasatt_sim *> sims;
   void *cells = nullptr;                 // BatchCell32 / BatchCell64 per cell
   FdtdInst *insts[2] = {nullptr, nullptr};   // per step parity (the current buffer read)
@@ -4003,27 +4012,38 @@ int batch_group_setup(gasatt_batch *b, BatchGroup &G) {
     GASATT_CUDA(ctx, cudaMemcpy(d, h.data(), sizeof(BatchCell64) * n, cudaMemcpyHostToDevice));
     G.cells = d;
   }
+  // one patch shape for the group: its cells' own knob value, or by all their tiles
+  if (!G.ph) {
+    long long t12 = 0, t16 = 0;
+    for (const gasatt_sim *s : G.sims) {
+      t12 += tma_tiles(12, s->cfg.n_r, s->cfg.n_z);
+      t16 += tma_tiles(16, s->cfg.n_r, s->cfg.n_z);
+    }
+    G.ph = tma_auto(t12, t16);
+  }
   std::vector<int2> table;
   for (int i = 0; i < n; ++i)
-    for (int t = 0; t < G.sims[i]->fdtd_inst[0].ntiles; ++t) table.push_back(make_int2(i, t));
+    for (int t = 0; t < tma_tiles(G.ph, G.sims[i]->cfg.n_r, G.sims[i]->cfg.n_z); ++t) table.push_back(make_int2(i, t));
   G.nitems = (int)table.size();
   SIM_TRY(batch_alloc(b, &G.table, table.size()));
   GASATT_CUDA(ctx, cudaMemcpy(G.table, table.data(), sizeof(int2) * table.size(), cudaMemcpyHostToDevice));
   for (int q = 0; q < 2; ++q) {
     std::vector<FdtdInst> hi(n);
-    for (int i = 0; i < n; ++i) hi[i] = G.sims[i]->fdtd_inst[q];
+    for (int i = 0; i < n; ++i)
+      SIM_TRY(G.form == 1 ? fdtd_inst_of<float>(G.sims[i], G.ph, q, hi[i])
+                          : fdtd_inst_of<double>(G.sims[i], G.ph, q, hi[i]));
     SIM_TRY(batch_alloc(b, &G.insts[q], (size_t)n));
     GASATT_CUDA(ctx, cudaMemcpy(G.insts[q], hi.data(), sizeof(FdtdInst) * n, cudaMemcpyHostToDevice));
   }
   SIM_TRY(batch_alloc(b, &G.chunk_next, 1));
   int nsm = 148, occ = 1;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
-  G.fdtd_smem = G.sims[0]->tma_smem;
+  G.fdtd_smem = G.form == 1 ? tma_block_bytes<float>(G.ph) : tma_block_bytes<double>(G.ph);
   const BatchFdtdTmaFn fk = G.form == 1 ? batch_fdtd_tma_fn<float>(G.ph) : batch_fdtd_tma_fn<double>(G.ph);
   GASATT_CUDA(ctx, cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G.fdtd_smem));
-  GASATT_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fk, 32 * kTmaWarps, G.fdtd_smem));
+  GASATT_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fk, 32 * tma_warps(G.ph), G.fdtd_smem));
   const long long fslots = (long long)nsm * (occ > 0 ? occ : 1);
-  const long long fblocks = (G.nitems + kTmaWarps - 1) / kTmaWarps;
+  const long long fblocks = G.nitems;
   G.fdtd_grid = (unsigned)(fslots < fblocks ? fslots : (fblocks > 0 ? fblocks : 1));
   occ = 1;
   for (const gasatt_sim *s : G.sims) G.wide = G.wide || win_cols(s->cfg.n_r) < s->cfg.n_r;
@@ -4045,7 +4065,7 @@ int batch_group_launch(gasatt_batch *b, BatchGroup &G, cudaStream_t cs, cudaStre
                        int q) {
   gasatt_ctx *ctx = b->ctx;
   const int n = (int)G.sims.size();
-  const dim3 fb(32 * kTmaWarps);
+  const dim3 fb(32 * tma_warps(G.ph));
   if (G.form == 1) {
     batch_fdtd_tma_fn<float>(G.ph)<<<G.fdtd_grid, fb, G.fdtd_smem, cs>>>(G.insts[q], G.table, G.nitems,
                                                                         G.commit, n);
@@ -4198,12 +4218,12 @@ int gasatt_batch_create(gasatt_ctx *ctx, gasatt_sim *const *sims, int n, int sor
     if (s->cfg.fdtd_ratio != 1) { b->singles.push_back(s); continue; }
     BatchGroup *G = nullptr;
     for (BatchGroup &g : b->groups)
-      if (g.form == s->form && g.ph == s->tma_rows && (int)g.sims.size() < kMaxBatch) G = &g;
+      if (g.form == s->form && g.ph == s->cfg.fdtd_tile_rows && (int)g.sims.size() < kMaxBatch) G = &g;
     if (!G) {
       b->groups.emplace_back();
       G = &b->groups.back();
       G->form = s->form;
-      G->ph = s->tma_rows;
+      G->ph = s->cfg.fdtd_tile_rows;
     }
     G->sims.push_back(s);
   }

@@ -7,11 +7,11 @@ update's arithmetic is the same for every patch):
   sort_period     steps between cell re-sorts: a sort costs a pass over the
                   state, while the particles' drift away from their sorted
                   order slowly makes the gather and the deposit less local;
-  fdtd_tile_rows  rows R of the field update's per-warp patch (12, 16 or 20;
-                  a warp computes 26 columns x R - 6 rows of output from 32 x R
-                  staged points): the halo recomputed per output point against
-                  the registers a warp holds and the number of patches for
-                  the warps to share;
+  fdtd_tile_rows  the field update's patch (12, 16 or 20: 16, 32 or 64 rows of
+                  32 columns on 4, 8 or 8 warps; a block computes 26 columns x
+                  rows - 6 of output): the halo recomputed per output point
+                  against the length of a warp's chain and the number of
+                  patches for the blocks to share;
   pass_chunk      particles per chunk of the FP32 particle pass (its deposit
                   window's span against the number of chunks for the blocks
                   to balance);

@@ -273,8 +273,10 @@ typedef struct gasatt_sim_config {
   int      ion_subcycle;    /* electron steps per ion push (50); the ion step is ion_subcycle*dt */
   /* launch-shape knobs (results do not depend on them; 0 = the default, and
    * the autotuner of the Python package picks them per workload): */
-  int      fdtd_tile_rows;  /* rows of the field update's per-warp patch: 12, 16 or 20
-                               (output 26 columns x rows - 6 per patch); default 12 */
+  int      fdtd_tile_rows;  /* the field update's patch: 12, 16 or 20 for a block of 4, 8 or
+                               8 warps on 16, 32 or 64 rows of 32 columns (output 26
+                               columns x rows - 6); default: by the number of tiles of
+                               the grid (of all grids in a batch) */
   int      pass_chunk;      /* FP32 particle pass: particles per chunk a block takes,
                                a multiple of 256 (256..1792); default: chosen every
                                step so that the population fills all blocks evenly,
