@@ -50,11 +50,11 @@ constexpr int kMccBlock = 64;             // collision kernels: two warps per bl
 // lines of their own, so those atomics do not hold up the reads.
 struct SimCounters {
   unsigned long long n_total;    // committed slots
-  long long step;                // FP64: index of the next particle pass; FP32: of the current one
+  long long step;                // FP32: index of the current (last) particle pass
   unsigned long long cap;        // slot capacity
   unsigned long long sorted_total;
-  long long cand_step[2];        // FP64: the pass that queued each queue
-  int uncommitted;               // FP64: a pass ran since the last commit (k_commit)
+  long long step64[2];           // FP64: index of the last pass of parity 0 / 1 (it queued that queue)
+  int pad0_;
   int chunk;                     // FP32: particles per chunk of the next pass
   int chunk_fixed, pass_blocks;  // FP32: the configured chunk (0: by population), blocks of a pass
   unsigned long long pad1_[8];
@@ -77,7 +77,7 @@ struct SimCounters {
   unsigned long long ion_alive, ion_charge, ion_kin_fx;   // diagnostics; kinetic: E * 2^32 [eV]
 };
 
-// slots holding particles, including births of the last pass not yet committed
+// slots holding particles, including births since the last commit or sort
 __device__ __forceinline__ long long slots_in_use(const SimCounters *cnt) {
   const unsigned long long nt = cnt->n_total + cnt->n_births;
   return (long long)(nt < cnt->cap ? nt : cnt->cap);
@@ -396,24 +396,15 @@ __device__ __forceinline__ void queue_push(bool want, long long p, unsigned long
   if (want) queue[base + __popc(m & ((1u << lane) - 1))] = (int)p;
 }
 
-// Commit of a particle pass (parity q), run as its own one-thread kernel after
-// the pass: the births of the collision kernel that ran before the pass join
-// the committed slots, the queue of the pass is labelled with its step, the
-// other queue (consumed by that collision kernel) is emptied, and the step
-// advances.  Idempotent: only the first commit after a pass does anything.
-// (Done at the end of the pass itself, by its last block, the atomics of 592
-// blocks on the counters' cache line slowed the pass by a tenth.)
-__device__ __forceinline__ void k_commit_body(SimCounters *cnt, int q) {
-  if (!cnt->uncommitted) return;
-  const unsigned long long nt = cnt->n_total + cnt->n_births;
-  cnt->n_total = nt < cnt->cap ? nt : cnt->cap;
-  cnt->n_births = 0;
-  cnt->cand_step[q] = cnt->step;
-  cnt->n_cand[1 - q] = 0;
-  cnt->step += 1;
-  cnt->uncommitted = 0;
-}
-__global__ void k_commit(SimCounters *cnt, int q) { k_commit_body(cnt, q); }
+// FP64 bookkeeping.  The pass of parity q runs one step after the pass of the
+// other parity (step64), and births go on counting from the slots of the last
+// sort, so nothing has to be committed between a pass and the collisions it
+// queued - a one-thread kernel in between lengthened the collision branch, the
+// critical path of a small cell's step, by 3 us.  Only the queue that the next
+// pass fills has to be empty: the pass itself does that for a cell on its own
+// (the other queue was consumed before it), and one kernel for all cells of a batch.
+__device__ __forceinline__ void clear_next_queue(SimCounters *cnt, int q) { cnt->n_cand[1 - q] = 0; }
+__global__ void k_clear_next_queue(SimCounters *cnt, int q) { clear_next_queue(cnt, q); }
 
 // ------------------------------------------------------ deposit
 // The ions' deposit.  Each one's four node contributions (q FN v w, both
@@ -757,8 +748,11 @@ __global__ void __launch_bounds__(kBlock, 3) k_pass64(SimParams P, State64 S, Fi
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int box_row0[2], box_rows[2], box_col0[2], box_cmax[2];   // of this chunk and the next
   const long long n0 = slots_in_use(cnt);
-  const long long step = cnt->step;
-  if (blockIdx.x == 0 && threadIdx.x == 0) cnt->uncommitted = 1;
+  const long long step = cnt->step64[1 - q] + 1;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    cnt->step64[q] = step;
+    clear_next_queue(cnt, q);
+  }
   const int chunk = even_chunk((unsigned)n0, gridDim.x, kChunk64);
   const int cols = win_cols(P.nr), ws = win_stride(cols), maxrows = min(kWin64Nodes / ws, P.nz);
   // the window starts zeroed; each chunk's flush leaves it zeroed again
@@ -792,7 +786,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_pass64(SimParams P, State64 S, Fi
 
 // The collision of candidate slot p queued at step `step` (FP64 form): MCC,
 // the ion and the secondary's birth at the parent's position.  n0: the
-// committed slots (births land beyond).
+// slots of the last sort (births land beyond).
 __device__ __forceinline__ void mcc64_one(const SimParams &P, const State64 &S, SimCounters *cnt,
                                           long long p, long long step, long long n0) {
   const double2 rz = S.rz[p], urt = S.urt[p];
@@ -831,7 +825,7 @@ __global__ void __launch_bounds__(kMccBlock) k_mcc64(SimParams P, State64 S, Sim
   // length, and lanes on different branches would run them one after another
   if ((threadIdx.x & 31) != 0) return;
   const long long n0 = (long long)cnt->n_total;
-  const long long step = cnt->cand_step[q];
+  const long long step = cnt->step64[q];
   const long long nq = (long long)cnt->n_cand[q];
   const int *qu = queue + (long long)q * P.cap;
   const long long nwarps = (long long)gridDim.x * (kMccBlock / 32);
@@ -860,9 +854,10 @@ struct BatchCell64 {
   int *queue;
   Fields<double> F[2];        // field buffers 0 / 1 (the pass into current buffer jb reads F[jb])
 };
+// empties every cell's queue that the pass after the one of parity q fills
 __global__ void k_batch_commit64(const BatchCell64 *__restrict__ cells, int ncell, int q) {
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x)
-    k_commit_body(cells[c].cnt, q);
+    clear_next_queue(cells[c].cnt, q);
 }
 
 // the collisions queued (parity q) by every cell's last pass, one per warp
@@ -884,7 +879,7 @@ __global__ void __launch_bounds__(kMccBlock) k_batch_mcc64(const BatchCell64 *__
     const BatchCell64 &C = cells[c];
     SimCounters *cc = C.cnt;
     const int *qu = C.queue + (long long)q * C.P[0].cap;
-    mcc64_one(C.P[0], C.S[cur], cc, qu[k - pre[c]], cc->cand_step[q], (long long)cc->n_total);
+    mcc64_one(C.P[0], C.S[cur], cc, qu[k - pre[c]], cc->step64[q], (long long)cc->n_total);
   }
 }
 
@@ -913,7 +908,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_batch_pass64(const BatchCell64 *_
     pre[0] = 0;
     for (int c = 0; c < ncell; ++c) pre[c + 1] = pre[c] + (pre[c + 1] + chunk - 1) / chunk;
     if (blockIdx.x == 0)
-      for (int c = 0; c < ncell; ++c) cells[c].cnt->uncommitted = 1;
+      for (int c = 0; c < ncell; ++c) cells[c].cnt->step64[q] = cells[c].cnt->step64[1 - q] + 1;
   }
   __syncthreads();
   const long long nitem = pre[ncell];
@@ -967,7 +962,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_batch_pass64(const BatchCell64 *_
     }
     const int cols = win_cols(sP.nr);
     const Win64 w{reinterpret_cast<unsigned *>(smem), box_row0, box_rows, box_col0, cols, win_stride(cols)};
-    chunk64<0>(sP, C->S[cur], C->F[jb], C->cnt, C->queue, q, C->cnt->step, (int)beg, (int)end, w, &box_cmax);
+    chunk64<0>(sP, C->S[cur], C->F[jb], C->cnt, C->queue, q, C->cnt->step64[1 - q] + 1, (int)beg, (int)end, w, &box_cmax);
     if (threadIdx.x == 0) resolve();
     __syncthreads();
     flush64(sP, w, box_cmax + 1);
@@ -2458,6 +2453,7 @@ struct gasatt_sim {
   IonState ion_tmp{};             // scratch store the ions are sorted into before a push
   FieldQuads quads{};             // FP32 form: gather quads, written with the fields
   bool mcc_pending = false;       // the last pass's collisions are not applied yet
+  bool batch_pass = false;        // FP64: the last pass was a batch's (clear_after_batch)
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;   // graph capture fork/join
   bool timing = false;
   // field update start/end, particle pass start/end, collision kernel start/end
@@ -2566,12 +2562,14 @@ int launch_pass(gasatt_sim *s, cudaStream_t st, int mode, int jb, int q, int fb)
   return GASATT_OK;
 }
 
-// the commit of the last pass (its parity q)
-int launch_commit(gasatt_sim *s, cudaStream_t st, int q) {
-  k_commit<<<1, 1, 0, st>>>(s->cnt, q);
+// FP64: before a pass of a cell on its own that follows a batch's (of parity q)
+int clear_after_batch(gasatt_sim *s, cudaStream_t st, int q) {
+  if (s->form != 0 || !s->batch_pass) return GASATT_OK;
+  s->batch_pass = false;
+  k_clear_next_queue<<<1, 1, 0, st>>>(s->cnt, q);
   s->ctx->launches++;
   cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(s->ctx, e, "commit launch");
+  if (e != cudaSuccess) return cuda_fail(s->ctx, e, "queue clear launch");
   return GASATT_OK;
 }
 
@@ -2597,7 +2595,6 @@ int flush_collisions(gasatt_sim *s) {
   if (!s->mcc_pending) return GASATT_OK;
   const int q = (int)((s->host_step - 1) & 1);
   cudaStream_t st = s->ctx->stream;
-  if (s->form == 0) SIM_TRY(launch_commit(s, st, q));
   SIM_TRY(launch_mcc(s, st, q));
   // The FP32 kernels pick their queue by the parity of the device's step
   // counter, which gasatt_sim_run_host moves against host_step's, so both
@@ -2732,6 +2729,7 @@ int sim_reset(gasatt_sim *s, int64_t n) {
   SimCounters zc{};
   zc.n_total = (unsigned long long)n;
   zc.step = -1;
+  zc.step64[0] = zc.step64[1] = -2;          // the prologue (parity 1) runs as step -1
   zc.cap = (unsigned long long)s->cfg.capacity;
   set_chunk(s, zc);
   GASATT_CUDA(ctx, cudaMemcpyAsync(s->cnt, &zc, sizeof(zc), cudaMemcpyHostToDevice, st));
@@ -2747,6 +2745,7 @@ int sim_reset(gasatt_sim *s, int64_t n) {
   GASATT_CUDA(ctx, cudaStreamSynchronize(st));
   s->primed = false;
   s->mcc_pending = false;
+  s->batch_pass = false;
   s->since_sort = 0;
   return GASATT_OK;
 }
@@ -2880,7 +2879,11 @@ int sim_prime(gasatt_sim *s) {
   cudaStream_t st = s->ctx->stream;
   if (s->cfg.sort_period > 0) SIM_TRY(gasatt_sim_sort(s));
   SIM_TRY(launch_pass(s, st, 1, 0, 1, fcur(s)));   // (a half drift reads no field)
-  if (s->form == 0) SIM_TRY(launch_commit(s, st, 1));
+  // (a run that goes on after gasatt_sim_run_host may start on odd parity: its
+  // first step then has the parity of the prologue and reads the other index)
+  if (s->form == 0 && (s->host_step & 1))
+    GASATT_CUDA(s->ctx, cudaMemcpyAsync(&s->cnt->step64[0], &s->cnt->step64[1], sizeof(long long),
+                                        cudaMemcpyDeviceToDevice, st));
   s->primed = true;
   return GASATT_OK;
 }
@@ -2937,8 +2940,7 @@ int build_graphs(gasatt_sim *s) {
       cudaError_t e = cudaEventRecord(s->fork_ev, cs);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(side, s->fork_ev, 0);
       if (e == cudaSuccess && s->timing) e = cudaEventRecordWithFlags(s->ev[4], side, cudaEventRecordExternal);
-      if (e == cudaSuccess) rc = launch_commit(s, side, 1 - q);
-      if (e == cudaSuccess && !rc) rc = launch_mcc(s, side, 1 - q);
+      if (e == cudaSuccess) rc = launch_mcc(s, side, 1 - q);
       if (e == cudaSuccess && !rc && s->timing) e = cudaEventRecordWithFlags(s->ev[5], side, cudaEventRecordExternal);
       if (e == cudaSuccess && !rc) e = cudaEventRecord(s->join_ev, side);
       if (e == cudaSuccess && !rc && s->timing) e = cudaEventRecordWithFlags(s->ev[0], cs, cudaEventRecordExternal);
@@ -3196,6 +3198,7 @@ int gasatt_sim_create(gasatt_ctx *ctx, const gasatt_sim_config *cfg, const gasat
   // zero state
   SimCounters z{};
   z.step = -1;
+  z.step64[0] = z.step64[1] = -2;
   z.cap = (unsigned long long)cap;
   set_chunk(s, z);
   if (cudaMemcpy(s->cnt, &z, sizeof(z), cudaMemcpyHostToDevice) != cudaSuccess)
@@ -3673,8 +3676,9 @@ int gasatt_sim_step(gasatt_sim *s, int nsteps) {
   GASATT_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;
   SIM_TRY(sim_prime(s));
-  // field update, (FP64: commit, collision kernel,) particle pass
-  const int per_step = s->form == 0 ? 4 : 2;
+  // field update, (FP64: collision kernel,) particle pass
+  const int per_step = s->form == 0 ? 3 : 2;
+  if (nsteps > 0) SIM_TRY(clear_after_batch(s, st, (int)((s->host_step - 1) & 1)));
   for (int k = 0; k < nsteps; ++k) {
     if (s->cfg.sort_period > 0 && s->since_sort >= s->cfg.sort_period) SIM_TRY(gasatt_sim_sort(s));
     GASATT_CUDA(ctx, cudaGraphLaunch(s->g_step[s->cur][s->host_step & 1], st));
@@ -3856,10 +3860,10 @@ int gasatt_sim_run_host(gasatt_sim *s, double *pos, double *vel, int64_t *n_io, 
   h.n_total = (unsigned long long)n;
   h.n_births = 0;
   h.n_cand[0] = h.n_cand[1] = 0;
-  h.uncommitted = 0;
   h.chunk_next = 0;
   set_chunk(s, h);
   h.step += 1;                               // never reuse the last pass's step
+  h.step64[0] = (h.step64[0] > h.step64[1] ? h.step64[0] : h.step64[1]) + 1;   // the prologue (parity 1) runs one later
   GASATT_CUDA(ctx, cudaMemcpyAsync(s->cnt, &h, sizeof(h), cudaMemcpyHostToDevice, st));
   for (int q = 0; q < 2; ++q) {
     GASATT_CUDA(ctx, cudaMemsetAsync(s->Jr[q], 0, jbytes(s), st));
@@ -3867,6 +3871,7 @@ int gasatt_sim_run_host(gasatt_sim *s, double *pos, double *vel, int64_t *n_io, 
   }
   s->primed = false;
   s->mcc_pending = false;
+  s->batch_pass = false;
   SIM_TRY(restart_steps(s, st));             // the prologue deposits into buffer 0
   s->since_sort = s->cfg.sort_period;       // sort the fresh population first
   SIM_TRY(gasatt_sim_step(s, nsteps - 1));
@@ -3876,7 +3881,6 @@ int gasatt_sim_run_host(gasatt_sim *s, double *pos, double *vel, int64_t *n_io, 
   SIM_TRY(launch_fdtd(s, st, (int)(s->host_step & 1)));
   SIM_TRY(launch_pass(s, st, 2, (int)((s->host_step + 1) & 1), (int)(s->host_step & 1),
                       (int)((s->host_step + 1) & 1)));
-  if (s->form == 0) SIM_TRY(launch_commit(s, st, (int)(s->host_step & 1)));
   SIM_TRY(gasatt_sim_sort(s));               // compacts away the dead
   s->host_step++;
   s->primed = false;
@@ -3908,7 +3912,7 @@ int gasatt_sim_run_host(gasatt_sim *s, double *pos, double *vel, int64_t *n_io, 
 // Many independent gas cells stepped together.  Cells of the same precision
 // form and field patch (fdtd_ratio 1) form a group that runs each step as a
 // few launches for the whole group - the field update over every cell's
-// tiles (k_batch_fdtd_tma), (FP64: the commits and the collisions beside it,)
+// tiles (k_batch_fdtd_tma), (FP64: the emptying of the next queues and the collisions beside it,)
 // then the particle pass over every cell's candidates and chunks
 // (k_batch_pass32 / k_batch_pass64) - instead of one set of launches per
 // cell, so the blocks of each launch share all cells' work and small cells
@@ -4155,10 +4159,10 @@ int batch_build_graphs(gasatt_batch *b) {
 
 // flush_collisions for every cell of the batch (before its sort): a group
 // whose cells are at the same step parity and state buffer does it in two
-// launches (FP32: k_batch_collide32) or three (FP64: the commits, then
+// launches (FP32: k_batch_collide32) or three (FP64: k_batch_commit64, then
 // k_batch_mcc64) for all of its cells, then empties their queues; any other
 // cell flushes on its own.  A cell with nothing pending finds an empty queue
-// (its own flush emptied it) and a commit already made.
+// (its own flush emptied it).
 int batch_flush_collisions(gasatt_batch *b) {
   gasatt_ctx *ctx = b->ctx;
   cudaStream_t st = ctx->stream;
@@ -4275,11 +4279,14 @@ int gasatt_batch_step(gasatt_batch *b, int nsteps) {
     if (lockstep) {
       GASATT_CUDA(ctx, cudaGraphLaunch(b->g[s0->cur][s0->host_step & 1], st));
       for (const BatchGroup &G : b->groups) ctx->launches += G.form == 0 ? 4 : 2;
-      for (const gasatt_sim *s : b->singles) ctx->launches += s->form == 0 ? 4 : 2;
+      for (const gasatt_sim *s : b->singles) ctx->launches += s->form == 0 ? 3 : 2;
+      for (const BatchGroup &G : b->groups)
+        for (gasatt_sim *s : G.sims) s->batch_pass = true;
     } else {
       for (gasatt_sim *s : b->sims) {
+        SIM_TRY(clear_after_batch(s, st, (int)((s->host_step - 1) & 1)));
         GASATT_CUDA(ctx, cudaGraphLaunch(s->g_step[s->cur][s->host_step & 1], st));
-        ctx->launches += s->form == 0 ? 4 : 2;
+        ctx->launches += s->form == 0 ? 3 : 2;
       }
     }
     for (gasatt_sim *s : b->sims) {

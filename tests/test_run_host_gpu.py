@@ -49,3 +49,49 @@ def test_collisions_applied_once(calls):
     assert w[1] > 100
     for k in range(3):
         assert abs(x[k] - w[k]) <= 3 + 0.003 * w[k], (k, x[:3], w[:3])
+
+
+def test_fp64_queues_survive_alternating_steps():
+    """FP64 cells stepped by a batch, on their own (odd counts, with reads in
+    between that apply pending collisions) and by the batch again end where
+    they end alone: every queue is emptied before it is filled again."""
+    from gasatt.dropin import Context
+    from gasatt.sim import Batch
+    ctx = Context(0)
+
+    def make(seed):
+        cfg = config(NR, NZ, D, 1e-14, 200.0, precision=_lib.FP64, capacity=20000, seed=seed, sort_period=4)
+        sim = Sim(cfg, ctx=ctx)
+        sim.load(*births(1500, 8.0, NZ * D, seed=seed, sigma_r=30e-6, Rp=0.98 * NR * D))
+        return sim
+
+    def state(sim):
+        st, d = sim.read(), sim.diag()
+        a = st["r"] >= 0
+        o = np.argsort(st["id"][a])
+        return [st[k][a][o] for k in ("id", "r", "z", "ur", "ut", "uz")] + list(sim.fields()) + [
+            np.array([d[k] for k in ("n_alive", "n_ionizations", "n_elastic", "n_excitation", "n_null")])]
+
+    alone = []
+    for seed in (3, 4):
+        sim = make(seed)
+        sim.step(16)
+        alone.append(state(sim))
+        sim.close()
+    sims = [make(3), make(4)]
+    batch = Batch(sims, sort_period=4)
+    for kind, n in (("batch", 3), ("own", 1), ("batch", 2), ("read", 0), ("own", 3), ("read", 0), ("batch", 1), ("own", 2),
+                    ("batch", 4)):
+        if kind == "batch":
+            batch.step(n)
+        for sim in sims:
+            if kind == "own":
+                sim.step(n)
+            elif kind == "read":
+                sim.read()
+    for sim, want in zip(sims, alone):
+        for g, w in zip(state(sim), want):
+            np.testing.assert_array_equal(g, w)
+    batch.close()
+    for sim in sims:
+        sim.close()
