@@ -2878,12 +2878,17 @@ int sim_prime(gasatt_sim *s) {
   if (s->primed) return GASATT_OK;
   cudaStream_t st = s->ctx->stream;
   if (s->cfg.sort_period > 0) SIM_TRY(gasatt_sim_sort(s));
+  // The prologue runs as parity 1, one step after the last pass (after a new
+  // population both indices are equal).  A run that goes on after
+  // gasatt_sim_run_host may have had its last pass on parity 1, or go on with
+  // parity 1: the other parity's index then takes over the last one's, before or after.
+  auto catch_up = [&]() {
+    return cudaMemcpyAsync(&s->cnt->step64[0], &s->cnt->step64[1], sizeof(long long), cudaMemcpyDeviceToDevice, st);
+  };
+  const bool odd = s->host_step & 1;
+  if (s->form == 0 && !odd) GASATT_CUDA(s->ctx, catch_up());
   SIM_TRY(launch_pass(s, st, 1, 0, 1, fcur(s)));   // (a half drift reads no field)
-  // (a run that goes on after gasatt_sim_run_host may start on odd parity: its
-  // first step then has the parity of the prologue and reads the other index)
-  if (s->form == 0 && (s->host_step & 1))
-    GASATT_CUDA(s->ctx, cudaMemcpyAsync(&s->cnt->step64[0], &s->cnt->step64[1], sizeof(long long),
-                                        cudaMemcpyDeviceToDevice, st));
+  if (s->form == 0 && odd) GASATT_CUDA(s->ctx, catch_up());
   s->primed = true;
   return GASATT_OK;
 }
@@ -3863,7 +3868,7 @@ int gasatt_sim_run_host(gasatt_sim *s, double *pos, double *vel, int64_t *n_io, 
   h.chunk_next = 0;
   set_chunk(s, h);
   h.step += 1;                               // never reuse the last pass's step
-  h.step64[0] = (h.step64[0] > h.step64[1] ? h.step64[0] : h.step64[1]) + 1;   // the prologue (parity 1) runs one later
+  h.step64[0] = h.step64[1] = (h.step64[0] > h.step64[1] ? h.step64[0] : h.step64[1]) + 1;   // the prologue runs one later
   GASATT_CUDA(ctx, cudaMemcpyAsync(s->cnt, &h, sizeof(h), cudaMemcpyHostToDevice, st));
   for (int q = 0; q < 2; ++q) {
     GASATT_CUDA(ctx, cudaMemsetAsync(s->Jr[q], 0, jbytes(s), st));

@@ -95,3 +95,4 @@ def test_fp64_queues_survive_alternating_steps():
     batch.close()
     for sim in sims:
         sim.close()
+
