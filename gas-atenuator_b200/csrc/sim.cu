@@ -110,6 +110,7 @@ struct SimParams {
   long long cap;
   double qm_dt2;            // -q_e/m_e dt/2
   double idr, idz, ic2;     // 1/dr, 1/dz, 1/c^2
+  double mc2_ev, imc2_ev, idlnE;   // m_e c^2 [eV] and its inverse; 1 / dlnE
   double mu_qm;             // mu0 q_e/m_e dt/2 with the sign of qm_dt2 (FP64 form)
   double dep_q;             // FP64 form: fixed-point factor of the electrons' current (x v)
   float aE, aB, hdr, hdz;   // FP32 form: impulse per (V/m), per (A/m); c dt/(2 dr), c dt/(2 dz)
@@ -145,7 +146,7 @@ struct Birth { bool born; double ux, uy, uz; double eloss; };   // eloss: excita
 
 __device__ __forceinline__ void xs_lookup(const SimParams &P, double Eev, double &se, double &si,
                                           double &sx, double &L) {
-  L = (log(Eev) - P.lnEmin) / P.dlnE;
+  L = (log(Eev) - P.lnEmin) * P.idlnE;
   int i;
   double f;
   if (!(L > 0)) { i = 0; f = 0; }
@@ -183,9 +184,10 @@ __device__ __forceinline__ double cdf_theta(const SimParams &P, double L, double
   return (lo + (U - c0) / (c1 - c0)) * (GASATT_PI / 180);
 }
 
-__device__ __forceinline__ double u_of_energy(double EJ, double m, double c) {
-  const double e = EJ / (m * c * c);
-  return c * sqrt(e * (2 + e));
+// gamma v of an electron of kinetic energy E [eV]
+__device__ __forceinline__ double u_of_energy(const SimParams &P, double E) {
+  const double e = E * P.imc2_ev;
+  return P.c * sqrt(e * (2 + e));
 }
 
 // Null-collision candidate test U1 < P_null on the integer draw: with
@@ -271,12 +273,11 @@ __device__ __forceinline__ int mcc_event(const SimParams &P, uint64_t id, long l
   b.born = false;
   b.eloss = 0;
   const U2 d0 = draw2(P.seed, id, step, 0);
-  const double c = P.c, me = P.me, qe = P.qe, I = GASATT_ION_I_EV;
+  const double I = GASATT_ION_I_EV;
   const double u2 = ux * ux + uy * uy + uz * uz;
-  const double g = sqrt(1 + u2 / (c * c));
-  const double EJ = me * c * c * ((u2 / (c * c)) / (g + 1));
-  const double Eev = EJ / qe;
-  const double um = sqrt(u2), v = um / g;
+  const double w2 = u2 * P.ic2, ig = rsqrt(1 + w2);
+  const double Eev = P.mc2_ev * (w2 / ((1 + w2) * ig + 1));
+  const double ium = u2 > 0 ? rsqrt(u2) : 0.0, um = u2 * ium, v = um * ig;
   double se, si, sx, L;
   xs_lookup(P, Eev, se, si, sx, L);
   const double nu_el = n_gas * se * v, nu_io = n_gas * si * v, nu_ex = n_gas * sx * v;
@@ -305,18 +306,18 @@ __device__ __forceinline__ int mcc_event(const SimParams &P, uint64_t id, long l
     // E_1 = T_0 + t tan(U (k_1 + k_2) - k_2), k_1 = atan((T_m - T_0)/t),
     // k_2 = atan(T_0/t): with k_1 + k_2 from one atan2 and
     // tan(x - k_2) = (tan x - tan k_2) / (1 + tan x tan k_2)
-    const double a1 = (T_m - T_0) / t, a2 = T_0 / t;
+    const double it = 1 / t, a1 = (T_m - T_0) * it, a2 = T_0 * it;
     const double tx = tan(d1.a * atan2(a1 + a2, 1 - a1 * a2));
     const double k0 = T_0 + t * ((tx - a2) / (1 + a2 * tx));
     const double E_1 = k0, E_2 = T - E_1 - I;
     double E_p, E_s;
     if (E_2 > E_1) { E_p = E_2; E_s = E_1; } else { E_p = E_1; E_s = E_2; }
-    const double E_e = me * c * c / qe;
     // polar angles as sines (the reference's asin arguments) and cosines
-    const double sp2 = (E_s / T) / ((1 - E_s / T) * T / (2 * E_e) + 1);
-    const double ss2 = (1 - E_s / T) / (1 + E_s / (2 * E_e));
-    const double ix = ux / um, iy = uy / um, iz = uz / um;
-    const double up = u_of_energy(E_p * qe, me, c), us = u_of_energy(E_s * qe, me, c);
+    const double h = 0.5 * P.imc2_ev, es = E_s / T;
+    const double sp2 = es / ((T - E_s) * h + 1);
+    const double ss2 = (1 - es) / (E_s * h + 1);
+    const double ix = ux * ium, iy = uy * ium, iz = uz * ium;
+    const double up = u_of_energy(P, E_p), us = u_of_energy(P, E_s);
     ux = ix * up; uy = iy * up; uz = iz * up;
     turn<FAST>(ux, uy, uz, sqrt(sp2), sqrt(1 - sp2), d1.b, 1.0);
     if (P.secondaries) {
@@ -336,8 +337,8 @@ __device__ __forceinline__ int mcc_event(const SimParams &P, uint64_t id, long l
     else { i = (int)L; f = L - i; }
     const double E_dep = P.edep[i] + f * (P.edep[i + 1] - P.edep[i]);
     if (!(E_dep > 0) || !(E_dep < Eev)) return 4;
-    const double up = u_of_energy((Eev - E_dep) * qe, me, c);
-    ux = ux / um * up; uy = uy / um * up; uz = uz / um * up;
+    const double up = u_of_energy(P, Eev - E_dep) * ium;
+    ux *= up; uy *= up; uz *= up;
     b.eloss = E_dep;
     return 3;
   }
@@ -3157,6 +3158,7 @@ int gasatt_sim_create(gasatt_ctx *ctx, const gasatt_sim_config *cfg, const gasat
   P.cdf = s->d_tab + 4 * c.table_n;
   P.exc_kmin = s->tabs.exc_kmin;
   P.G = c.table_n; P.lnEmin = s->tabs.lnEmin; P.dlnE = s->tabs.dlnE;
+  P.mc2_ev = c.m_e * c.c * c.c / c.q_e; P.imc2_ev = 1 / P.mc2_ev; P.idlnE = 1 / P.dlnE;
   P.n_exc = s->tabs.n_exc;
   std::memcpy(P.exc, s->tabs.exc, sizeof(P.exc));
   P.Jr = s->Jr[0]; P.Jz = s->Jz[0];
