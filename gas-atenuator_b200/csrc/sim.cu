@@ -2389,6 +2389,13 @@ __global__ void k_field_energy(const T *Er, const T *Ez, const T *H, int nr, int
 
 }  // namespace
 
+// Steps that one graph launch takes where no sort, ion push or odd start falls
+// between them.  A graph of one step each leaves the GPU idle for a launch's
+// time between steps: 2 to 3 us of every step (64 x 256 cells FP64 16.8 us a step
+// with graphs of one step, 14.1 with ten; 2M electrons FP32 55.2 and 53.1).  Ten
+// divides the usual sort periods.
+constexpr int kGraphSteps = 10;
+
 // ================================================================ sim object
 struct gasatt_sim {
   gasatt_ctx *ctx = nullptr;
@@ -2438,6 +2445,7 @@ struct gasatt_sim {
   int64_t since_sort = 0;
   cudaGraphExec_t g_step[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [state buffer][step parity]
   cudaGraph_t gr_step[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};     // the same, not instantiated
+  cudaGraphExec_t g_steps[2] = {nullptr, nullptr};   // kGraphSteps steps from parity 0 on [state buffer]
   cudaGraphExec_t g_sort[2] = {nullptr, nullptr};
   cudaGraph_t gr_sort[2] = {nullptr, nullptr};       // the same, not instantiated
   double scale = 1.0;
@@ -2660,6 +2668,14 @@ bool ion_push_due(const gasatt_sim *s) {
   return s->cfg.ion_capacity > 0 && s->host_step % s->cfg.ion_subcycle == 0;
 }
 
+// whether kGraphSteps more steps end at the latest with the step before the
+// next sort, and with the next ion push
+bool steps_fit(const gasatt_sim *s, int sort_period) {
+  const auto &c = s->cfg;
+  return (sort_period <= 0 || sort_period - s->since_sort >= kGraphSteps) &&
+         (c.ion_capacity <= 0 || c.ion_subcycle - s->host_step % c.ion_subcycle >= kGraphSteps);
+}
+
 // sort from buffer `from` into 1 - from
 int launch_sort(gasatt_sim *s, cudaStream_t st, int from) {
   const auto &c = s->cfg;
@@ -2689,6 +2705,8 @@ int launch_sort(gasatt_sim *s, cudaStream_t st, int from) {
 
 void drop_graphs(gasatt_sim *s) {
   for (int i = 0; i < 2; ++i) {
+    if (s->g_steps[i]) cudaGraphExecDestroy(s->g_steps[i]);
+    s->g_steps[i] = nullptr;
     for (int q = 0; q < 2; ++q) {
       if (s->g_step[i][q]) cudaGraphExecDestroy(s->g_step[i][q]);
       s->g_step[i][q] = nullptr;
@@ -2902,6 +2920,62 @@ int sim_prime(gasatt_sim *s) {
 //
 // The field update needs only the current of pass s-1 and the collisions only
 // the particles, so the two run side by side.  Also one sort b -> 1-b.
+int capture_step(gasatt_sim *s, cudaStream_t cs, cudaStream_t side, int q) {
+  int rc = GASATT_OK;
+  cudaError_t e = cudaSuccess;
+  auto mark = [&](int k, cudaStream_t st) {
+    if (e == cudaSuccess && !rc && s->timing) e = cudaEventRecordWithFlags(s->ev[k], st, cudaEventRecordExternal);
+  };
+  if (s->form == 1) {
+    // FP32: the field kernel commits the previous pass, the pass runs the
+    // previous step's collisions itself.  Timing: one event before, one
+    // between and one after the two kernels (the pass's collisions have
+    // no kernel of their own)
+    mark(0, cs);
+    if (e == cudaSuccess) rc = launch_fdtd(s, cs, q);
+    mark(1, cs);
+    if (e == cudaSuccess && !rc) rc = launch_pass(s, cs, 0, 1 - q, q, 1 - q);
+    mark(3, cs);
+  } else {
+    e = cudaEventRecord(s->fork_ev, cs);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(side, s->fork_ev, 0);
+    mark(4, side);
+    if (e == cudaSuccess) rc = launch_mcc(s, side, 1 - q);
+    mark(5, side);
+    if (e == cudaSuccess && !rc) e = cudaEventRecord(s->join_ev, side);
+    mark(0, cs);
+    if (e == cudaSuccess && !rc) rc = launch_fdtd(s, cs, q);
+    mark(1, cs);
+    if (e == cudaSuccess && !rc) e = cudaStreamWaitEvent(cs, s->join_ev, 0);
+    mark(2, cs);
+    if (e == cudaSuccess && !rc) rc = launch_pass(s, cs, 0, 1 - q, q, 1 - q);
+    mark(3, cs);
+  }
+  if (!rc && e != cudaSuccess) rc = cuda_fail(s->ctx, e, "capture step");
+  return rc;
+}
+
+// `count` steps, the first of parity q, as one graph; the graph itself is
+// kept where `keep` is given
+int capture_steps(gasatt_sim *s, cudaStream_t cs, cudaStream_t side, int q, int count, cudaGraphExec_t *exec,
+                  cudaGraph_t *keep) {
+  cudaGraph_t g;
+  GASATT_CUDA(s->ctx, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
+  int rc = GASATT_OK;
+  for (int k = 0; k < count && !rc; ++k) rc = capture_step(s, cs, side, (q + k) & 1);
+  cudaError_t e = cudaStreamEndCapture(cs, &g);
+  const bool captured = e == cudaSuccess;
+  if (!rc && !captured) rc = cuda_fail(s->ctx, e, "capture step");
+  if (!rc) {
+    e = cudaGraphInstantiate(exec, g, 0);
+    if (e != cudaSuccess) rc = cuda_fail(s->ctx, e, "instantiate step");
+  }
+  if (captured) {
+    if (!rc && keep) *keep = g; else cudaGraphDestroy(g);
+  }
+  return rc;
+}
+
 int build_graphs(gasatt_sim *s) {
   // the field update goes on a higher-priority stream than the collision
   // branch, so its blocks are placed first when both are ready
@@ -2916,57 +2990,8 @@ int build_graphs(gasatt_sim *s) {
   for (int b = 0; b < 2 && !rc; ++b) {
     cudaGraph_t g;
     s->cur = b;
-    for (int q = 0; q < 2 && !rc; ++q) {
-      GASATT_CUDA(s->ctx, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-      if (s->form == 1) {
-        // FP32: the field kernel commits the previous pass, the pass runs the
-        // previous step's collisions itself.  Timing: one event before, one
-        // between and one after the two kernels (the pass's collisions have
-        // no kernel of their own)
-        cudaError_t e = cudaSuccess;
-        if (s->timing) e = cudaEventRecordWithFlags(s->ev[0], cs, cudaEventRecordExternal);
-        if (e == cudaSuccess) rc = launch_fdtd(s, cs, q);
-        if (e == cudaSuccess && !rc && s->timing)
-          e = cudaEventRecordWithFlags(s->ev[1], cs, cudaEventRecordExternal);
-        if (e == cudaSuccess && !rc) rc = launch_pass(s, cs, 0, 1 - q, q, 1 - q);
-        if (e == cudaSuccess && !rc && s->timing)
-          e = cudaEventRecordWithFlags(s->ev[3], cs, cudaEventRecordExternal);
-        cudaError_t e2 = cudaStreamEndCapture(cs, &g);
-        if (!rc && e != cudaSuccess) rc = cuda_fail(s->ctx, e, "capture step");
-        if (!rc && e2 != cudaSuccess) rc = cuda_fail(s->ctx, e2, "capture step");
-        if (!rc) {
-          e = cudaGraphInstantiate(&s->g_step[b][q], g, 0);
-          if (e != cudaSuccess) rc = cuda_fail(s->ctx, e, "instantiate step");
-        }
-        if (e2 == cudaSuccess) {
-          if (!rc) s->gr_step[b][q] = g; else cudaGraphDestroy(g);
-        }
-        continue;
-      }
-      cudaError_t e = cudaEventRecord(s->fork_ev, cs);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(side, s->fork_ev, 0);
-      if (e == cudaSuccess && s->timing) e = cudaEventRecordWithFlags(s->ev[4], side, cudaEventRecordExternal);
-      if (e == cudaSuccess) rc = launch_mcc(s, side, 1 - q);
-      if (e == cudaSuccess && !rc && s->timing) e = cudaEventRecordWithFlags(s->ev[5], side, cudaEventRecordExternal);
-      if (e == cudaSuccess && !rc) e = cudaEventRecord(s->join_ev, side);
-      if (e == cudaSuccess && !rc && s->timing) e = cudaEventRecordWithFlags(s->ev[0], cs, cudaEventRecordExternal);
-      if (e == cudaSuccess && !rc) rc = launch_fdtd(s, cs, q);
-      if (e == cudaSuccess && !rc && s->timing) e = cudaEventRecordWithFlags(s->ev[1], cs, cudaEventRecordExternal);
-      if (e == cudaSuccess && !rc) e = cudaStreamWaitEvent(cs, s->join_ev, 0);
-      if (e == cudaSuccess && !rc && s->timing) e = cudaEventRecordWithFlags(s->ev[2], cs, cudaEventRecordExternal);
-      if (e == cudaSuccess && !rc) rc = launch_pass(s, cs, 0, 1 - q, q, 1 - q);
-      if (e == cudaSuccess && !rc && s->timing) e = cudaEventRecordWithFlags(s->ev[3], cs, cudaEventRecordExternal);
-      cudaError_t e2 = cudaStreamEndCapture(cs, &g);
-      if (!rc && e != cudaSuccess) rc = cuda_fail(s->ctx, e, "capture step");
-      if (!rc && e2 != cudaSuccess) rc = cuda_fail(s->ctx, e2, "capture step");
-      if (!rc) {
-        e = cudaGraphInstantiate(&s->g_step[b][q], g, 0);
-        if (e != cudaSuccess) rc = cuda_fail(s->ctx, e, "instantiate step");
-      }
-      if (e2 == cudaSuccess) {
-        if (!rc) s->gr_step[b][q] = g; else cudaGraphDestroy(g);
-      }
-    }
+    for (int q = 0; q < 2 && !rc; ++q) rc = capture_steps(s, cs, side, q, 1, &s->g_step[b][q], &s->gr_step[b][q]);
+    if (!rc && !s->timing) rc = capture_steps(s, cs, side, 0, kGraphSteps, &s->g_steps[b], nullptr);
     if (rc) break;
     GASATT_CUDA(s->ctx, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     rc = launch_sort(s, cs, b);
@@ -3688,10 +3713,15 @@ int gasatt_sim_step(gasatt_sim *s, int nsteps) {
   if (nsteps > 0) SIM_TRY(clear_after_batch(s, st, (int)((s->host_step - 1) & 1)));
   for (int k = 0; k < nsteps; ++k) {
     if (s->cfg.sort_period > 0 && s->since_sort >= s->cfg.sort_period) SIM_TRY(gasatt_sim_sort(s));
-    GASATT_CUDA(ctx, cudaGraphLaunch(s->g_step[s->cur][s->host_step & 1], st));
-    ctx->launches += per_step;
-    s->host_step++;
-    s->since_sort++;
+    // several steps by one launch: from an even step, up to the next sort and ion push
+    int many = 1;
+    if (s->g_steps[s->cur] && !(s->host_step & 1) && nsteps - k >= kGraphSteps && steps_fit(s, s->cfg.sort_period))
+      many = kGraphSteps;
+    GASATT_CUDA(ctx, cudaGraphLaunch(many > 1 ? s->g_steps[s->cur] : s->g_step[s->cur][s->host_step & 1], st));
+    ctx->launches += many * per_step;
+    s->host_step += many;
+    s->since_sort += many;
+    k += many - 1;
     s->mcc_pending = true;
     if (ion_push_due(s)) SIM_TRY(launch_ion_push(s, st));
   }
@@ -3951,6 +3981,7 @@ struct gasatt_batch {
   int sort_period = 0;
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   cudaGraphExec_t g[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [state buffer][parity]
+  cudaGraphExec_t g_steps[2] = {nullptr, nullptr};  // kGraphSteps steps from parity 0 on [state buffer]
   cudaGraphExec_t g_sort[2] = {nullptr, nullptr};   // every cell's sort side by side [state buffer]
 };
 
@@ -3961,6 +3992,7 @@ int gasatt_batch_destroy(gasatt_batch *b) {
   for (int i = 0; i < 2; ++i) {
     for (int q = 0; q < 2; ++q)
       if (b->g[i][q]) cudaGraphExecDestroy(b->g[i][q]);
+    if (b->g_steps[i]) cudaGraphExecDestroy(b->g_steps[i]);
     if (b->g_sort[i]) cudaGraphExecDestroy(b->g_sort[i]);
   }
   if (b->fork_ev) cudaEventDestroy(b->fork_ev);
@@ -4104,6 +4136,46 @@ int batch_group_launch(gasatt_batch *b, BatchGroup &G, cudaStream_t cs, cudaStre
   return GASATT_OK;
 }
 
+// `count` steps of the batch (state buffer bi, the first of parity q) as one
+// graph: a branch per group and per cell of its own, each its steps in turn
+int batch_capture_steps(gasatt_batch *b, cudaStream_t cs, cudaStream_t side, int bi, int q, int count,
+                        cudaGraphExec_t *exec) {
+  gasatt_ctx *ctx = b->ctx;
+  int rc = GASATT_OK;
+  cudaGraph_t g = nullptr;
+  cudaError_t e = cudaGraphCreate(&g, 0);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "batch graph");
+  for (BatchGroup &G : b->groups) {
+    cudaGraph_t child = nullptr;
+    e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) { rc = cuda_fail(ctx, e, "batch capture"); break; }
+    for (int k = 0; k < count && !rc; ++k) rc = batch_group_launch(b, G, cs, side, bi, (q + k) & 1);
+    const cudaError_t e2 = cudaStreamEndCapture(cs, &child);
+    if (!rc && e2 != cudaSuccess) rc = cuda_fail(ctx, e2, "batch capture");
+    if (!rc) {
+      cudaGraphNode_t node;
+      e = cudaGraphAddChildGraphNode(&node, g, nullptr, 0, child);
+      if (e != cudaSuccess) rc = cuda_fail(ctx, e, "batch graph");
+    }
+    if (child) cudaGraphDestroy(child);
+    if (rc) break;
+  }
+  for (size_t i = 0; i < b->singles.size() && !rc; ++i) {
+    cudaGraphNode_t last, node;
+    for (int k = 0; k < count && !rc; ++k, last = node) {
+      e = cudaGraphAddChildGraphNode(&node, g, k > 0 ? &last : nullptr, k > 0 ? 1 : 0,
+                                     b->singles[i]->gr_step[bi][(q + k) & 1]);
+      if (e != cudaSuccess) rc = cuda_fail(ctx, e, "batch graph");
+    }
+  }
+  if (!rc) {
+    e = cudaGraphInstantiate(exec, g, 0);
+    if (e != cudaSuccess) rc = cuda_fail(ctx, e, "batch graph");
+  }
+  cudaGraphDestroy(g);
+  return rc;
+}
+
 int batch_build_graphs(gasatt_batch *b) {
   gasatt_ctx *ctx = b->ctx;
   cudaStream_t cs, side;
@@ -4128,37 +4200,10 @@ int batch_build_graphs(gasatt_batch *b) {
     }
     cudaGraphDestroy(g);
   }
-  for (int bi = 0; bi < 2 && !rc; ++bi)
-    for (int q = 0; q < 2 && !rc; ++q) {
-      cudaGraph_t g = nullptr;
-      cudaError_t e = cudaGraphCreate(&g, 0);
-      if (e != cudaSuccess) { rc = cuda_fail(ctx, e, "batch graph"); break; }
-      for (BatchGroup &G : b->groups) {
-        cudaGraph_t child = nullptr;
-        e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-        if (e != cudaSuccess) { rc = cuda_fail(ctx, e, "batch capture"); break; }
-        rc = batch_group_launch(b, G, cs, side, bi, q);
-        const cudaError_t e2 = cudaStreamEndCapture(cs, &child);
-        if (!rc && e2 != cudaSuccess) rc = cuda_fail(ctx, e2, "batch capture");
-        if (!rc) {
-          cudaGraphNode_t node;
-          e = cudaGraphAddChildGraphNode(&node, g, nullptr, 0, child);
-          if (e != cudaSuccess) rc = cuda_fail(ctx, e, "batch graph");
-        }
-        if (child) cudaGraphDestroy(child);
-        if (rc) break;
-      }
-      for (size_t i = 0; i < b->singles.size() && !rc; ++i) {
-        cudaGraphNode_t node;
-        e = cudaGraphAddChildGraphNode(&node, g, nullptr, 0, b->singles[i]->gr_step[bi][q]);
-        if (e != cudaSuccess) rc = cuda_fail(ctx, e, "batch graph");
-      }
-      if (!rc) {
-        e = cudaGraphInstantiate(&b->g[bi][q], g, 0);
-        if (e != cudaSuccess) rc = cuda_fail(ctx, e, "batch graph");
-      }
-      cudaGraphDestroy(g);
-    }
+  for (int bi = 0; bi < 2 && !rc; ++bi) {
+    for (int q = 0; q < 2 && !rc; ++q) rc = batch_capture_steps(b, cs, side, bi, q, 1, &b->g[bi][q]);
+    if (!rc) rc = batch_capture_steps(b, cs, side, bi, 0, kGraphSteps, &b->g_steps[bi]);
+  }
   cudaStreamDestroy(side);
   cudaStreamDestroy(cs);
   return rc;
@@ -4280,13 +4325,18 @@ int gasatt_batch_step(gasatt_batch *b, int nsteps) {
     }
     const gasatt_sim *s0 = b->sims[0];
     bool lockstep = true;
-    for (const gasatt_sim *s : b->sims)
+    // several steps by one launch: from an even step, up to every cell's next sort and ion push
+    int many = !(s0->host_step & 1) && nsteps - k >= kGraphSteps ? kGraphSteps : 1;
+    for (const gasatt_sim *s : b->sims) {
       lockstep = lockstep && s->cur == s0->cur && (s->host_step & 1) == (s0->host_step & 1) &&
                  !s->timing;
+      if (!steps_fit(s, b->sort_period)) many = 1;
+    }
+    if (!lockstep) many = 1;
     if (lockstep) {
-      GASATT_CUDA(ctx, cudaGraphLaunch(b->g[s0->cur][s0->host_step & 1], st));
-      for (const BatchGroup &G : b->groups) ctx->launches += G.form == 0 ? 4 : 2;
-      for (const gasatt_sim *s : b->singles) ctx->launches += s->form == 0 ? 3 : 2;
+      GASATT_CUDA(ctx, cudaGraphLaunch(many > 1 ? b->g_steps[s0->cur] : b->g[s0->cur][s0->host_step & 1], st));
+      for (const BatchGroup &G : b->groups) ctx->launches += many * (G.form == 0 ? 4 : 2);
+      for (const gasatt_sim *s : b->singles) ctx->launches += many * (s->form == 0 ? 3 : 2);
       for (const BatchGroup &G : b->groups)
         for (gasatt_sim *s : G.sims) s->batch_pass = true;
     } else {
@@ -4297,11 +4347,12 @@ int gasatt_batch_step(gasatt_batch *b, int nsteps) {
       }
     }
     for (gasatt_sim *s : b->sims) {
-      s->host_step++;
-      s->since_sort++;
+      s->host_step += many;
+      s->since_sort += many;
       s->mcc_pending = true;
       if (ion_push_due(s)) SIM_TRY(launch_ion_push(s, st));
     }
+    k += many - 1;
   }
   return GASATT_OK;
 }
