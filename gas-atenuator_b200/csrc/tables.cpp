@@ -145,6 +145,8 @@ int build_sim_tables(const gasatt_tables *t, int G, double emin_ev, double emax_
   }
   const double h = GASATT_PI / 180;
   const int ne = el.ne;
+  double sines[181];
+  for (int k = 0; k <= 180; ++k) sines[k] = std::sin(k * h);
   for (int g = 0; g < G; ++g) {
     double le = std::log(Eg[g] / 1000);
     if (le < el.xInterp[0]) le = el.xInterp[0];
@@ -158,7 +160,7 @@ int build_sim_tables(const gasatt_tables *t, int G, double emin_ev, double emax_
     C[0] = 0;
     for (int k = 0; k <= 180; ++k) {
       const double vI = a0 * el.V[(size_t)i * 181 + k] + b0 * el.V[(size_t)(i + 1) * 181 + k];
-      const double pdf = 2 * GASATT_PI * std::sin(k * h) * std::exp(vI) * 2;
+      const double pdf = 2 * GASATT_PI * sines[k] * std::exp(vI) * 2;
       if (k > 0) C[k] = C[k - 1] + (prev + pdf) / 2 * h;
       prev = pdf;
     }
