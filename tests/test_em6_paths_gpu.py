@@ -39,3 +39,24 @@ def test_against_oracle(nr, nz, n, steps, PHIp, flags):
     # 1e-12 of each quantity's largest value, as the drop-in's own test
     for g, w, k in zip(got, want, ("e_pos", "e_vel", "i1_pos", "i1_vel", "i2_pos", "i2_vel", "Er", "Ez", "Hphi", "kin")):
         close(g.cpu().numpy(), w, 1e-12, k)
+
+
+@pytest.mark.parametrize("n,steps", [(68000, 9), (67742, 12), (67743, 10), (70000, 35)])
+def test_sorted_particles(n, steps):
+    """From 100,000 particles (n + n / 3 + n / 7) and ten steps on the particles
+    are sorted by cell, and again after 25 steps: electrons that leave before
+    and after a sort, order and energies as without it."""
+    rng = np.random.default_rng(n + steps)
+    d, nr, nz, PHIp = 1e-4, 24, 60, 0.1
+    Er, Ez, H = grid_fields(nr, nz, rng, E0=3e5, H0=300.0)
+    e = wedge_particles(n, nr * d, nz * d, PHIp, rng, vmag=4e7)
+    i1 = wedge_particles(n // 3, nr * d, nz * d, PHIp, rng, vmag=2e3)
+    i2 = wedge_particles(n // 7, nr * d, nz * d, PHIp, rng, vmag=2e3)
+    args = (*e, *i1, *i2, Er, Ez, H, d, 1e-13, nr * d, nz * d, PHIp, 100.0, 5 * steps)
+    flags = _lib.FAITHFUL | _lib.POS_IN_CYL
+    got = gasatt.electricmagneticfield6(*[torch.tensor(a) if isinstance(a, np.ndarray) else a for a in args],
+                                        flags=flags)
+    want = O.electricmagneticfield6(*args, flags)
+    # as above, times the number of steps: the rounding errors of a step add up
+    for g, w, k in zip(got, want, ("e_pos", "e_vel", "i1_pos", "i1_vel", "i2_pos", "i2_vel", "Er", "Ez", "Hphi", "kin")):
+        close(g.cpu().numpy(), w, 1e-12 * steps, k)
