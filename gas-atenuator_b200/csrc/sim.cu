@@ -748,6 +748,9 @@ __global__ void __launch_bounds__(kBlock, 3) k_pass64(SimParams P, State64 S, Fi
                                                       SimCounters *cnt, int *queue, int q) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int box_row0[2], box_rows[2], box_col0[2], box_cmax[2];   // of this chunk and the next
+  // the window starts zeroed; each chunk's flush leaves it zeroed again
+  for (int i = threadIdx.x; i < kWin64Nodes; i += kBlock) reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0, 0, 0, 0);
+  // (never started early: it follows the field update and the collisions)
   const long long n0 = slots_in_use(cnt);
   const long long step = cnt->step64[1 - q] + 1;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -756,8 +759,6 @@ __global__ void __launch_bounds__(kBlock, 3) k_pass64(SimParams P, State64 S, Fi
   }
   const int chunk = even_chunk((unsigned)n0, gridDim.x, kChunk64);
   const int cols = win_cols(P.nr), ws = win_stride(cols), maxrows = min(kWin64Nodes / ws, P.nz);
-  // the window starts zeroed; each chunk's flush leaves it zeroed again
-  for (int i = threadIdx.x; i < kWin64Nodes; i += kBlock) reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0, 0, 0, 0);
   // the blocks take the chunks in turn, so neighbouring blocks work on
   // neighbouring grid rows; thread 0 brings the block's next chunk into L2
   // and, at the end of this one, places its box
@@ -783,6 +784,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_pass64(SimParams P, State64 S, Fi
     flush64(P, w, box_cmax[b] + 1);
     __syncthreads();
   }
+  let_next_start();
 }
 
 // The collision of candidate slot p queued at step `step` (FP64 form): MCC,
@@ -885,7 +887,7 @@ __global__ void __launch_bounds__(kMccBlock) k_batch_mcc64(const BatchCell64 *__
 }
 
 // The FP64 pass of every cell of a batch: (cell, chunk) work items from one
-// counter (*chunk_next, zeroed before the launch), the cell's parameters
+// counter (*chunk_next, zeroed by the field kernel), the cell's parameters
 // copied into shared memory when the cell changes.
 __global__ void __launch_bounds__(kBlock, 3) k_batch_pass64(const BatchCell64 *__restrict__ cells,
                                                             int ncell, int cur, int jb, int q,
@@ -969,6 +971,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_batch_pass64(const BatchCell64 *_
     flush64(sP, w, box_cmax + 1);
     __syncthreads();
   }
+
 }
 
 // ----------------------------------------------------------- ions
@@ -1639,12 +1642,13 @@ __global__ void __launch_bounds__(kBlock, 4) k_pass32(SimParams P, State32 S, Fi
   __shared__ int win_row0, win_rows, win_col0;
   __shared__ int box_cmax;                       // highest window column the chunk touched
   __shared__ long long chunk_at;
+  // the window starts zeroed; each chunk's flush leaves it zeroed again
+  for (int i = threadIdx.x; i < kWinNodes; i += kBlock) reinterpret_cast<int2 *>(win_rz)[i] = make_int2(0, 0);
+  wait_for_previous();
   const long long n0 = (long long)cnt->n_total;   // births of this pass land beyond
   const long long step = cnt->step;
   const int par = (int)(step & 1);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // the window starts zeroed; each chunk's flush leaves it zeroed again
-  for (int i = threadIdx.x; i < kWinNodes; i += kBlock) reinterpret_cast<int2 *>(win_rz)[i] = make_int2(0, 0);
   const int cols = win_cols(P.nr), ws = win_stride(cols);
   const int maxrows = min(kWinNodes / ws, P.nz);
   const int chunk = max(cnt->chunk, kBlock);      // chosen with the commit (no division here)
@@ -1704,6 +1708,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_pass32(SimParams P, State32 S, Fi
     flush32(P, w, box_cmax + 1);
     __syncthreads();
   }
+  let_next_start();
 }
 
 // ------------------------------------------------------- batched FP32 pass
@@ -1722,7 +1727,7 @@ struct BatchCell32 {
 // block reads the cells' counters and forms the prefix sums of their
 // collision candidates and chunks; the candidates of all cells go first, one
 // per warp, then the blocks take (cell, chunk) work items from one counter
-// (*chunk_next, zeroed before the launch), copying the cell's parameters into
+// (*chunk_next, zeroed by the field kernel), copying the cell's parameters into
 // shared memory when the cell changes.  Every cell gives what its own
 // k_pass32 gives.
 template <bool WIDE>
@@ -1742,6 +1747,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_batch_pass32(const BatchCell32 *_
   for (int i = threadIdx.x; i < kWinNodes; i += kBlock) reinterpret_cast<int2 *>(win_rz)[i] = make_int2(0, 0);
   if (threadIdx.x == 0) total = 0;
   __syncthreads();
+  wait_for_previous();
   // per-cell candidates (of the previous pass) and chunks, then prefix sums
   for (int c = threadIdx.x; c < ncell; c += kBlock) {
     const SimCounters *cc = cells[c].cnt;
@@ -1837,6 +1843,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_batch_pass32(const BatchCell32 *_
     __syncthreads();
     flush32(sP, w, box_cmax + 1);
   }
+  let_next_start();
 }
 
 // The collisions still queued by the last FP32 pass, without the next push
@@ -1917,8 +1924,10 @@ __device__ __forceinline__ void commit_pass32(SimCounters *cnt) {
 template <typename T, int K>
 __global__ void __launch_bounds__(32 * tma_warps(K), tma_blocks(K)) k_sim_fdtd_tma(
     const __grid_constant__ FdtdInst I, SimCounters *cnt) {
+  wait_for_previous();
   if (cnt && blockIdx.x == 0 && threadIdx.x == 0) commit_pass32(cnt);
   fdtd_block_body<T, K>(FdtdWork{&I, nullptr, I.ntiles});
+  let_next_start();
 }
 
 // The field update of every cell of a batch in one launch: the blocks walk a
@@ -1926,14 +1935,18 @@ __global__ void __launch_bounds__(32 * tma_warps(K), tma_blocks(K)) k_sim_fdtd_t
 // commit the previous pass of every cell.
 template <typename T, int K>
 __global__ void __launch_bounds__(32 * tma_warps(K), tma_blocks(K)) k_batch_fdtd_tma(
-    const FdtdInst *insts, const int2 *table, int nitems, SimCounters *const *commit, int ninst) {
+    const FdtdInst *insts, const int2 *table, int nitems, SimCounters *const *commit, int ninst,
+    unsigned long long *chunk_next) {
+  wait_for_previous();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *chunk_next = 0;        // the pass's, which runs next
   if (commit && threadIdx.x == 0)
     for (int i = blockIdx.x; i < ninst; i += gridDim.x) commit_pass32(commit[i]);
   fdtd_block_body<T, K>(FdtdWork{insts, table, nitems});
+  let_next_start();
 }
 
 using SimFdtdTmaFn = void (*)(const FdtdInst, SimCounters *);
-using BatchFdtdTmaFn = void (*)(const FdtdInst *, const int2 *, int, SimCounters *const *, int);
+using BatchFdtdTmaFn = void (*)(const FdtdInst *, const int2 *, int, SimCounters *const *, int, unsigned long long *);
 
 // the instance of each kernel, and its dynamic shared memory, for knob value `rows`
 template <typename T>
@@ -1962,6 +1975,8 @@ __global__ void __launch_bounds__(32 * kFdtdRows, 3) k_sim_fdtd(Fields<T> in, Fi
                                                   double dt, int R, unsigned flags,
                                                   SimCounters *cnt, ExtraCurrent ion,
                                                   FieldQuads quads) {
+  wait_for_previous();
+  let_next_start();
   if (cnt && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0)
     commit_pass32(cnt);
   fdtd_tiled<T>(in.Er, in.Ez, in.H, out.Er, out.Ez, out.H, Jr, Jz, Jr_next, Jz_next, nr, nz, ldf, ldj,
@@ -2507,7 +2522,7 @@ inline int fcur(const gasatt_sim *s) { return (int)(s->host_step & 1); }
 
 // field update of a step of parity q: reads field buffer q and current
 // buffer q, writes field buffer 1 - q and clears current buffer 1 - q
-int launch_fdtd(gasatt_sim *s, cudaStream_t st, int q) {
+int launch_fdtd(gasatt_sim *s, cudaStream_t st, int q, bool early = false) {
   const auto &c = s->cfg;
   const int nr = c.n_r, nz = c.n_z, R = c.fdtd_ratio;
   const FdtdCoef fc = fdtd_coef(s);
@@ -2516,57 +2531,50 @@ int launch_fdtd(gasatt_sim *s, cudaStream_t st, int q) {
   const ExtraCurrent ion{s->Jir, s->Jiz, s->scale / s->ion_scale};
   if (R == 1) {
     const dim3 block(32 * tma_warps(s->tma_rows));
-    if (s->form == 0)
-      sim_fdtd_tma_fn<double>(s->tma_rows)<<<s->tma_grid, block, s->tma_smem, st>>>(s->fdtd_inst[q], nullptr);
-    else
-      sim_fdtd_tma_fn<float>(s->tma_rows)<<<s->tma_grid, block, s->tma_smem, st>>>(s->fdtd_inst[q], s->cnt);
+    const cudaError_t e =
+        launch_early(early, s->form == 0 ? sim_fdtd_tma_fn<double>(s->tma_rows) : sim_fdtd_tma_fn<float>(s->tma_rows),
+                     dim3(s->tma_grid), block, s->tma_smem, st, s->fdtd_inst[q], s->form == 0 ? nullptr : s->cnt);
     s->ctx->launches++;
-    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(s->ctx, e, "fdtd launch");
     return GASATT_OK;
   }
   const int tile = fdtd_tile(R);
   const dim3 grid((nr + 1 + tile - 1) / tile, (nz + 1 + tile - 1) / tile);
   const dim3 block(32, kFdtdRows);
-  auto k64 = k_sim_fdtd<double>;
-  auto k32 = k_sim_fdtd<float>;
+  cudaError_t e;
   if (s->form == 0)
-    k64<<<grid, block, 0, st>>>(
-        fields_of<double>(s, q), fields_of<double>(s, 1 - q), s->Jr[q], s->Jz[q], s->Jr[1 - q],
-        s->Jz[1 - q], nr, nz, s->ldf, s->ldj, fc, s->invV, c.mu0, dt, R, c.flags, nullptr, ion, FieldQuads{});
+    e = launch_early(early, k_sim_fdtd<double>, grid, block, 0, st, fields_of<double>(s, q), fields_of<double>(s, 1 - q),
+                     s->Jr[q], s->Jz[q], s->Jr[1 - q], s->Jz[1 - q], nr, nz, s->ldf, s->ldj, fc, s->invV, c.mu0, dt, R,
+                     c.flags, nullptr, ion, FieldQuads{});
   else
-    k32<<<grid, block, 0, st>>>(
-        fields_of<float>(s, q), fields_of<float>(s, 1 - q), s->Jr[q], s->Jz[q], s->Jr[1 - q],
-        s->Jz[1 - q], nr, nz, s->ldf, s->ldj, fc, s->invV, c.mu0, dt, R, c.flags, s->cnt, ion, s->quads);
+    e = launch_early(early, k_sim_fdtd<float>, grid, block, 0, st, fields_of<float>(s, q), fields_of<float>(s, 1 - q),
+                     s->Jr[q], s->Jz[q], s->Jr[1 - q], s->Jz[1 - q], nr, nz, s->ldf, s->ldj, fc, s->invV, c.mu0, dt, R,
+                     c.flags, s->cnt, ion, s->quads);
   s->ctx->launches++;
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(s->ctx, e, "fdtd launch");
   return GASATT_OK;
 }
 
 // particle pass; its collision candidates (mode 0) go to queue q, its
 // current to buffer jb; it gathers from field buffer fb
-int launch_pass(gasatt_sim *s, cudaStream_t st, int mode, int jb, int q, int fb) {
+int launch_pass(gasatt_sim *s, cudaStream_t st, int mode, int jb, int q, int fb, bool early = false) {
   SimParams P = s->P;
   P.Jr = s->Jr[jb];
   P.Jz = s->Jz[jb];
   const int b = s->cur;
-  if (s->form == 0)
-  {
+  cudaError_t e;
+  if (s->form == 0) {
     auto kern = mode == 0 ? k_pass64<0> : mode == 1 ? k_pass64<1> : k_pass64<2>;
-    kern<<<s->pass_grid, kBlock, kWin64Bytes, st>>>(P, s->s64[b], fields_of<double>(s, fb), s->cnt,
-                                                    s->queue, q);
-  }
-  else
-  {
+    e = launch_early(early, kern, dim3(s->pass_grid), dim3(kBlock), kWin64Bytes, st, P, s->s64[b],
+                     fields_of<double>(s, fb), s->cnt, s->queue, q);
+  } else {
     auto kern = win_cols(P.nr) < P.nr
                     ? (mode == 0 ? k_pass32<0, true> : mode == 1 ? k_pass32<1, true> : k_pass32<2, true>)
                     : (mode == 0 ? k_pass32<0, false> : mode == 1 ? k_pass32<1, false> : k_pass32<2, false>);
-    kern<<<s->pass_grid, kBlock, 0, st>>>(P, s->s32[b], fields_of<float>(s, fb), s->cnt, s->queue,
-                                          s->d_P + jb);
+    e = launch_early(early, kern, dim3(s->pass_grid), dim3(kBlock), 0, st, P, s->s32[b], fields_of<float>(s, fb),
+                     s->cnt, s->queue, s->d_P + jb);
   }
   s->ctx->launches++;
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(s->ctx, e, "particle pass launch");
   return GASATT_OK;
 }
@@ -2920,7 +2928,9 @@ int sim_prime(gasatt_sim *s) {
 //
 // The field update needs only the current of pass s-1 and the collisions only
 // the particles, so the two run side by side.  Also one sort b -> 1-b.
-int capture_step(gasatt_sim *s, cudaStream_t cs, cudaStream_t side, int q) {
+// early: where a kernel has one other before it, it may start early (but for
+// the first of a graph).  FP64: the field update after the pass only.
+int capture_step(gasatt_sim *s, cudaStream_t cs, cudaStream_t side, int q, bool first, bool early) {
   int rc = GASATT_OK;
   cudaError_t e = cudaSuccess;
   auto mark = [&](int k, cudaStream_t st) {
@@ -2932,9 +2942,9 @@ int capture_step(gasatt_sim *s, cudaStream_t cs, cudaStream_t side, int q) {
     // between and one after the two kernels (the pass's collisions have
     // no kernel of their own)
     mark(0, cs);
-    if (e == cudaSuccess) rc = launch_fdtd(s, cs, q);
+    if (e == cudaSuccess) rc = launch_fdtd(s, cs, q, early && !first);
     mark(1, cs);
-    if (e == cudaSuccess && !rc) rc = launch_pass(s, cs, 0, 1 - q, q, 1 - q);
+    if (e == cudaSuccess && !rc) rc = launch_pass(s, cs, 0, 1 - q, q, 1 - q, early);
     mark(3, cs);
   } else {
     e = cudaEventRecord(s->fork_ev, cs);
@@ -2944,7 +2954,7 @@ int capture_step(gasatt_sim *s, cudaStream_t cs, cudaStream_t side, int q) {
     mark(5, side);
     if (e == cudaSuccess && !rc) e = cudaEventRecord(s->join_ev, side);
     mark(0, cs);
-    if (e == cudaSuccess && !rc) rc = launch_fdtd(s, cs, q);
+    if (e == cudaSuccess && !rc) rc = launch_fdtd(s, cs, q, early && !first);
     mark(1, cs);
     if (e == cudaSuccess && !rc) e = cudaStreamWaitEvent(cs, s->join_ev, 0);
     mark(2, cs);
@@ -2956,13 +2966,13 @@ int capture_step(gasatt_sim *s, cudaStream_t cs, cudaStream_t side, int q) {
 }
 
 // `count` steps, the first of parity q, as one graph; the graph itself is
-// kept where `keep` is given
+// kept where `keep` is given (a child of a batch's graph: no early starts)
 int capture_steps(gasatt_sim *s, cudaStream_t cs, cudaStream_t side, int q, int count, cudaGraphExec_t *exec,
                   cudaGraph_t *keep) {
   cudaGraph_t g;
   GASATT_CUDA(s->ctx, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
   int rc = GASATT_OK;
-  for (int k = 0; k < count && !rc; ++k) rc = capture_step(s, cs, side, (q + k) & 1);
+  for (int k = 0; k < count && !rc; ++k) rc = capture_step(s, cs, side, (q + k) & 1, k == 0, !keep);
   cudaError_t e = cudaStreamEndCapture(cs, &g);
   const bool captured = e == cudaSuccess;
   if (!rc && !captured) rc = cuda_fail(s->ctx, e, "capture step");
@@ -4103,20 +4113,21 @@ int batch_group_setup(gasatt_batch *b, BatchGroup &G) {
 }
 
 // one step of group G (state buffer cur, step parity q) onto the capturing
-// stream cs (side: a second stream for the FP64 collision branch)
+// stream cs (side: a second stream for the FP64 collision branch).  FP32: both
+// kernels start early (but for a graph's first); FP64: neither, since the
+// collisions start with the field update and would find its blocks in their
+// slots (6 cells 115.7 -> 123 us a step, with the spills that the signal costs
+// the pass)
 int batch_group_launch(gasatt_batch *b, BatchGroup &G, cudaStream_t cs, cudaStream_t side, int cur,
-                       int q) {
+                       int q, bool first) {
   gasatt_ctx *ctx = b->ctx;
   const int n = (int)G.sims.size();
   const dim3 fb(32 * tma_warps(G.ph));
   if (G.form == 1) {
-    batch_fdtd_tma_fn<float>(G.ph)<<<G.fdtd_grid, fb, G.fdtd_smem, cs>>>(G.insts[q], G.table, G.nitems,
-                                                                        G.commit, n);
-    GASATT_CUDA(ctx, cudaGetLastError());
-    GASATT_CUDA(ctx, cudaMemsetAsync(G.chunk_next, 0, 8, cs));
-    (G.wide ? k_batch_pass32<true> : k_batch_pass32<false>)<<<G.pass_grid, kBlock, 0, cs>>>(
-        (const BatchCell32 *)G.cells, n, cur, 1 - q, G.chunk_next);
-    GASATT_CUDA(ctx, cudaGetLastError());
+    GASATT_CUDA(ctx, launch_early(!first, batch_fdtd_tma_fn<float>(G.ph), dim3(G.fdtd_grid), fb, G.fdtd_smem, cs,
+                                  G.insts[q], G.table, G.nitems, G.commit, n, G.chunk_next));
+    GASATT_CUDA(ctx, launch_early(true, G.wide ? k_batch_pass32<true> : k_batch_pass32<false>, dim3(G.pass_grid),
+                                  dim3(kBlock), 0, cs, (const BatchCell32 *)G.cells, n, cur, 1 - q, G.chunk_next));
     return GASATT_OK;
   }
   GASATT_CUDA(ctx, cudaEventRecord(b->fork_ev, cs));
@@ -4125,11 +4136,10 @@ int batch_group_launch(gasatt_batch *b, BatchGroup &G, cudaStream_t cs, cudaStre
   k_batch_mcc64<<<G.mcc_grid, kMccBlock, 0, side>>>((const BatchCell64 *)G.cells, n, cur, 1 - q);
   GASATT_CUDA(ctx, cudaGetLastError());
   GASATT_CUDA(ctx, cudaEventRecord(b->join_ev, side));
-  batch_fdtd_tma_fn<double>(G.ph)<<<G.fdtd_grid, fb, G.fdtd_smem, cs>>>(G.insts[q], G.table, G.nitems,
-                                                                       nullptr, n);
+  batch_fdtd_tma_fn<double>(G.ph)<<<G.fdtd_grid, fb, G.fdtd_smem, cs>>>(G.insts[q], G.table, G.nitems, nullptr, n,
+                                                                       G.chunk_next);
   GASATT_CUDA(ctx, cudaGetLastError());
   GASATT_CUDA(ctx, cudaStreamWaitEvent(cs, b->join_ev, 0));
-  GASATT_CUDA(ctx, cudaMemsetAsync(G.chunk_next, 0, 8, cs));
   k_batch_pass64<<<G.pass_grid, kBlock, kWin64Bytes, cs>>>((const BatchCell64 *)G.cells, n, cur, 1 - q, q,
                                                            G.chunk_next);
   GASATT_CUDA(ctx, cudaGetLastError());
@@ -4149,7 +4159,7 @@ int batch_capture_steps(gasatt_batch *b, cudaStream_t cs, cudaStream_t side, int
     cudaGraph_t child = nullptr;
     e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) { rc = cuda_fail(ctx, e, "batch capture"); break; }
-    for (int k = 0; k < count && !rc; ++k) rc = batch_group_launch(b, G, cs, side, bi, (q + k) & 1);
+    for (int k = 0; k < count && !rc; ++k) rc = batch_group_launch(b, G, cs, side, bi, (q + k) & 1, k == 0);
     const cudaError_t e2 = cudaStreamEndCapture(cs, &child);
     if (!rc && e2 != cudaSuccess) rc = cuda_fail(ctx, e2, "batch capture");
     if (!rc) {
