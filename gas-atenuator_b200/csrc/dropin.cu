@@ -404,9 +404,9 @@ __global__ void k_em_scatter(EmState a, EmState b, EmParams g, int64_t N, const 
 // EM4.cu:33-177, then (more steps to come) EM2.cu and EM7.cu of the next step
 template <bool LAST>
 __global__ void __launch_bounds__(kBlock) k_em_push(Species sp, EmState st, EmParams g, int64_t N,
-                                                    const double *__restrict__ Er,
-                                                    const double *__restrict__ Ez,
-                                                    const double *__restrict__ H, double *__restrict__ E) {
+                                                    const double *Er, const double *Ez,
+                                                    const double *H, double *E) {
+  wait_for_previous();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < N;
        o += (int64_t)gridDim.x * blockDim.x) {
     const int of = st.of[o];
@@ -448,6 +448,7 @@ __global__ void __launch_bounds__(kBlock) k_em_push(Species sp, EmState st, EmPa
     st.vx[o] = vx; st.vy[o] = vy; st.vz[o] = vz;
     if (del) st.of[o] = ~of;
   }
+  let_next_start();
 }
 
 // `pairs` H and E updates of the field sub-cycle (EM3_1.cu:2-17, EM3.cu:2-43;
@@ -478,10 +479,10 @@ __host__ __device__ inline int em_tile_cols(int pairs) { return 32 - 2 * pairs -
 __host__ __device__ inline int em_tile_rows(int pairs) { return kEmRows - 2 * pairs - 1; }
 
 __global__ void __launch_bounds__(32 * kEmWarps) k_em_fields(EmFields f, EmFieldParams P,
-                                                             const unsigned long long *__restrict__ Jr,
-                                                             const unsigned long long *__restrict__ Jz,
-                                                             unsigned long long *__restrict__ Jr_next,
-                                                             unsigned long long *__restrict__ Jz_next) {
+                                                             const unsigned long long *Jr,
+                                                             const unsigned long long *Jz,
+                                                             unsigned long long *Jr_next,
+                                                             unsigned long long *Jz_next) {
   constexpr unsigned FULL = 0xFFFFFFFFu;
   constexpr int S = kEmSeg;
   // the rows of a segment its neighbours read: first and last Er, last H
@@ -500,6 +501,7 @@ __global__ void __launch_bounds__(32 * kEmWarps) k_em_fields(EmFields f, EmField
     ezm = col == 0 ? 0.0 : P.dt_eps * (1 / (2 * ri) - id);
   }
   double er[S], ez[S], h[S], jr[S], jz[S];
+  wait_for_previous();
   {
     auto current = [&](const unsigned long long *J, int j) {
       return in && j >= 0 && j < nz ? (double)(long long)J[col + (int64_t)j * nr] * iv : 0.0;
@@ -585,6 +587,7 @@ __global__ void __launch_bounds__(32 * kEmWarps) k_em_fields(EmFields f, EmField
       }
     }
   }
+  let_next_start();                     // (a lane that returned has signalled by that)
 }
 
 // counts[0..3]: the scan at the species' starts and the end; electricmagneticfield6.m:168-188
@@ -1224,13 +1227,15 @@ int gasatt_electricmagneticfield6(gasatt_ctx *ctx, double *e_pos, double *e_vel,
   const bool single = (int64_t)one.x * one.y <= kEmOneLaunch;
   const EmFields there{Er, Ez, Hphi, Er2, Ez2, H2}, back{Er2, Ez2, H2, Er, Ez, Hphi};
   bool away = false;                                   // the fields are in the scratch set
+  // (every kernel of the loop starts while the one before it drains)
   auto launch_fields = [&](int pairs, bool first, bool last, int b) {
     fp.pairs = pairs;
     fp.h_first = first ? (dt / 4) / (mu * delta) : fp.h_mid;      // dt/2 after the -dt/4 that opens the sub-cycle
     fp.h_last = last ? (dt / 4) / (mu * delta) : 0;
-    k_em_fields<<<tiles(pairs), 32 * kEmWarps, 0, ctx->stream>>>(away ? back : there, fp, J[b][0], J[b][1],
-                                                                 J[1 - b][0], J[1 - b][1]);
+    const cudaError_t err = launch_early(true, k_em_fields, tiles(pairs), dim3(32 * kEmWarps), 0, ctx->stream,
+                                         away ? back : there, fp, J[b][0], J[b][1], J[1 - b][0], J[1 - b][1]);
     away = !away;
+    return err;
   };
   if (steps > 0)
     for (int i = 0; i < (N > 0 ? 2 : 4); ++i)
@@ -1254,21 +1259,20 @@ int gasatt_electricmagneticfield6(gasatt_ctx *ctx, double *e_pos, double *e_vel,
     }
     // (an odd number of single launches would leave the fields in the scratch set)
     if (single && !(k == steps - 1 && !away)) {
-      launch_fields(whole, true, true, b);
-      GASATT_LAUNCHED(ctx);
+      GASATT_CUDA(ctx, launch_fields(whole, true, true, b));
+      ctx->launches++;
     } else {
-      launch_fields(ratio, true, false, b);
-      GASATT_LAUNCHED(ctx);
-      launch_fields(ratio, false, true, b);
-      GASATT_LAUNCHED(ctx);
+      GASATT_CUDA(ctx, launch_fields(ratio, true, false, b));
+      GASATT_CUDA(ctx, launch_fields(ratio, false, true, b));
+      ctx->launches += 2;
     }
     if (N > 0) {
       ep.Jr = J[1 - b][0]; ep.Jz = J[1 - b][1];
       if (sorted) E = slots[1 - cur].x;                 // (written in the last step)
       auto push = k == steps - 1 ? k_em_push<true> : k_em_push<false>;
-      push<<<g, kBlock, 0, ctx->stream>>>(sp, slots[cur], ep, N, away ? Er2 : Er, away ? Ez2 : Ez,
-                                          away ? H2 : Hphi, E);
-      GASATT_LAUNCHED(ctx);
+      GASATT_CUDA(ctx, launch_early(true, push, dim3(g), dim3(kBlock), 0, ctx->stream, sp, slots[cur], ep, N,
+                                    away ? Er2 : Er, away ? Ez2 : Ez, away ? H2 : Hphi, E));
+      ctx->launches++;
     }
   }
   int64_t outs[3] = {0, 0, 0};
