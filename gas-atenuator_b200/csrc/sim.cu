@@ -2914,7 +2914,10 @@ int sim_prime(gasatt_sim *s) {
   };
   const bool odd = s->host_step & 1;
   if (s->form == 0 && !odd) GASATT_CUDA(s->ctx, catch_up());
-  SIM_TRY(launch_pass(s, st, 1, 0, 1, fcur(s)));   // (a half drift reads no field)
+  // The current goes to the buffer that the next step reads: buffer host_step & 1,
+  // which the last field update left empty (both are empty in a new run).  (A half drift
+  // reads no field.)
+  SIM_TRY(launch_pass(s, st, 1, (int)odd, 1, fcur(s)));
   if (s->form == 0 && odd) GASATT_CUDA(s->ctx, catch_up());
   s->primed = true;
   return GASATT_OK;
