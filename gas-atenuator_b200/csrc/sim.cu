@@ -1919,6 +1919,9 @@ __device__ __forceinline__ void commit_pass32(SimCounters *cnt) {
   cnt->step = ns;
 }
 
+// the same before a pass that no field update precedes (sim_prime)
+__global__ void k_commit32(SimCounters *cnt) { commit_pass32(cnt); }
+
 // The field sub-cycle of one step for fdtd_ratio 1: one block per patch of
 // shape K (fdtd_tma.cuh).
 template <typename T, int K>
@@ -2478,6 +2481,7 @@ struct gasatt_sim {
   FieldQuads quads{};             // FP32 form: gather quads, written with the fields
   bool mcc_pending = false;       // the last pass's collisions are not applied yet
   bool batch_pass = false;        // FP64: the last pass was a batch's (clear_after_batch)
+  bool uncommitted = false;       // FP32: gasatt_sim_run_host's last pass, which no field update has committed
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;   // graph capture fork/join
   bool timing = false;
   // field update start/end, particle pass start/end, collision kernel start/end
@@ -2773,6 +2777,7 @@ int sim_reset(gasatt_sim *s, int64_t n) {
   s->primed = false;
   s->mcc_pending = false;
   s->batch_pass = false;
+  s->uncommitted = false;
   s->since_sort = 0;
   return GASATT_OK;
 }
@@ -2914,6 +2919,13 @@ int sim_prime(gasatt_sim *s) {
   };
   const bool odd = s->host_step & 1;
   if (s->form == 0 && !odd) GASATT_CUDA(s->ctx, catch_up());
+  // FP32: as a step of its own, else it would find the chunks of the last pass
+  // handed out and its electrons marked as pushed
+  if (s->form == 1 && s->uncommitted) {
+    k_commit32<<<1, 1, 0, st>>>(s->cnt);
+    GASATT_LAUNCHED(s->ctx);
+  }
+  s->uncommitted = false;
   // The current goes to the buffer that the next step reads: buffer host_step & 1,
   // which the last field update left empty (both are empty in a new run).  (A half drift
   // reads no field.)
@@ -3922,6 +3934,7 @@ int gasatt_sim_run_host(gasatt_sim *s, double *pos, double *vel, int64_t *n_io, 
   s->primed = false;
   s->mcc_pending = false;
   s->batch_pass = false;
+  s->uncommitted = false;
   SIM_TRY(restart_steps(s, st));             // the prologue deposits into buffer 0
   s->since_sort = s->cfg.sort_period;       // sort the fresh population first
   SIM_TRY(gasatt_sim_step(s, nsteps - 1));
@@ -3934,6 +3947,7 @@ int gasatt_sim_run_host(gasatt_sim *s, double *pos, double *vel, int64_t *n_io, 
   SIM_TRY(gasatt_sim_sort(s));               // compacts away the dead
   s->host_step++;
   s->primed = false;
+  s->uncommitted = true;
   GASATT_CUDA(ctx, cudaMemcpyAsync(s->h_cnt, s->cnt, sizeof(SimCounters), cudaMemcpyDeviceToHost, st));
   GASATT_CUDA(ctx, cudaStreamSynchronize(st));
   const int64_t nout = (int64_t)s->h_cnt->n_total;

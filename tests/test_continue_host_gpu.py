@@ -61,3 +61,21 @@ def test_fp64(nsteps, step):
     assert np.abs(want[-1]).max() > 0
     for g, w in zip(got, want):
         np.testing.assert_array_equal(g, w)
+
+
+@pytest.mark.parametrize("step", STEPS)
+@pytest.mark.parametrize("nsteps", [1, 4, 5])
+def test_fp32(nsteps, step):
+    """The stochastic rounding draws differ, so the momenta differ by float
+    roundings (6e-8 of c a step at most, so 1e-5 of 0.17 c in 14 steps with
+    room) and the positions by what these move an electron: far less than the
+    half drift of 0.05 cells that a missing prologue costs."""
+    got, want = after_host_call(_lib.FP32_SPLIT, nsteps, step)
+    np.testing.assert_array_equal(got[0], want[0])
+    for k in (1, 2):
+        assert np.abs(got[k] - want[k]).max() < 1e-4 * D
+    for k in (3, 4, 5):
+        assert np.abs(got[k] - want[k]).max() < 1e-5 * 0.17 * C
+    for g, w in zip(got[6:], want[6:]):
+        assert np.abs(w).max() > 0
+        assert np.abs(g - w).max() < 1e-4 * np.abs(w).max()
