@@ -470,6 +470,7 @@ struct EmFields { const double *Er, *Ez, *H; double *oEr, *oEz, *oH; };
 
 struct EmFieldParams {
   int nr, nz, pairs;
+  int tiles_x;                            // tiles across (one block per tile, a row of tiles after the other)
   double delta, PHIp, inv_scale, dt_eps, dt_eps_dz, axis;
   double h_first, h_mid, h_last;          // h / (mu delta)
   bool endcopy, jsign, rshift;
@@ -490,8 +491,9 @@ __global__ void __launch_bounds__(32 * kEmWarps) k_em_fields(EmFields f, EmField
   __shared__ double s_first[2][kEmWarps][32], s_last[2][kEmWarps][32], s_h[kEmWarps][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nr = P.nr, nz = P.nz;
-  const int col = (int)blockIdx.x * em_tile_cols(P.pairs) - P.pairs + lane;
-  const int y0 = (int)blockIdx.y * em_tile_rows(P.pairs) - P.pairs + w * S;     // the segment's first row
+  const int ty = (int)blockIdx.x / P.tiles_x, tx = (int)blockIdx.x - ty * P.tiles_x;
+  const int col = tx * em_tile_cols(P.pairs) - P.pairs + lane;
+  const int y0 = ty * em_tile_rows(P.pairs) - P.pairs + w * S;     // the segment's first row
   const bool in = col >= 0 && col < nr;
   double iv = 0, ezp = 0, ezm = 0;        // coefficients of EM3.cu; Ez at column n_r stays as it is
   if (in) {
@@ -1220,19 +1222,18 @@ int gasatt_electricmagneticfield6(gasatt_ctx *ctx, double *e_pos, double *e_vel,
   // with one launch / two: 100 x 500 cells 1069 / 1188 us, 200 x 1000 cells
   // 1956 / 1916, 400 x 2000 cells 2837 / 2574.
   const int whole = 2 * ratio;
-  auto tiles = [&](int pairs) {
-    return dim3((n_r + em_tile_cols(pairs)) / em_tile_cols(pairs), (n_z + em_tile_rows(pairs)) / em_tile_rows(pairs));
-  };
-  const dim3 one = tiles(whole);
-  const bool single = (int64_t)one.x * one.y <= kEmOneLaunch;
+  auto tiles_x = [&](int pairs) { return (n_r + em_tile_cols(pairs)) / em_tile_cols(pairs); };
+  auto tiles = [&](int pairs) { return (int64_t)tiles_x(pairs) * ((n_z + em_tile_rows(pairs)) / em_tile_rows(pairs)); };
+  const bool single = tiles(whole) <= kEmOneLaunch;
   const EmFields there{Er, Ez, Hphi, Er2, Ez2, H2}, back{Er2, Ez2, H2, Er, Ez, Hphi};
   bool away = false;                                   // the fields are in the scratch set
   // (every kernel of the loop starts while the one before it drains)
   auto launch_fields = [&](int pairs, bool first, bool last, int b) {
     fp.pairs = pairs;
+    fp.tiles_x = tiles_x(pairs);
     fp.h_first = first ? (dt / 4) / (mu * delta) : fp.h_mid;      // dt/2 after the -dt/4 that opens the sub-cycle
     fp.h_last = last ? (dt / 4) / (mu * delta) : 0;
-    const cudaError_t err = launch_early(true, k_em_fields, tiles(pairs), dim3(32 * kEmWarps), 0, ctx->stream,
+    const cudaError_t err = launch_early(true, k_em_fields, dim3((unsigned)tiles(pairs)), dim3(32 * kEmWarps), 0, ctx->stream,
                                          away ? back : there, fp, J[b][0], J[b][1], J[1 - b][0], J[1 - b][1]);
     away = !away;
     return err;
