@@ -114,7 +114,7 @@ class Sim:
 
     def set_gas_density(self, density):
         """Per-cell N2 density [m^-3] of shape (n_r, n_z) for the collisions, or
-        None to go back to the uniform cfg.gas_density.  Step graphs are rebuilt;
+        None to go back to the uniform cfg.gas_density.  The step graphs take the new values;
         a Batch must be created after this call."""
         if density is None:
             check(self.ctx.handle, lib.gasatt_sim_set_gas_density(self.h, None, 0))

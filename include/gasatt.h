@@ -358,7 +358,7 @@ int gasatt_sim_read_ions(gasatt_sim *sim, double *r, double *z, double *ur, doub
  * collides against the density of the cell it ends the step in, and the
  * null-collision bound becomes max(density) x max(sigma_tot v).  Values must be
  * finite and >= 0 (GASATT_E_ARG otherwise).  Collisions still queued are
- * applied first, with the old density; the step graphs are rebuilt, so a
+ * applied first, with the old density; the step graphs take the new values, so a
  * batch (gasatt_batch_create) holding this simulation must be created after
  * the call.  on_device: 1 = device pointer, 0 = host pointer. */
 int gasatt_sim_set_gas_density(gasatt_sim *sim, const double *density, int on_device);
@@ -368,7 +368,7 @@ int gasatt_sim_set_gas_density(gasatt_sim *sim, const double *density, int on_de
  * the newborn ion's Maxwellian (electron_transport.cu:202-204).  An ion born
  * in a cell gets velocity components of spread sqrt(kb T / m_ion) of that
  * cell.  Values finite and >= 0.  Collisions still queued are applied first;
- * the step graphs are rebuilt, so create a batch after this call. */
+ * the step graphs take the new values, but a batch has to be created after this call. */
 int gasatt_sim_set_gas_temperature(gasatt_sim *sim, const double *temperature, int on_device);
 int gasatt_sim_read(gasatt_sim *sim, double *r, double *z,
                     double *ur, double *ut, double *uz, uint64_t *id,
