@@ -2716,18 +2716,23 @@ int launch_sort(gasatt_sim *s, cudaStream_t st, int from) {
   return GASATT_OK;
 }
 
-void drop_graphs(gasatt_sim *s) {
-  for (int i = 0; i < 2; ++i) {
-    if (s->g_steps[i]) cudaGraphExecDestroy(s->g_steps[i]);
-    s->g_steps[i] = nullptr;
-    if (s->gr_steps[i]) cudaGraphDestroy(s->gr_steps[i]);
-    s->gr_steps[i] = nullptr;
+void drop_step_graphs(gasatt_sim *s) {
+  for (int i = 0; i < 2; ++i)
     for (int q = 0; q < 2; ++q) {
       if (s->g_step[i][q]) cudaGraphExecDestroy(s->g_step[i][q]);
       s->g_step[i][q] = nullptr;
       if (s->gr_step[i][q]) cudaGraphDestroy(s->gr_step[i][q]);
       s->gr_step[i][q] = nullptr;
     }
+}
+
+void drop_graphs(gasatt_sim *s) {
+  drop_step_graphs(s);
+  for (int i = 0; i < 2; ++i) {
+    if (s->g_steps[i]) cudaGraphExecDestroy(s->g_steps[i]);
+    s->g_steps[i] = nullptr;
+    if (s->gr_steps[i]) cudaGraphDestroy(s->gr_steps[i]);
+    s->gr_steps[i] = nullptr;
     if (s->g_sort[i]) cudaGraphExecDestroy(s->g_sort[i]);
     s->g_sort[i] = nullptr;
     if (s->gr_sort[i]) cudaGraphDestroy(s->gr_sort[i]);
@@ -3060,6 +3065,8 @@ int renew_params(gasatt_sim *s) {
   return GASATT_OK;
 }
 
+// the graphs that there are not yet (with the timing on, those of one step
+// hold its events, and those of ten are not used)
 int build_graphs(gasatt_sim *s) {
   // the field update goes on a higher-priority stream than the collision
   // branch, so its blocks are placed first when both are ready
@@ -3075,8 +3082,9 @@ int build_graphs(gasatt_sim *s) {
     cudaGraph_t g;
     s->cur = b;
     for (int q = 0; q < 2 && !rc; ++q) rc = capture_steps(s, cs, side, q, 1, &s->g_step[b][q], &s->gr_step[b][q]);
-    if (!rc && !s->timing) rc = capture_steps(s, cs, side, 0, kGraphSteps, &s->g_steps[b], &s->gr_steps[b]);
+    if (!rc && !s->timing && !s->g_steps[b]) rc = capture_steps(s, cs, side, 0, kGraphSteps, &s->g_steps[b], &s->gr_steps[b]);
     if (rc) break;
+    if (s->g_sort[b]) continue;
     GASATT_CUDA(s->ctx, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     rc = launch_sort(s, cs, b);
     cudaError_t e = cudaStreamEndCapture(cs, &g);
@@ -3797,7 +3805,7 @@ int gasatt_sim_step(gasatt_sim *s, int nsteps) {
     if (s->cfg.sort_period > 0 && s->since_sort >= s->cfg.sort_period) SIM_TRY(gasatt_sim_sort(s));
     // several steps by one launch: from an even step, up to the next sort and ion push
     int many = 1;
-    if (s->g_steps[s->cur] && !(s->host_step & 1) && nsteps - k >= kGraphSteps && steps_fit(s, s->cfg.sort_period))
+    if (!s->timing && !(s->host_step & 1) && nsteps - k >= kGraphSteps && steps_fit(s, s->cfg.sort_period))
       many = kGraphSteps;
     GASATT_CUDA(ctx, cudaGraphLaunch(many > 1 ? s->g_steps[s->cur] : s->g_step[s->cur][s->host_step & 1], st));
     ctx->launches += many * per_step;
@@ -3880,7 +3888,7 @@ int gasatt_sim_enable_timing(gasatt_sim *s, int enable) {
   if ((bool)enable == s->timing) return GASATT_OK;
   GASATT_CUDA(s->ctx, cudaSetDevice(s->ctx->device));
   GASATT_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
-  drop_graphs(s);
+  drop_step_graphs(s);
   s->timing = enable != 0;
   return build_graphs(s);
 }

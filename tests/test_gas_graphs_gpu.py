@@ -1,5 +1,6 @@
 """A gas map set between steps reaches every step graph (of one step and of ten, both
-state buffers) and costs less than building them."""
+state buffers) and costs less than building them; only the graphs of one step are built
+again when the timing is turned on or off."""
 import statistics
 import time
 
@@ -28,6 +29,16 @@ def state(sim):
     o, p = np.argsort(st["id"][a]), np.argsort(i["id"])
     return [st[k][a][o] for k in ("id", "r", "z", "ur", "ut", "uz")] + [i["ur"][p]] + list(sim.fields()) + \
         list(sim.current()) + [np.array([d[k] for k in ("n_alive", "n_ionizations", "n_elastic", "n_null")])]
+
+
+def median(sim, f):
+    t = []
+    for _ in range(15):
+        sim.synchronize()
+        t0 = time.perf_counter()
+        f()
+        t.append(time.perf_counter() - t0)
+    return statistics.median(t)
 
 
 @pytest.mark.parametrize("precision", [_lib.FP64, _lib.FP32_SPLIT])
@@ -60,16 +71,25 @@ def test_setting_a_map_does_not_build_graphs(precision):
     fraction of that."""
     sim = make(precision)
     n = np.full((NR, NZ), sim.cfg.gas_density)
-
-    def median(f):
-        t = []
-        for _ in range(15):
-            sim.synchronize()
-            t0 = time.perf_counter()
-            f()
-            t.append(time.perf_counter() - t0)
-        return statistics.median(t)
-
-    build = median(lambda: [lib.gasatt_sim_enable_timing(sim.h, on) for on in (1, 0)])
-    assert median(lambda: sim.set_gas_density(n)) < 0.4 * build
+    build = median(sim, lambda: [lib.gasatt_sim_enable_timing(sim.h, on) for on in (1, 0)])
+    assert median(sim, lambda: sim.set_gas_density(n)) < 0.4 * build
     sim.close()
+
+
+def test_timing_on_and_off_builds_the_graphs_of_one_step():
+    """The FP64 form's graphs of one step cost about twice the FP32 form's (their fork); its
+    graphs of ten steps would cost as much again."""
+    t = []
+    for precision in (_lib.FP64, _lib.FP32_SPLIT):
+        sim = make(precision, 20)
+        t.append(median(sim, lambda: [lib.gasatt_sim_enable_timing(sim.h, on) for on in (1, 0)]))
+        one = make(precision, 20)
+        for k in range(3):                # with the timing on, off and on again the steps are the same
+            lib.gasatt_sim_enable_timing(sim.h, (k + 1) & 1)
+            sim.step(12)
+            one.step(12)
+        for a, b in zip(state(sim), state(one)):
+            np.testing.assert_array_equal(a, b)
+        sim.close()
+        one.close()
+    assert t[0] < 2.3 * t[1]
