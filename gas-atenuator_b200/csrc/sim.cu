@@ -4074,6 +4074,7 @@ struct gasatt_batch {
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   cudaGraphExec_t g[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [state buffer][parity]
   cudaGraphExec_t g_steps[2] = {nullptr, nullptr};  // kGraphSteps steps from parity 0 on [state buffer]
+  int64_t lone[2] = {0, 0}, worth = 0;   // steps taken without g_steps that it fits, and how many of them it is worth
   cudaGraphExec_t g_sort[2] = {nullptr, nullptr};   // every cell's sort side by side [state buffer]
 };
 
@@ -4268,14 +4269,23 @@ int batch_capture_steps(gasatt_batch *b, cudaStream_t cs, cudaStream_t side, int
   return rc;
 }
 
-int batch_build_graphs(gasatt_batch *b) {
-  gasatt_ctx *ctx = b->ctx;
+// two capturing streams for the time of `build`
+template <typename F>
+int with_capture_streams(gasatt_ctx *ctx, F build) {
   cudaStream_t cs, side;
   GASATT_CUDA(ctx, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) {
     cudaStreamDestroy(cs);
     return fail(ctx, GASATT_E_CUDA, "batch: stream");
   }
+  const int rc = build(cs, side);
+  cudaStreamDestroy(side);
+  cudaStreamDestroy(cs);
+  return rc;
+}
+
+int batch_build_graphs(gasatt_batch *b, cudaStream_t cs, cudaStream_t side) {
+  gasatt_ctx *ctx = b->ctx;
   int rc = GASATT_OK;
   for (int bi = 0; bi < 2 && !rc; ++bi) {
     cudaGraph_t g = nullptr;
@@ -4292,13 +4302,28 @@ int batch_build_graphs(gasatt_batch *b) {
     }
     cudaGraphDestroy(g);
   }
-  for (int bi = 0; bi < 2 && !rc; ++bi) {
+  for (int bi = 0; bi < 2 && !rc; ++bi)
     for (int q = 0; q < 2 && !rc; ++q) rc = batch_capture_steps(b, cs, side, bi, q, 1, &b->g[bi][q]);
-    if (!rc) rc = batch_capture_steps(b, cs, side, bi, 0, kGraphSteps, &b->g_steps[bi]);
-  }
-  cudaStreamDestroy(side);
-  cudaStreamDestroy(cs);
+  // A graph of ten steps gives 4 to 6 us a step and costs, to build and to
+  // destroy, 0.2 ms for chains of kernels and 1.2 ms more for each branch with the
+  // FP64 form's forks (0.12 ms a fork): it is built once as many steps were taken without
+  // it.  Both built at once, the creation of a batch took 4.2 ms (FP64) and 2.0 ms
+  // (FP32); now 2.2 ms and 1.8 ms.
+  b->worth = 40;
+  for (const BatchGroup &G : b->groups) b->worth += G.form == 0 ? 320 : 0;
+  for (const gasatt_sim *s : b->singles) b->worth += s->form == 0 ? 320 : 0;
   return rc;
+}
+
+// whether the graph of ten steps is there, or worth building now (and built)
+int batch_steps_ready(gasatt_batch *b, int cur, bool *ready) {
+  if (!b->g_steps[cur] && b->lone[cur] >= b->worth)
+    SIM_TRY(with_capture_streams(b->ctx, [&](cudaStream_t cs, cudaStream_t side) {
+      return batch_capture_steps(b, cs, side, cur, 0, kGraphSteps, &b->g_steps[cur]);
+    }));
+  *ready = b->g_steps[cur] != nullptr;
+  if (!*ready) b->lone[cur] += 2;          // (asked at every other step)
+  return GASATT_OK;
 }
 
 // flush_collisions for every cell of the batch (before its sort): a group
@@ -4380,7 +4405,7 @@ int gasatt_batch_create(gasatt_ctx *ctx, gasatt_sim *const *sims, int n, int sor
       cudaEventCreateWithFlags(&b->join_ev, cudaEventDisableTiming) != cudaSuccess)
     rc = fail(ctx, GASATT_E_CUDA, "batch: event");
   for (size_t i = 0; i < b->groups.size() && !rc; ++i) rc = batch_group_setup(b, b->groups[i]);
-  if (!rc) rc = batch_build_graphs(b);
+  if (!rc) rc = with_capture_streams(ctx, [&](cudaStream_t cs, cudaStream_t side) { return batch_build_graphs(b, cs, side); });
   if (rc) {
     gasatt_batch_destroy(b);
     return rc;
@@ -4425,6 +4450,11 @@ int gasatt_batch_step(gasatt_batch *b, int nsteps) {
       if (!steps_fit(s, b->sort_period)) many = 1;
     }
     if (!lockstep) many = 1;
+    if (many > 1) {
+      bool ready;
+      SIM_TRY(batch_steps_ready(b, s0->cur, &ready));
+      if (!ready) many = 1;
+    }
     if (lockstep) {
       GASATT_CUDA(ctx, cudaGraphLaunch(many > 1 ? b->g_steps[s0->cur] : b->g[s0->cur][s0->host_step & 1], st));
       for (const BatchGroup &G : b->groups) ctx->launches += many * (G.form == 0 ? 4 : 2);
