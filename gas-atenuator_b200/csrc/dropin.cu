@@ -320,6 +320,18 @@ __device__ __forceinline__ void em_halfdrift(const EmParams &g, double &x, doubl
   z = Z;
 }
 
+// k b rounded to a whole number.  In one FMA where it is known to be at most
+// 2^50 (fast) - but for velocities or positions that are not finite (on the axis atan(y/x) is
+// none) or far beyond the speed of light: the sum has then left the binade of
+// 1.5 2^52, and the conversion's rules hold.
+__device__ __forceinline__ long long em_fixed(bool fast, double k, double b) {
+  if (fast) {
+    const double v = fma(k, b, 6755399441055744.0);
+    if ((__double2hiint(v) >> 20) == 0x433) return __double_as_longlong(v) - 0x4338000000000000LL;
+  }
+  return __double2ll_rn(k * b);
+}
+
 // EM7.cu:51-202: q FN v w of a particle at (r, z) into its four nodes, in fixed point
 __device__ __forceinline__ void em_deposit(const EmParams &g, double r, double z, double vr, double vz,
                                            double q) {
@@ -329,14 +341,7 @@ __device__ __forceinline__ void em_deposit(const EmParams &g, double r, double z
   for (int n = 0; n < 4; ++n) {
     const int64_t a = (n & 1 ? R.hi : R.lo) + (int64_t)(n & 2 ? Z.hi : Z.lo) * g.nr;
     const double b = (n & 1 ? R.w : 1 - R.w) * (n & 2 ? Z.w : 1 - Z.w);
-    long long vr_fx, vz_fx;
-    if (g.fast_fx) {
-      vr_fx = __double_as_longlong(fma(kr, b, 6755399441055744.0)) - 0x4338000000000000LL;
-      vz_fx = __double_as_longlong(fma(kz, b, 6755399441055744.0)) - 0x4338000000000000LL;
-    } else {
-      vr_fx = __double2ll_rn(kr * b);
-      vz_fx = __double2ll_rn(kz * b);
-    }
+    const long long vr_fx = em_fixed(g.fast_fx, kr, b), vz_fx = em_fixed(g.fast_fx, kz, b);
     if (vr_fx) atomicAdd(g.Jr + a, (unsigned long long)vr_fx);
     if (vz_fx) atomicAdd(g.Jz + a, (unsigned long long)vz_fx);
   }

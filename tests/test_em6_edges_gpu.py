@@ -1,4 +1,5 @@
-"""electricmagneticfield6 at the edges of what it takes: grids of millions of rows."""
+"""electricmagneticfield6 at the edges of what it takes: grids of millions of rows, currents
+that are not finite."""
 import numpy as np
 import pytest
 import torch
@@ -31,3 +32,25 @@ def test_more_rows_of_tiles_than_a_grid_dimension_holds(nr, nz):
         # 1e-12 of the largest value, as the drop-in's own test; a coordinate of 3.5 million cells holds its
         # place in a cell, and so the weights of the gather, to 3.5e6 x 2^-52 = 8e-10 only
         close(g.cpu().numpy(), w, 1e-12 if k[-3:] == "pos" else 1e-8, k)
+
+
+@pytest.mark.parametrize("r,v", [(0.0, (0, 0, 3e7)), (2e-4, (0, 0, np.nan)), (2e-4, (0, 0, np.inf)), (2e-4, (0, 0, 1e10))])
+@pytest.mark.parametrize("flags", [0, _lib.FAITHFUL])
+def test_currents_that_are_not_finite(r, v, flags):
+    """One electron moves, on the axis (whose azimuth atan(y / x) is none) or with an impossible
+    velocity, among 4094 or 4095 that rest: its current is rounded by the same rules on both sides of
+    the 4096 particles from which one FMA rounds (both in units of the same power of two)."""
+    nr, nz, d = 12, 20, 1e-4
+    out = []
+    for n in (4095, 4096):
+        pos = np.tile([3.3e-4, 0.05, 1e-3], (n, 1))
+        vel = np.zeros((n, 3))
+        pos[7], vel[7] = (r, 0.05, 4.4e-4), v
+        no = np.zeros((0, 3))
+        f = [np.zeros(s, order="F") for s in ((nr, nz + 1), (nr + 1, nz), (nr, nz))]
+        out.append(run((pos, vel, no, no, no, no, *f, d, 1e-14, nr * d, nz * d, 0.1, 1e4, 5), flags | _lib.POS_IN_CYL))
+    for k in (6, 7, 8):
+        a, b = (o[k].cpu().numpy() for o in out)
+        np.testing.assert_array_equal(a, b)
+    if np.isfinite(v[2]):
+        assert np.abs(a).max() > 0
