@@ -295,6 +295,7 @@ __device__ __forceinline__ void em_halfdrift(const EmParams &g, double &x, doubl
       s = r > 0 ? Y * ir : 0.0;
     }
     if (g.wrap) {
+      const double s0 = s;
       for (int it = 0; s < 0 && it < (1 << 20); ++it) {
         const double k = c * g.cP - s * g.sP;
         s = c * g.sP + s * g.cP;
@@ -310,6 +311,13 @@ __device__ __forceinline__ void em_halfdrift(const EmParams &g, double &x, doubl
         const double w = vx * g.cP + vy * g.sP;
         vy = -vx * g.sP + vy * g.cP;
         vx = w;
+      }
+      // the turns' roundings off the length of (c, s), which would become the radius
+      // (thousands of turns into a narrow wedge: 1e-13)
+      if (s != s0) {
+        const double k = fma(-0.5, fma(c, c, s * s), 1.5);
+        c *= k;
+        s *= k;
       }
     }
   }

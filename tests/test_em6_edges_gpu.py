@@ -1,5 +1,7 @@
 """electricmagneticfield6 at the edges of what it takes: grids of millions of rows, currents
-that are not finite."""
+that are not finite, many turns into a narrow wedge."""
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -54,3 +56,22 @@ def test_currents_that_are_not_finite(r, v, flags):
         np.testing.assert_array_equal(a, b)
     if np.isfinite(v[2]):
         assert np.abs(a).max() > 0
+
+
+@pytest.mark.parametrize("flags", [0, _lib.FAITHFUL])
+@pytest.mark.parametrize("PHIp", [7e-4, 1e-3, 2.9e-3, 0.1, math.pi / 2])
+def test_turns_into_the_wedge_keep_the_radius(PHIp, flags):
+    """Electrons at rest at any azimuth, turned into the wedge up to 4500 times.  Two half drifts
+    round the radius, its inverse, the sine, the cosine, their length and the coordinates: some
+    twelve roundings of 1.1e-16 with the test's own."""
+    rng = np.random.default_rng(5)
+    nr, nz, d, n = 12, 20, 1e-4, 2000
+    rr, phi = rng.uniform(0.1, 0.9, n) * nr * d, rng.uniform(-math.pi, math.pi, n)
+    pos = np.stack([rr * np.cos(phi), rr * np.sin(phi), np.full(n, 1e-3)], 1)
+    no = np.zeros((0, 3))
+    f = [np.zeros(s, order="F") for s in ((nr, nz + 1), (nr + 1, nz), (nr, nz))]
+    got = run((pos, np.zeros((n, 3)), no, no, no, no, *f, d, 1e-13, nr * d, nz * d, PHIp, 1e4, 5), flags)[0].cpu().numpy()
+    was, now = (np.hypot(*p[:, :2].T.astype(np.longdouble)) for p in (pos, got))
+    assert np.abs(now / was - 1).max() < 2e-15
+    az = np.arctan2(got[:, 1], got[:, 0])
+    assert az.min() > -1e-12 and az.max() < PHIp + 1e-12
