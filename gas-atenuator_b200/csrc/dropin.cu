@@ -46,11 +46,12 @@ __device__ double d_loglog(const double *x, int sx, const double *y, int sy, int
 }
 
 // x^e; the excitation table's exponents are 1, 3 and 3/4, whose powers need no
-// logarithm (200,000 energies: 53 us with pow throughout, 18 us so)
+// logarithm (200,000 energies: 53 us with pow throughout, 18 us so).  Below 0 sqrt
+// is no number, but pow(-infinity, 3/4), of an energy of 0, is infinite.
 __device__ __forceinline__ double pow_table(double x, double e) {
   if (e == 1) return x;
   if (e == 3) return x * x * x;
-  if (e == 0.75) {
+  if (e == 0.75 && x >= 0) {
     const double r = sqrt(x);
     return r * sqrt(r);
   }
