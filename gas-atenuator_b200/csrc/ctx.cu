@@ -12,6 +12,7 @@ int fail(gasatt_ctx *ctx, int code, const std::string &msg) {
 
 int cuda_fail(gasatt_ctx *ctx, cudaError_t e, const char *what) {
   std::string m = std::string(what) + ": " + cudaGetErrorString(e);
+  cudaGetLastError();              // returned here, not left for the next call's check
   return fail(ctx, GASATT_E_CUDA, m);
 }
 
@@ -21,6 +22,7 @@ int scratch(gasatt_ctx *ctx, size_t bytes, void **ptr) {
       GASATT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
       GASATT_CUDA(ctx, cudaFree(ctx->scratch));
       ctx->scratch = nullptr;
+      ctx->scratch_bytes = 0;      // (the allocation may fail)
     }
     size_t nb = bytes + bytes / 4 + 4096;
     GASATT_CUDA(ctx, cudaMalloc(&ctx->scratch, nb));
