@@ -1372,21 +1372,23 @@ __device__ __forceinline__ bool push32(const SimParams &P, const Fields<float> &
   half_shift(iz, fz, az, wz);
   // the field loads go out first, their latency hidden behind Philox: one
   // packed quad per field (corners already clamped at the edges), or the
-  // same four corners from the fields themselves (the same floats)
+  // same four corners from the fields themselves (the same floats).  Ordinary
+  // loads: the field update may still be writing when this kernel starts, so the
+  // arrays are not read-only for its whole life, as __ldg requires.
   float4 a4, b4, c4;
   if (P.qEr) {
-    a4 = __ldg(P.qEr + ((ar + 1) + iz * (P.nr + 1)));
-    b4 = __ldg(P.qEz + (ir + (az + 1) * P.nr));
-    c4 = __ldg(P.qH + ((ar + 1) + (az + 1) * (P.nr + 1)));
+    a4 = P.qEr[(ar + 1) + iz * (P.nr + 1)];
+    b4 = P.qEz[ir + (az + 1) * P.nr];
+    c4 = P.qH[(ar + 1) + (az + 1) * (P.nr + 1)];
   } else {
     const int c0 = max(ar, 0), c1 = min(ar + 1, P.nr - 1);
     const int ra = max(az, 0), rb = min(az + 1, P.nz - 1);
     const float *e0 = F.Er + iz * P.ldf, *e1 = e0 + P.ldf;
-    a4 = make_float4(__ldg(e0 + c0), __ldg(e0 + c1), __ldg(e1 + c0), __ldg(e1 + c1));
+    a4 = make_float4(e0[c0], e0[c1], e1[c0], e1[c1]);
     const float *z0 = F.Ez + ra * P.ldf + ir, *z1 = F.Ez + rb * P.ldf + ir;
-    b4 = make_float4(__ldg(z0), __ldg(z0 + 1), __ldg(z1), __ldg(z1 + 1));
+    b4 = make_float4(z0[0], z0[1], z1[0], z1[1]);
     const float *h0 = F.H + ra * P.ldf, *h1 = F.H + rb * P.ldf;
-    c4 = make_float4(__ldg(h0 + c0), __ldg(h0 + c1), __ldg(h1 + c0), __ldg(h1 + c1));
+    c4 = make_float4(h0[c0], h0[c1], h1[c0], h1[c1]);
   }
   philox4x32_10(c, P.pk);
   // bilinear mixes from the quads' corners (c0,r0), (c1,r0), (c0,r1), (c1,r1)
