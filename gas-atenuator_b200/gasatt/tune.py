@@ -14,7 +14,8 @@ update's arithmetic is the same for every patch):
                   patches for the blocks to share;
   pass_chunk      particles per chunk of the FP32 particle pass (its deposit
                   window's span against the number of chunks for the blocks
-                  to balance);
+                  to balance; 0: chosen every step by the population, which
+                  no fixed chunk follows);
   gather          where the FP32 push reads E and H: packed 2 x 2 quads the
                   field update writes beside the fields (fewer loads per
                   electron, 48 more bytes written per cell), or the fields.
@@ -33,7 +34,7 @@ from .sim import Sim
 
 DEFAULT_SORT_PERIODS = (10, 20, 30, 40, 60)
 DEFAULT_TILE_ROWS = (12, 16, 20)
-DEFAULT_CHUNKS = (1024, 1280, 1536, 1792)
+DEFAULT_CHUNKS = (0, 1024, 1280, 1536, 1792)     # 0: by the population, every step
 
 
 def time_steps(sim, steps, warmup=5):
