@@ -10,16 +10,21 @@ DATA = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
                     "n2_tables.npz")
 
 
-_packaged = {}      # the packaged file's arrays, read once per process
+_packaged = (None, None)     # the packaged file as last read: its stamp, its arrays
 
 
 def _raw(path):
+    global _packaged
     if path != DATA:
         return np.load(path)
-    if not _packaged:
+    st = os.stat(DATA)
+    stamp = (DATA, st.st_ino, st.st_size, st.st_mtime_ns)
+    held, arrays = _packaged
+    if held != stamp:
         with np.load(DATA) as z:
-            _packaged.update({k: z[k] for k in z.files})
-    return _packaged
+            arrays = {k: z[k] for k in z.files}
+        _packaged = (stamp, arrays)
+    return arrays
 
 
 class N2Tables:
