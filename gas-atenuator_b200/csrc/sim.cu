@@ -1981,11 +1981,11 @@ __global__ void __launch_bounds__(32 * kFdtdRows, 3) k_sim_fdtd(Fields<T> in, Fi
                                                   SimCounters *cnt, ExtraCurrent ion,
                                                   FieldQuads quads) {
   wait_for_previous();
-  let_next_start();
   if (cnt && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0)
     commit_pass32(cnt);
   fdtd_tiled<T>(in.Er, in.Ez, in.H, out.Er, out.Ez, out.H, Jr, Jz, Jr_next, Jz_next, nr, nz, ldf, ldj,
                 c, invV, mu, dt, R, flags, ion, quads);
+  let_next_start();
 }
 
 // ---------------------------------------------------------- load/read
