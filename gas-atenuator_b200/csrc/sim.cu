@@ -4271,9 +4271,18 @@ int batch_capture_steps(gasatt_batch *b, cudaStream_t cs, cudaStream_t side, int
   return rc;
 }
 
+// This thread's calls are not bound, for the time of this object, by a capture that another
+// thread of the program has under way: building a graph would fail, and spoil that capture.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // two capturing streams for the time of `build`
 template <typename F>
 int with_capture_streams(gasatt_ctx *ctx, F build) {
+  const RelaxedCapture relaxed;
   cudaStream_t cs, side;
   GASATT_CUDA(ctx, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) {

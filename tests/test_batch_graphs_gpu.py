@@ -2,9 +2,11 @@
 no more in the FP64 form than its other graphs, and its steps are the same before and after."""
 import statistics
 import time
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import pytest
+import torch
 
 from gasatt import _lib
 from gasatt.dropin import Context
@@ -68,3 +70,31 @@ def test_creation():
         for s in sims:
             s.close()
     assert t[0] < 1.7 * t[1]
+
+
+@pytest.mark.parametrize("precision,steps", [(_lib.FP64, 2000), (_lib.FP32_SPLIT, 100)])
+def test_built_while_another_thread_captures(precision, steps):
+    """The steps that build the graph neither fail because another thread of the program
+    captures a graph of its own, in the mode that binds all threads, nor spoil that capture."""
+    ctx = Context(0)
+    sims = [make(precision, k, ctx) for k in (1, 2)]
+    sims[0].bind_stream(torch.cuda.Stream())
+    batch = Batch(sims, sort_period=0)
+    batch.step(10)
+    torch.cuda.synchronize()
+    x, g = torch.zeros(8, device="cuda"), torch.cuda.CUDAGraph()
+    with ThreadPoolExecutor(1) as other, torch.cuda.graph(g):
+        x.add_(1)
+        other.submit(batch.step, steps).result()
+        x.add_(1)
+    g.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [2.0] * 8
+    batch.close()
+    for k, s in zip((1, 2), sims):
+        alone = make(precision, k, ctx)
+        alone.step(10 + steps)
+        for a, b in zip(state(s), state(alone)):
+            np.testing.assert_array_equal(a, b)
+        alone.close()
+        s.close()
