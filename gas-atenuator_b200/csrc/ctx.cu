@@ -50,6 +50,7 @@ int gasatt_create(gasatt_ctx **out, int device, uint64_t seed) {
   if (cudaSetDevice(device) != cudaSuccess) return GASATT_E_CUDA;
   gasatt_ctx *ctx = new gasatt_ctx();
   ctx->device = device;
+  cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, device);
   ctx->seed = seed;
   if (cudaMallocHost(&ctx->pinned, 4096) != cudaSuccess) {
     delete ctx;

@@ -247,7 +247,7 @@ constexpr int64_t kEmSortParticles = 100000;
 struct EmParams {
   double Rp, Lp, PHIp, cP, sP, hdt;       // hdt: half the particle step
   double id, mu, c, ic2, FN, scale;       // id: 1 / cell size
-  double q[3], m[3], qm[3], qm_dt[3];     // per species: charge, mass, q/m, q/m x particle step
+  double q[3], m[3], qm_dt[3];            // per species: charge, mass, q/m x particle step
   int nr, nz;
   int wrap;                               // azimuth: 0 full ring, 1 wedge of at most pi/2, 2 any other wedge
   bool atan_phi, euler, fast_fx;          // fast_fx: |fixed-point contribution| <= 2^50
@@ -475,10 +475,9 @@ __global__ void __launch_bounds__(kBlock) k_em_push(Species sp, EmState st, EmPa
 // so `pairs` columns and rows on the low side and pairs + 1 on the high side of
 // a patch are recomputed by its neighbours instead of exchanged.  Points outside the grid
 // take the same expressions on zeros; no point inside reads them
-// (fdtd_warp_body has the same rules).  The first H update takes h_first, the
+// (fdtd_block_body has the same rules).  The first H update takes h_first, the
 // others dt/2; a last one takes h_last (0: none).
 constexpr int kEmWarps = 8, kEmSeg = 8, kEmRows = kEmWarps * kEmSeg;
-constexpr int kEmOneLaunch = 148;        // tiles of one launch at most (see gasatt_electricmagneticfield6)
 
 struct EmFields { const double *Er, *Ez, *H; double *oEr, *oEz, *oH; };
 
@@ -1214,8 +1213,7 @@ int gasatt_electricmagneticfield6(gasatt_ctx *ctx, double *e_pos, double *e_vel,
   for (int k = 0; k < 3; ++k) {
     ep.q[k] = k == 0 ? -e : k * e;
     ep.m[k] = k == 0 ? GASATT_EM_ME : GASATT_EM_MION;
-    ep.qm[k] = ep.q[k] / ep.m[k];
-    ep.qm_dt[k] = ep.qm[k] * ddt;
+    ep.qm_dt[k] = ep.q[k] / ep.m[k] * ddt;
   }
   ep.nr = n_r; ep.nz = n_z;
   ep.atan_phi = (flags & GASATT_Q_ATAN_PHI) != 0;
@@ -1238,7 +1236,7 @@ int gasatt_electricmagneticfield6(gasatt_ctx *ctx, double *e_pos, double *e_vel,
   const int whole = 2 * ratio;
   auto tiles_x = [&](int pairs) { return (n_r + em_tile_cols(pairs)) / em_tile_cols(pairs); };
   auto tiles = [&](int pairs) { return (int64_t)tiles_x(pairs) * ((n_z + em_tile_rows(pairs)) / em_tile_rows(pairs)); };
-  const bool single = tiles(whole) <= kEmOneLaunch;
+  const bool single = tiles(whole) <= ctx->sms;
   const EmFields there{Er, Ez, Hphi, Er2, Ez2, H2}, back{Er2, Ez2, H2, Er, Ez, Hphi};
   bool away = false;                                   // the fields are in the scratch set
   // (every kernel of the loop starts while the one before it drains)
@@ -1385,7 +1383,7 @@ int gasatt_electron_collision(gasatt_ctx *ctx, double *e_pos, double *e_vel, int
     k_collision_other<<<grid_for(n, kElThreads), kElThreads, 0, s>>>(e_vel, cap_e, electron_kinetic, t, out, ls, draws,
                                                                     ctx->seed, call, flags);
     GASATT_LAUNCHED(ctx);
-    k_collision_elastic<<<grid_for(n, kElGroup, 4u * 148u), kElThreads, kElSmem, s>>>(
+    k_collision_elastic<<<grid_for(n, kElGroup, 4u * ctx->sms), kElThreads, kElSmem, s>>>(
         e_vel, cap_e, electron_kinetic, t, ls, draws, ctx->seed, call, flags);
     GASATT_LAUNCHED(ctx);
   } else {

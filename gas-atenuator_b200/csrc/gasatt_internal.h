@@ -8,6 +8,7 @@
 
 struct gasatt_ctx {
   int device = 0;
+  int sms = 148;             // its multiprocessors
   uint64_t seed = 0;
   cudaStream_t stream = nullptr;
   std::string err;

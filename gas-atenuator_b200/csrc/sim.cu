@@ -858,7 +858,7 @@ struct BatchCell64 {
   Fields<double> F[2];        // field buffers 0 / 1 (the pass into current buffer jb reads F[jb])
 };
 // empties every cell's queue that the pass after the one of parity q fills
-__global__ void k_batch_commit64(const BatchCell64 *__restrict__ cells, int ncell, int q) {
+__global__ void k_batch_clear_next64(const BatchCell64 *__restrict__ cells, int ncell, int q) {
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x)
     clear_next_queue(cells[c].cnt, q);
 }
@@ -1727,8 +1727,8 @@ struct BatchCell32 {
 
 // The FP32 pass of one step for every cell of a batch in one launch: each
 // block reads the cells' counters and forms the prefix sums of their
-// collision candidates and chunks; the candidates of all cells go first, one
-// per warp, then the blocks take (cell, chunk) work items from one counter
+// collision candidates and chunks; the candidates of all cells go first, two
+// lanes each, then the blocks take (cell, chunk) work items from one counter
 // (*chunk_next, zeroed by the field kernel), copying the cell's parameters into
 // shared memory when the cell changes.  Every cell gives what its own
 // k_pass32 gives.
@@ -2572,7 +2572,8 @@ int launch_pass(gasatt_sim *s, cudaStream_t st, int mode, int jb, int q, int fb,
   cudaError_t e;
   if (s->form == 0) {
     auto kern = mode == 0 ? k_pass64<0> : mode == 1 ? k_pass64<1> : k_pass64<2>;
-    e = launch_early(early, kern, dim3(s->pass_grid), dim3(kBlock), kWin64Bytes, st, P, s->s64[b],
+    // (never early: two kernels are before it)
+    e = launch_early(false, kern, dim3(s->pass_grid), dim3(kBlock), kWin64Bytes, st, P, s->s64[b],
                      fields_of<double>(s, fb), s->cnt, s->queue, q);
   } else {
     auto kern = win_cols(P.nr) < P.nr
@@ -2839,12 +2840,14 @@ int encode_map(gasatt_sim *s, CUtensorMap *m, CUtensorMapDataType type, void *ba
 
 // The patch shape for cells of the given numbers of tiles in the three shapes
 // (fdtd_tile_rows 0): the smallest patches (short segments, so the shortest
-// chain) while they leave half of the GPU's block slots free, the middle ones
+// chain) while they leave half of the GPU's block slots (nsm SMs) free, the middle ones
 // while their tiles are one wave of blocks, beyond that the tallest (the least
 // halo recomputed).  FP32 step with shape 12 / 16 / 20: 32 x 64 cells 18.4 / 19.2
 // / 21.2 us; 256 x 1024 54.3 / 54.4 / 56.7 (FP64 79.7 / 78.5 / 78.4); 1024 x
 // 4096 423 / 417 / 405; 16 batched cells 328 / 314 / 301.
-int tma_auto(long long tiles12, long long tiles16) { return tiles12 <= 4 * 148 ? 12 : tiles16 <= 4 * 148 ? 16 : 20; }
+int tma_auto(long long tiles12, long long tiles16, int nsm) {
+  return tiles12 <= 4 * nsm ? 12 : tiles16 <= 4 * nsm ? 16 : 20;
+}
 
 // The field update's descriptor of a cell for the steps of parity q with patch
 // shape k: tensor maps of the fields and of the current read, where the
@@ -2887,7 +2890,7 @@ template <typename T>
 int setup_fdtd_tma(gasatt_sim *s, int nsm) {
   const auto &c = s->cfg;
   const int k = c.fdtd_tile_rows > 0 ? c.fdtd_tile_rows
-                                     : tma_auto(tma_tiles(12, c.n_r, c.n_z), tma_tiles(16, c.n_r, c.n_z));
+                                     : tma_auto(tma_tiles(12, c.n_r, c.n_z), tma_tiles(16, c.n_r, c.n_z), nsm);
   if (!tma_rows_ok(k)) return fail(s->ctx, GASATT_E_ARG, "fdtd_tile_rows: 12, 16 or 20");
   s->tma_rows = k;
   s->tma_smem = tma_block_bytes<T>(k);
@@ -3294,8 +3297,7 @@ int gasatt_sim_create(gasatt_ctx *ctx, const gasatt_sim_config *cfg, const gasat
   if ((rc = sim_alloc(s, &s->d_P, 2)) || (rc = upload_params(s))) return cleanup(rc);
   if (fdtd_tile(c.fdtd_ratio) < 4)
     return cleanup(fail(ctx, GASATT_E_ARG, "fdtd_ratio too large for the fused field update (max 6)"));
-  int dev = ctx->device, nsm = 148;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int nsm = ctx->sms;
   if (c.fdtd_ratio == 1) {
     if ((rc = s->form == 0 ? setup_fdtd_tma<double>(s, nsm) : setup_fdtd_tma<float>(s, nsm)))
       return cleanup(rc);
@@ -4150,6 +4152,7 @@ int batch_group_setup(gasatt_batch *b, BatchGroup &G) {
     GASATT_CUDA(ctx, cudaMemcpy(d, h.data(), sizeof(BatchCell64) * n, cudaMemcpyHostToDevice));
     G.cells = d;
   }
+  const int nsm = ctx->sms;
   // one patch shape for the group: its cells' own knob value, or by all their tiles
   if (!G.ph) {
     long long t12 = 0, t16 = 0;
@@ -4157,7 +4160,7 @@ int batch_group_setup(gasatt_batch *b, BatchGroup &G) {
       t12 += tma_tiles(12, s->cfg.n_r, s->cfg.n_z);
       t16 += tma_tiles(16, s->cfg.n_r, s->cfg.n_z);
     }
-    G.ph = tma_auto(t12, t16);
+    G.ph = tma_auto(t12, t16, nsm);
   }
   std::vector<int2> table;
   for (int i = 0; i < n; ++i)
@@ -4174,8 +4177,7 @@ int batch_group_setup(gasatt_batch *b, BatchGroup &G) {
     GASATT_CUDA(ctx, cudaMemcpy(G.insts[q], hi.data(), sizeof(FdtdInst) * n, cudaMemcpyHostToDevice));
   }
   SIM_TRY(batch_alloc(b, &G.chunk_next, 1));
-  int nsm = 148, occ = 1;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
+  int occ = 1;
   G.fdtd_smem = G.form == 1 ? tma_block_bytes<float>(G.ph) : tma_block_bytes<double>(G.ph);
   const BatchFdtdTmaFn fk = G.form == 1 ? batch_fdtd_tma_fn<float>(G.ph) : batch_fdtd_tma_fn<double>(G.ph);
   GASATT_CUDA(ctx, cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G.fdtd_smem));
@@ -4217,7 +4219,7 @@ int batch_group_launch(gasatt_batch *b, BatchGroup &G, cudaStream_t cs, cudaStre
   }
   GASATT_CUDA(ctx, cudaEventRecord(b->fork_ev, cs));
   GASATT_CUDA(ctx, cudaStreamWaitEvent(side, b->fork_ev, 0));
-  k_batch_commit64<<<1, 256, 0, side>>>((const BatchCell64 *)G.cells, n, 1 - q);
+  k_batch_clear_next64<<<1, 256, 0, side>>>((const BatchCell64 *)G.cells, n, 1 - q);
   k_batch_mcc64<<<G.mcc_grid, kMccBlock, 0, side>>>((const BatchCell64 *)G.cells, n, cur, 1 - q);
   GASATT_CUDA(ctx, cudaGetLastError());
   GASATT_CUDA(ctx, cudaEventRecord(b->join_ev, side));
@@ -4339,7 +4341,7 @@ int batch_steps_ready(gasatt_batch *b, int cur, bool *ready) {
 
 // flush_collisions for every cell of the batch (before its sort): a group
 // whose cells are at the same step parity and state buffer does it in two
-// launches (FP32: k_batch_collide32) or three (FP64: k_batch_commit64, then
+// launches (FP32: k_batch_collide32) or three (FP64: k_batch_clear_next64, then
 // k_batch_mcc64) for all of its cells, then empties their queues; any other
 // cell flushes on its own.  A cell with nothing pending finds an empty queue
 // (its own flush emptied it).
@@ -4364,7 +4366,7 @@ int batch_flush_collisions(gasatt_batch *b) {
       k_batch_clear_cand<<<1, 256, 0, st>>>((const BatchCell32 *)G.cells, n, -1);   // see flush_collisions
       ctx->launches += 2;
     } else {
-      k_batch_commit64<<<1, 256, 0, st>>>((const BatchCell64 *)G.cells, n, q);
+      k_batch_clear_next64<<<1, 256, 0, st>>>((const BatchCell64 *)G.cells, n, q);
       k_batch_mcc64<<<G.mcc_grid, kMccBlock, 0, st>>>((const BatchCell64 *)G.cells, n, cur, q);
       k_batch_clear_cand<<<1, 256, 0, st>>>((const BatchCell64 *)G.cells, n, q);
       ctx->launches += 3;
