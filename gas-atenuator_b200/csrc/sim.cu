@@ -4287,9 +4287,10 @@ int with_capture_streams(gasatt_ctx *ctx, F build) {
   const RelaxedCapture relaxed;
   cudaStream_t cs, side;
   GASATT_CUDA(ctx, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-  if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) {
+  const cudaError_t e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+  if (e != cudaSuccess) {
     cudaStreamDestroy(cs);
-    return fail(ctx, GASATT_E_CUDA, "batch: stream");
+    return cuda_fail(ctx, e, "batch: stream");
   }
   const int rc = build(cs, side);
   cudaStreamDestroy(side);
@@ -4328,15 +4329,24 @@ int batch_build_graphs(gasatt_batch *b, cudaStream_t cs, cudaStream_t side) {
   return rc;
 }
 
-// whether the graph of ten steps is there, or worth building now (and built)
-int batch_steps_ready(gasatt_batch *b, int cur, bool *ready) {
-  if (!b->g_steps[cur] && b->lone[cur] >= b->worth)
-    SIM_TRY(with_capture_streams(b->ctx, [&](cudaStream_t cs, cudaStream_t side) {
+// Whether the graph of ten steps is there, or worth building now (and built).  A batch that
+// cannot build it, for want of memory say, goes on without.
+bool batch_steps_ready(gasatt_batch *b, int cur) {
+  if (!b->g_steps[cur] && b->lone[cur] >= b->worth) {
+    const std::string err = b->ctx->err;
+    const int rc = with_capture_streams(b->ctx, [&](cudaStream_t cs, cudaStream_t side) {
       return batch_capture_steps(b, cs, side, cur, 0, kGraphSteps, &b->g_steps[cur]);
-    }));
-  *ready = b->g_steps[cur] != nullptr;
-  if (!*ready) b->lone[cur] += 2;          // (asked at every other step)
-  return GASATT_OK;
+    });
+    if (rc) {
+      cudaGetLastError();                  // (the capture's end may have left one)
+      b->g_steps[cur] = nullptr;
+      b->worth = INT64_MAX;
+      b->ctx->err = err;
+    }
+  }
+  if (b->g_steps[cur]) return true;
+  b->lone[cur] += 2;                       // (asked at every other step)
+  return false;
 }
 
 // flush_collisions for every cell of the batch (before its sort): a group
@@ -4463,11 +4473,7 @@ int gasatt_batch_step(gasatt_batch *b, int nsteps) {
       if (!steps_fit(s, b->sort_period)) many = 1;
     }
     if (!lockstep) many = 1;
-    if (many > 1) {
-      bool ready;
-      SIM_TRY(batch_steps_ready(b, s0->cur, &ready));
-      if (!ready) many = 1;
-    }
+    if (many > 1 && !batch_steps_ready(b, s0->cur)) many = 1;
     if (lockstep) {
       GASATT_CUDA(ctx, cudaGraphLaunch(many > 1 ? b->g_steps[s0->cur] : b->g[s0->cur][s0->host_step & 1], st));
       for (const BatchGroup &G : b->groups) ctx->launches += many * (G.form == 0 ? 4 : 2);
